@@ -214,6 +214,310 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
   return ok;
 }
 
+// ---- small clique-tree nodes, closed in one step ------------------------------
+//
+// A pivoting node (candidate set F of nc vertices, `drop` pivots, r = k - held)
+// contributes sum_j C(drop, j) cliques(G[F], r - j). Walked node by node that
+// costs a warp about 1.5 us of latency per tree node (frame, candidate list,
+// scores, reductions) with most lanes idle, and almost all nodes of a tree are
+// small and near its leaves. Two kinds are therefore counted whole: r = 3 with
+// at most 128 candidates (triangles, edges and vertices of G[F]) and r in
+// 4..20 with at most 32 candidates (a lane per pair of adjacent candidates).
+// Both first copy G[F] into a compact bitmap of nc rows and ceil(nc / 32)
+// words. Larger nodes are worth splitting further: their branches are what
+// the walkers share. R-MAT scale 17, k = 5 (edge units): 37.8M tree nodes,
+// 37.1 ms before; 1.4M, 6.3 ms now. Chung-Lu 1M + planted cliques, k = 6
+// (node units): 76.7M, 145 ms before; 3.7M, 48 ms now. R-MAT of 21k edges,
+// k = 8, built, oriented and counted: 3.5 ms before, 1.6 ms now.
+
+// The compact bitmap of the candidates cand[0, nc) (ascending): bit i of row j
+// is set when cand[i] and cand[j] are adjacent (UPPER: and i > j). The lanes
+// test a row's nc bits side by side, and a ballot makes 32 of them a word: the
+// lanes read one row of B at a time, so there are no bank conflicts, and there
+// is no dependence between rows. Rows have ST words in out (ST = 1, 2 or 4).
+template <int NW, int ST, bool UPPER>
+__device__ __forceinline__ void compact_rows(const uint32_t* B, uint32_t Ws, const uint32_t* cand, uint32_t nc,
+                                             uint32_t* out) {
+  const uint32_t lane = lane_id();
+  uint32_t cw[NW], cb[NW];
+#pragma unroll
+  for (int t = 0; t < NW; ++t) {
+    const uint32_t i = (uint32_t)t * 32u + lane;
+    const uint32_t c = cand[i < nc ? i : 0u];
+    cw[t] = c >> 5;
+    cb[t] = i < nc ? (1u << (c & 31u)) : 0u;
+  }
+#pragma unroll 4
+  for (uint32_t j = 0; j < nc; ++j) {
+    const uint32_t* row = B + cand[j] * Ws;
+    uint32_t m[ST];
+#pragma unroll
+    for (int t = 0; t < ST; ++t) {
+      m[t] = 0u;
+      if (t < NW) {
+        m[t] = __ballot_sync(0xffffffffu, (row[cw[t < NW ? t : 0]] & cb[t < NW ? t : 0]) != 0u);
+        if (UPPER)
+          m[t] &= (uint32_t)t > (j >> 5) ? 0xffffffffu : ((uint32_t)t == (j >> 5) ? 0xfffffffeu << (j & 31u) : 0u);
+      }
+    }
+    if (lane == 0) {
+      if constexpr (ST == 4) *reinterpret_cast<uint4*>(out + j * 4u) = make_uint4(m[0], m[1], m[2], m[3]);
+      else if constexpr (ST == 2) *reinterpret_cast<uint2*>(out + j * 2u) = make_uint2(m[0], m[1]);
+      else out[j] = m[0];
+    }
+  }
+  __syncwarp();
+}
+
+// Carry-save counter of set bits: POPC runs at an eighth of the logic rate, so
+// four words are added into `ones` / `twos` with six LOP3 and one POPC.
+struct BitCount {
+  uint32_t ones = 0, twos = 0, fours = 0;  // fours: already popcounted
+  __device__ __forceinline__ void add4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    const uint32_t t1 = (ones & a) | (ones & b) | (a & b);
+    ones = ones ^ a ^ b;
+    const uint32_t t2 = (ones & c) | (ones & d) | (c & d);
+    ones = ones ^ c ^ d;
+    const uint32_t f = (twos & t1) | (twos & t2) | (t1 & t2);
+    twos = twos ^ t1 ^ t2;
+    fours += __popc(f);
+  }
+  __device__ __forceinline__ uint32_t total() const { return 4u * fours + 2u * __popc(twos) + __popc(ones); }
+};
+
+// Triangles of a graph of nc <= 32 NW vertices whose upper rows (ST words
+// each, zero rows up to a multiple of four) are in up: lane i keeps rows i,
+// i + 32, .., every row j is broadcast to all lanes, and a lane whose row holds
+// j adds the common upper neighbours. No divergence and no bank conflicts,
+// about nc^2 / 64 words per lane whatever the density. Returns the lane's
+// share of the triangles and, in edges, of the edges.
+template <int NW, int ST>
+__device__ __forceinline__ uint32_t count_triangles(const uint32_t* up, uint32_t nc, uint32_t& edges) {
+  const uint32_t lane = lane_id();
+  uint32_t P[NW][ST];
+  edges = 0;
+#pragma unroll
+  for (int g = 0; g < NW; ++g) {
+    const uint32_t i = (uint32_t)g * 32u + lane;
+#pragma unroll
+    for (int w = 0; w < ST; ++w) P[g][w] = 0u;
+    if (i < nc) {
+      if constexpr (ST > 1) {
+        load_row<ST>(up, i, P[g]);
+      } else {
+        P[g][0] = up[i];
+      }
+    }
+#pragma unroll
+    for (int w = g; w < NW; ++w) edges += __popc(P[g][w]);
+  }
+  BitCount bc;
+#pragma unroll
+  for (int jb = 0; jb < NW; ++jb) {  // rows 32 jb .. 32 jb + 31
+    const uint32_t je = min(nc, (uint32_t)jb * 32u + 32u);
+    for (uint32_t j0 = (uint32_t)jb * 32u; j0 < je; j0 += 4u) {
+      uint32_t U[4][ST];
+      if constexpr (ST == 1) {
+        load_row<4>(up + j0, 0u, *reinterpret_cast<uint32_t(*)[4]>(&U[0][0]));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) load_row<ST>(up, j0 + (uint32_t)q, U[q]);
+      }
+#pragma unroll
+      for (int g = 0; g <= jb; ++g) {
+        uint32_t has[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) has[q] = 0u - ((P[g][jb] >> ((j0 + (uint32_t)q) & 31u)) & 1u);
+#pragma unroll
+        for (int w = jb; w < NW; ++w)
+          bc.add4(P[g][w] & U[0][w] & has[0], P[g][w] & U[1][w] & has[1], P[g][w] & U[2][w] & has[2],
+                  P[g][w] & U[3][w] & has[3]);
+      }
+    }
+  }
+  return bc.total();
+}
+
+// Words of the compact bitmap of up to `n` candidates, and of the prefix table
+// of close_small.
+__host__ __device__ constexpr uint32_t compact_words(uint32_t n) {
+  return n <= 32u ? 36u : (n <= 64u ? 64u * 2u : 128u * 4u);
+}
+constexpr uint32_t kPairPrefix = 36;   // close_small: exclusive prefix of the row lengths
+constexpr uint32_t kTriangleMax = 128; // most candidates of an r = 3 node closed whole
+constexpr uint32_t kSmallMax = 32;     // most candidates of an r > 3 node closed whole
+constexpr int kSmallStack = 16;        // close_small: pushed frames (r - 5 at most)
+constexpr uint32_t kSmallMaxR = 20;
+
+// r = 3: triangles + drop edges + C(drop, 2) vertices + C(drop, 3). Every lane
+// returns its share.
+template <int NW, int ST>
+__device__ __forceinline__ unsigned long long close_triangles(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
+                                                           uint32_t nc, uint32_t* up, uint32_t drop) {
+  const uint32_t pad = (nc + 3u) & ~3u;
+  if (lane_id() < (pad - nc) * ST) up[nc * ST + lane_id()] = 0u;  // (nc is at most 32 NW, a multiple of four)
+  compact_rows<NW, ST, true>(B, Ws, cand, nc, up);
+  uint32_t edges = 0;
+  unsigned long long t = count_triangles<NW, ST>(up, nc, edges);
+  const unsigned long long d = drop;
+  t += d * edges;
+  if (lane_id() == 0) {
+    if (d >= 2ull) t += d * (d - 1ull) / 2ull * nc;
+    if (d >= 3ull) t += d * (d - 1ull) / 2ull * (d - 2ull) / 3ull;
+  }
+  return t;
+}
+
+__device__ __forceinline__ unsigned __int128 binom_at(const unsigned long long* binom, uint32_t cols, uint32_t nn,
+                                                      uint32_t r) {
+  if (r > nn) return 0;
+  const unsigned long long* e = binom + 2ull * ((size_t)nn * (cols + 1u) + r);
+  return ((unsigned __int128)e[1] << 64) | e[0];
+}
+
+// r >= 3 with at most 32 candidates: adj holds their rows (one word each,
+// symmetric). The empty set and single candidates are closed; every pair
+// i < j of adjacent candidates is a task (pairs, not vertices: a dense node's
+// first vertices hold most of its cliques), taken by the lanes in turn, with
+// the common neighbours above j as its candidate set X and r - 2 vertices to
+// go. A lane counts its tasks alone, with sets in registers: r = 1 to 3 by
+// listing, above that by pivoting. Vertices adjacent to the whole set are
+// moved to the pivots at once (their branches are empty). Returns the lane's
+// share; pre[32] receives the most rows any lane visited.
+__device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, uint32_t* pre, uint32_t nc, uint32_t r,
+                                                      uint32_t drop, const unsigned long long* binom, uint32_t cols) {
+  const uint32_t lane = lane_id();
+  const uint32_t mine = lane < nc ? adj[lane] & (0xfffffffeu << lane) : 0u;
+  const uint32_t c = __popc(mine);
+  uint32_t incl = c;
+#pragma unroll
+  for (uint32_t o = 1; o < 32u; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  pre[lane] = incl - c;
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+  unsigned __int128 acc = 0;
+  if (lane == 0) {
+    acc = binom_at(binom, cols, drop, r);
+    if (drop + 1u >= r) acc += (unsigned __int128)nc * binom_at(binom, cols, drop, r - 1u);
+  }
+  __syncwarp();
+  uint32_t it = 0;
+  uint32_t sP[kSmallStack], sR[kSmallStack], sX[kSmallStack];  // set, branches left, pivot and drop
+  for (uint32_t t = lane; t < total; t += 32u) {
+    uint32_t i = 0;  // pre[i] <= t < pre[i + 1]
+#pragma unroll
+    for (uint32_t s = 16; s; s >>= 1)
+      if (pre[i + s] <= t) i += s;
+    const uint32_t ui = adj[i] & (0xfffffffeu << i);
+    const uint32_t j = select_bit(ui, t - pre[i]);
+    uint32_t P = ui & adj[j] & (0xfffffffeu << j);
+    uint32_t rr = r - 2u, dd = drop;
+    int lv = 0;
+    for (;;) {
+      // the node (P, rr, dd)
+      const uint32_t n = __popc(P);
+      if (n + dd >= rr) {
+        if (n == 0u) {
+          acc += binom_at(binom, cols, dd, rr);
+        } else if (rr == 1u) {
+          acc += n + dd;
+        } else if (rr <= 3u) {
+          uint32_t e = 0, tri = 0;
+          for (uint32_t x = P; x; x &= x - 1u) {
+            const uint32_t u = (uint32_t)__ffs(x) - 1u;
+            const uint32_t X = (x & (x - 1u)) & adj[u];
+            e += __popc(X);
+            ++it;
+            if (rr == 3u)
+              for (uint32_t y = X; y; y &= y - 1u) {
+                tri += __popc((y & (y - 1u)) & adj[__ffs(y) - 1]);
+                ++it;
+              }
+          }
+          const unsigned long long d1 = dd, d2 = d1 * (d1 - 1ull) / 2ull;  // (0 for dd = 0)
+          if (rr == 2u) {
+            acc += e + d1 * n + (dd >= 2u ? d2 : 0ull);
+          } else {
+            acc += tri + d1 * e + (dd >= 2u ? d2 * n : 0ull) + (dd >= 3u ? d2 * (d1 - 2ull) / 3ull : 0ull);
+          }
+        } else {
+          uint32_t best = 0, uni = 0;  // best: 1 + score, in the high half, of a non-universal candidate
+          for (uint32_t x = P; x; x &= x - 1u) {
+            const uint32_t u = (uint32_t)__ffs(x) - 1u;
+            const uint32_t s = __popc(P & adj[u]);
+            if (s + 1u == n) uni |= 1u << u;
+            else best = max(best, ((s + 1u) << 16) | u);
+            ++it;
+          }
+          dd += __popc(uni);
+          P &= ~uni;
+          if (P == 0u) {
+            acc += binom_at(binom, cols, dd, rr);
+          } else if (KC_IN_BOUNDS(lv, kSmallStack, nullptr)) {
+            const uint32_t piv = best & 0xffffu;
+            sP[lv] = P;
+            sR[lv] = P & ~adj[piv] & ~(1u << piv);
+            sX[lv] = (rr << 24) | (piv << 16) | dd;
+            ++lv;
+          }
+        }
+      }
+      // the next branch: the candidates outside the pivot's neighbourhood,
+      // then the pivot's own branch in its parent's frame
+      if (lv == 0) break;
+      const uint32_t R = sR[lv - 1], x = sX[lv - 1];
+      P = sP[lv - 1];
+      rr = x >> 24;
+      dd = x & 0xffffu;
+      if (R) {
+        const uint32_t u = (uint32_t)__ffs(R) - 1u;
+        sR[lv - 1] = R & (R - 1u);
+        sP[lv - 1] = P & ~(1u << u);
+        P &= adj[u];
+        --rr;
+      } else {
+        --lv;
+        P &= adj[(x >> 16) & 31u];
+        ++dd;
+      }
+    }
+  }
+  it = __reduce_max_sync(0xffffffffu, it);
+  if (lane == 0) pre[32] = it;
+  return acc;
+}
+
+// A node counted whole (see above): its candidates are cand[0, nc), or, with
+// cand null, its symmetric rows of one word are B itself. One copy of this
+// code serves every call site. The lane's share is returned and cmp[0] holds
+// the node's cost, in tree nodes of the work budget.
+__device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t Ws, const uint32_t* cand, uint32_t nc,
+                                                     uint32_t* cmp, uint32_t r, uint32_t drop,
+                                                     const unsigned long long* binom, uint32_t cols) {
+  unsigned __int128 t;
+  uint32_t cost = 1u + (nc >> 5);
+  if (r > 3u) {
+    if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
+    t = close_small(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols);
+    __syncwarp();
+    cost = 1u + (cmp[kPairPrefix + 32u] >> 5);
+  } else if (nc <= 32u) {
+    t = close_triangles<1, 1>(B, Ws, cand, nc, cmp, drop);
+  } else if (nc <= 64u) {
+    t = close_triangles<2, 2>(B, Ws, cand, nc, cmp, drop);
+  } else if (nc <= 96u) {
+    t = close_triangles<3, 4>(B, Ws, cand, nc, cmp, drop);
+  } else {
+    t = close_triangles<4, 4>(B, Ws, cand, nc, cmp, drop);
+  }
+  __syncwarp();
+  if (lane_id() == 0) cmp[0] = cost;
+  __syncwarp();
+  return t;
+}
+
 // Register budgets: orientation fits 56 registers without spills (four
 // 256-thread CTAs per SM); pivoting needs 80 (three), spilling below that.
 template <int MODE, bool LOCAL>
@@ -251,7 +555,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   uint32_t* B = p.bitmap_global ? gb : sb + p.off_B;
   uint32_t* R0 = sb + p.off_R0;
   uint32_t* frames = (p.frames_global ? gb + p.goff_fr : sb + p.off_fr) + (size_t)part * p.pstride;
-  uint32_t* cand = frames + (size_t)p.depth * p.fw;  // pivoting: the candidates of the node being entered
+  uint32_t* cand = frames + p.off_cand;  // pivoting: the candidates of the node being entered
+  // pivoting: the compact bitmap of a node counted whole (then its prefix table)
+  const bool compact = MODE == 1 && !LOCAL && p.compact != 0u && p.nk == 0u;
+  uint32_t* cmp = cand + ((p.dcap + 3u) & ~3u);
   // open-addressing hash of S: vertex -> local index (linear probing, load <= 1/2)
   const uint32_t hT = p.hash_T;
   uint32_t* hkey = sb + p.off_H;
@@ -306,14 +613,16 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // until the unit is known to have finished.
   const bool budgeted = p.budget != 0;
   unsigned __int128 uacc = 0;
+  unsigned __int128 lacc = 0;  // pivoting: this lane's share of the nodes counted whole
   uint32_t since_charge = 0;
   auto over_budget = [&]() -> bool {  // partition-uniform
     uint32_t stop = 0;
     if (pt.plane == 0) {
       stop = *(volatile uint32_t*)&hdr[5];
       if (!stop && ++since_charge >= 64) {
+        const uint32_t add = since_charge;
         since_charge = 0;
-        if (atomicAdd(&hdr[4], 64u) + 64u > p.budget) {
+        if (atomicAdd(&hdr[4], add) + add > p.budget) {
           hdr[5] = 1u;
           stop = 1u;
         }
@@ -399,6 +708,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (timing) tc = clk32();
     const uint32_t unit = p.queue[pos];
     uacc = 0;
+    lacc = 0;
     since_charge = 0;
     uint32_t src, d;
     if (!p.edge_units) {
@@ -858,6 +1168,17 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           }
         }
       }
+    } else if (MODE == 1 && compact && (d <= kSmallMax || (d <= kTriangleMax && k == (p.edge_units ? 5u : 4u))) &&
+               k <= kSmallMaxR) {
+      // ---- a unit counted whole (edge roots: their sum is the unit's count)
+      const uint32_t r = k - (p.edge_units ? 2u : 1u);  // >= 3 here
+      if (part == 0 && !helper) {
+        st_nodes++;
+        for (uint32_t i = pt.plane; i < d; i += 32u) cand[i] = i;
+        __syncwarp();
+        lacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
+        st_words += 32u * cmp[0];
+      }
     } else {
       // ---- pivot traversal (succinct clique tree)
       // Root: a pivot p0 of G[S] and its branches R0 = S \ N(p0). With edge
@@ -895,6 +1216,41 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         const unsigned long long* e = p.binom + 2ull * ((size_t)nn * (p.binom_cols + 1u) + r);
         return ((unsigned __int128)e[1] << 64) | e[0];
       };
+      // Work split inside the unit: the clique tree (root at depth 0) is cut
+      // at depth L and the nodes at depth L go out by ticket (hdr[1]) to the
+      // group's partitions. Every partition walks the levels above the cut
+      // itself, re-deriving the same pivots, so no frame crosses partitions;
+      // partition 0 alone adds what the nodes above the cut contribute.
+      // L grows when the root has few branches (dense units, whose pivot
+      // neighbours nearly everything).
+      // The cut is sized for the CTA's own partitions (helpers take what is
+      // left of it): a deeper cut would make every walker, helpers included,
+      // walk more levels above it, and on bushy trees that costs more than
+      // the finer split gains.
+      const uint32_t nparts = G / pt.P;
+      uint32_t nr0 = 0;
+      for (uint32_t w = pt.plane; w < W; w += pt.P) nr0 += __popc(R0[w]);
+      nr0 = __reduce_add_sync(pt.pmask, nr0);
+      const uint32_t L = (nparts == 1u || nr0 >= 4u * nparts) ? 1u : (nr0 <= 2u ? 3u : 2u);
+      const bool top_owner = part == 0u && !helper;
+      uint32_t* cut_ticket = help ? p.help_ticket + pos : &hdr[1];
+      if (help && !helper && gt == 0) {  // the unit can take helpers from now on
+        __threadfence();
+        *(volatile uint32_t*)&p.help_active[blockIdx.x] = (uint32_t)pos + 1u;
+      }
+      auto ticket = [&]() -> uint32_t {
+        uint32_t t = 0;
+        if (pt.plane == 0) t = atomicAdd(cut_ticket, 1u);
+        return __shfl_sync(pt.pmask, t, pt.pbase);
+      };
+      uint32_t seen = 0, mine = ticket();
+      auto claim = [&]() -> bool {  // at a depth-L node: does this partition take it?
+        const bool take = seen == mine;
+        ++seen;
+        if (take) mine = ticket();
+        return take;
+      };
+
       // A clique-tree node with `hold` held vertices, `drop` pivots and the
       // candidate set F[0, W) contributes sum_j C(drop, j) * cliques(G[F], r - j)
       // with r = k - hold. For r <= 2 that sum is closed (cliques of size 0,
@@ -914,7 +1270,9 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
       unsigned __int128 leaf_cnt = 0, leaf_pinc = 0;
       // pchild: the node is its parent's pivot branch (same held vertices);
       // otherwise it holds one vertex more than its parent
-      auto enter = [&](uint32_t* F, uint32_t hold, uint32_t drop, bool own, bool pchild) -> bool {
+      // above: a node above the cut, which every walker of the unit enters; a
+      // node counted whole there goes to the walker that holds its ticket
+      auto enter = [&](uint32_t* F, uint32_t hold, uint32_t drop, bool own, bool pchild, bool above) -> bool {
         uint32_t nc = 0, nzm = 0;
         if (narrow) {
           const uint32_t x = pt.plane < W ? F[pt.plane] : 0u;
@@ -949,11 +1307,16 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
               for (uint32_t x = F[w]; x; x &= x - 1u) loc2_add(w * 32u + (uint32_t)__ffs(x) - 1u, 1u);
           return false;
         }
-        // score every candidate u by |F ∩ N(u)|: the candidates are listed
-        // in order first (one pass over the words, a bit per lane), then the
-        // lanes take them in turn, so each lane scores ceil(nc / P) of them
-        uint32_t best = 0;
+        // a small node is counted whole: the walker that owns it copies G[F]
+        // and counts it (see close_triangles and close_small)
+        auto small = [&](uint32_t n) { return compact && r >= 3u && n <= (r == 3u ? kTriangleMax : kSmallMax) && r <= kSmallMaxR; };
+        bool whole = small(nc);
+        if (whole && !(above ? claim() : own)) return false;
+        uint32_t best = 0, nw = 0;
         unsigned long long esum = 0;
+      relist:
+        // the candidates are listed in order first (one pass over the words,
+        // a bit per lane)
         if (narrow) {
           uint32_t base = 0;
           for (uint32_t m = nzm; m; m &= m - 1u) {
@@ -975,16 +1338,29 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           }
         }
         __syncwarp(pt.pmask);
+        nw = narrow ? (uint32_t)__popc(nzm) : W;
+        if (whole) {
+          lacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
+          const uint32_t cost = cmp[0];
+          since_charge += cost;
+          st_words += 32u * cost;
+          return false;
+        }
+        // score every candidate u by |F ∩ N(u)|; the lanes take the listed
+        // candidates in turn, so each lane scores ceil(nc / P) of them.
         // Q lanes score one candidate, each over every Q-th word: as many as
         // leave no lane idle (one per candidate once there are 32 of them),
         // at most the launch's partition size
-        const uint32_t nw = narrow ? (uint32_t)__popc(nzm) : W;
         uint32_t Q = 1u;
         while ((Q << 1) * nc <= pt.P && Q < nw) Q <<= 1;
         if (p.Q != 0u && Q > p.Q) Q = p.Q;
         const uint32_t qs = (uint32_t)__ffs(Q) - 1u;  // Q is a power of two
         const uint32_t ng = pt.P >> qs, gq = pt.plane >> qs, lq = pt.plane & (Q - 1u);
-        for (uint32_t i0 = 0; i0 < nc; i0 += ng) {
+        // Universal candidates (adjacent to every other one): their branch
+        // sets are empty, so all of them become pivots in this one step.
+        const bool univ = !LOCAL && nc <= 32u * ng;  // (a bit of `um` per candidate of this lane)
+        uint32_t um = 0, ub = 1u;
+        for (uint32_t i0 = 0; i0 < nc; i0 += ng, ub <<= 1) {
           const uint32_t i = i0 + gq;
           uint32_t c = 0, u = 0;
           if (i < nc) {
@@ -1004,7 +1380,8 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           for (uint32_t o = 1; o < Q; o <<= 1) c += __shfl_xor_sync(pt.pmask, c, o);
           if (i < nc && lq == 0u) {
             esum += c;
-            best = max(best, (c << 16) | (0xffffu - u));
+            if (univ && c + 1u == nc) um |= ub;
+            else best = max(best, (c << 16) | (0xffffu - u));
             // r = 2: candidate u is in a clique with each neighbour in F and each pivot
             if (lc && own && r == 2u && c + drop) loc2_add(u, c + drop);
           }
@@ -1020,6 +1397,27 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         // several k: a smaller k that reaches k - hold = 2 here is closed here
         if (mk && own && kopen && kl == hold + 2u)
           uacc += (unsigned __int128)(esum / 2u) + (unsigned __int128)drop * nc + binom(drop, 2u);
+        if (univ && __any_sync(pt.pmask, um != 0u)) {
+          const uint32_t nu = __reduce_add_sync(pt.pmask, (uint32_t)__popc(um));
+          for (uint32_t x = um; x; x &= x - 1u) {
+            const uint32_t u = cand[((uint32_t)__ffs(x) - 1u) * ng + gq];
+            atomicAnd(&F[u >> 5], ~(1u << (u & 31u)));
+          }
+          __syncwarp(pt.pmask);
+          drop += nu;
+          nc -= nu;
+          if (nc == 0u) {  // F was a clique: a leaf with all of it as pivots
+            leaf_cnt = binom(drop, r);
+            if (own) uacc += mk ? ((kopen && kl >= hold + 3u) ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
+            return false;
+          }
+          if (narrow) nzm = __ballot_sync(pt.pmask, pt.plane < W && F[pt.plane] != 0u);
+          if (small(nc)) {  // what is left is small
+            whole = true;
+            if (!(above ? claim() : own)) return false;
+            goto relist;
+          }
+        }
         best = __reduce_max_sync(pt.pmask, best);
         const uint32_t piv = 0xffffu - (best & 0xffffu);
         // branch set: candidates outside N(piv), less the pivot itself, whose
@@ -1038,41 +1436,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         }
         __syncwarp(pt.pmask);
         return true;
-      };
-
-      // Work split inside the unit: the clique tree (root at depth 0) is cut
-      // at depth L and the nodes at depth L go out by ticket (hdr[1]) to the
-      // group's partitions. Every partition walks the levels above the cut
-      // itself, re-deriving the same pivots, so no frame crosses partitions;
-      // partition 0 alone adds what the nodes above the cut contribute.
-      // L grows when the root has few branches (dense units, whose pivot
-      // neighbours nearly everything).
-      // The cut is sized for the CTA's own partitions (helpers take what is
-      // left of it): a deeper cut would make every walker, helpers included,
-      // walk more levels above it, and on bushy trees that costs more than
-      // the finer split gains.
-      const uint32_t nparts = G / pt.P;
-      uint32_t nr0 = 0;
-      for (uint32_t w = pt.plane; w < W; w += pt.P) nr0 += __popc(R0[w]);
-      nr0 = __reduce_add_sync(pt.pmask, nr0);
-      const uint32_t L = (nparts == 1u || nr0 >= 4u * nparts) ? 1u : (nr0 <= 2u ? 3u : 2u);
-      const bool top_owner = part == 0u && !helper;
-      uint32_t* cut_ticket = help ? p.help_ticket + pos : &hdr[1];
-      if (help && !helper && gt == 0) {  // the unit can take helpers from now on
-        __threadfence();
-        *(volatile uint32_t*)&p.help_active[blockIdx.x] = (uint32_t)pos + 1u;
-      }
-      auto ticket = [&]() -> uint32_t {
-        uint32_t t = 0;
-        if (pt.plane == 0) t = atomicAdd(cut_ticket, 1u);
-        return __shfl_sync(pt.pmask, t, pt.pbase);
-      };
-      uint32_t seen = 0, mine = ticket();
-      auto claim = [&]() -> bool {  // at a depth-L node: does this partition take it?
-        const bool take = seen == mine;
-        ++seen;
-        if (take) mine = ticket();
-        return take;
       };
 
       // Local counts: a frame also keeps its held vertex (the branch that
@@ -1130,7 +1493,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         uint32_t* F0 = frames;
         for (uint32_t w = pt.plane; w < W; w += pt.P) F0[w] = B[v * Ws + w] & ~(R0[w] & low_mask(v, w));
         __syncwarp(pt.pmask);
-        if (!enter(F0, hold, drop, own1, v == p0)) {
+        if (!enter(F0, hold, drop, own1, v == p0, L > 1u)) {
           if (lc && own1 && pt.plane == 0) {
             const unsigned __int128 x = (v != p0) ? leaf_cnt : leaf_pinc;
             if (x) loc2_add(v, x);
@@ -1169,7 +1532,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
             }
             for (uint32_t w = pt.plane; w < W; w += pt.P) F[w] &= B[fp * Ws + w];
             __syncwarp(pt.pmask);
-            if (!enter(F, fh, fd + 1u, own, true)) {
+            if (!enter(F, fh, fd + 1u, own, true, (uint32_t)lv + 1u < L)) {
               if (lc) {
                 if (pt.plane == 0) {
                   if (own) fr_take(F);
@@ -1204,7 +1567,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           __syncwarp(pt.pmask);
           if (pt.plane == 0) F[u >> 5] &= ~(1u << (u & 31u));  // later siblings exclude u
           __syncwarp(pt.pmask);
-          if (descend && enter(Fc, h2, fd, own, false)) {
+          if (descend && enter(Fc, h2, fd, own, false, (uint32_t)lv + 2u < L)) {
             if (lc) {
               if (pt.plane == 0) fr_open(Fc, u);
               __syncwarp(pt.pmask);
@@ -1230,6 +1593,16 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (budgeted && hdr[5]) {
       if (gt == 0) p.heavy[atomicAdd(p.heavy_count, 1u)] = unit;
     } else {
+      if (MODE == 1 && compact) {  // the lanes' shares: every lane of the partition gets their sum
+        if (__any_sync(pt.pmask, lacc != 0)) {
+          for (uint32_t o = 1; o < pt.P; o <<= 1) {
+            const unsigned long long lo = __shfl_xor_sync(pt.pmask, (unsigned long long)lacc, o);
+            const unsigned long long hi = __shfl_xor_sync(pt.pmask, (unsigned long long)(lacc >> 64), o);
+            lacc += ((unsigned __int128)hi << 64) | lo;
+          }
+          uacc += lacc;
+        }
+      }
       acc += uacc;
       if (LOCAL) {
         // the unit's total (its own vertices are in every one of its cliques)
@@ -1321,9 +1694,15 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   const bool pivot = lp.mode != KC_MODE_ORIENT;
   const size_t sB = (size_t)dcap * (pivot ? (W | 1u) : W);  // pivot rows use an odd stride
   // per walker: the frames, then (pivoting) the candidate list and, for local
-  // counts, the drop list
-  const size_t pstride = (size_t)depth * fw + (pivot ? al4(dcap) * (lp.local ? 2 : 1) : 0);
-  const size_t sFr = lane ? 0 : al4((size_t)nparts * pstride);
+  // counts, the drop list, else the compact bitmap of a node counted whole
+  bool compact = pivot && !lp.local && p.nk == 0;
+  const size_t sCmp = compact_words(dcap) + kPairPrefix;
+  const size_t frame_words = al4((size_t)depth * fw);
+  auto pstride_of = [&]() {
+    return frame_words + (pivot ? al4(dcap) * (lp.local ? 2 : 1) : 0) + (compact ? al4(sCmp) : 0);
+  };
+  size_t pstride = pstride_of();
+  size_t sFr = lane ? 0 : al4((size_t)nparts * pstride);
   const size_t limit_words = ((size_t)ctx->max_smem_optin - kStaticSmemBytes) / 4;
   // hash of S for the bitmap build: 2*hT words, hT the power of two >= 2 dcap
   // (load at most 1/2)
@@ -1346,6 +1725,11 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
            std::max<size_t>(frames_global ? 0 : sFr,
                             !hT ? 0 : (G == 32 ? gather_rows_at(hT) + sRow : 2 * (size_t)hT));
   };
+  if (compact && (size_t)gpb * group_words() > limit_words) {  // the frames come before the compact bitmaps
+    compact = false;
+    pstride = pstride_of();
+    sFr = al4((size_t)nparts * pstride);
+  }
   if ((size_t)gpb * group_words() > limit_words) frames_global = true;
   if ((size_t)gpb * group_words() > limit_words) bitmap_global = true;
   if ((size_t)gpb * group_words() > limit_words) hT = 0;
@@ -1358,6 +1742,8 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   p.depth = depth;
   p.fw = fw;
   p.pstride = (uint32_t)pstride;
+  p.off_cand = (uint32_t)frame_words;
+  p.compact = compact ? 1u : 0u;
   p.group_words = (uint32_t)group_words();
   p.off_R0 = (uint32_t)(hdr + sS);
   p.hash_T = hT;

@@ -34,7 +34,9 @@ struct CountParams {
   uint32_t G;                // threads per unit group (32 or blockDim.x)
   uint32_t depth;            // traversal stack frames per partition
   uint32_t fw;               // words per frame
-  uint32_t pstride;          // words per partition: depth frames, then (pivoting) a candidate list of dcap
+  uint32_t pstride;          // words per partition: depth frames, then (pivoting) a candidate list of dcap, ...
+  uint32_t off_cand;         // ... at this offset, and the compact bitmap of a node counted whole
+  uint32_t compact;          // pivoting: small nodes are counted whole
   uint32_t Q;                // pivoting: most lanes that score one candidate (0 = no bound)
   unsigned long long* local; // local counts: (lo, hi) per rank label, or null
   uint32_t off_loc;          // shared-memory offset of the per-vertex local counters (u64 each)

@@ -1,0 +1,49 @@
+"""Clique-tree nodes that the pivoting kernel counts whole: r = k - held = 3
+with up to 128 candidates and any r with up to 32, at the edges of the word
+and size ranges, with pivots already dropped (dense graphs), universal
+vertices (planted cliques), the largest r (20) and one beyond it."""
+import math
+
+import numpy as np
+import pytest
+
+import kcgpu_b200 as kc
+from oracle.oracle import OracleGraph
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(n: int, p: float, seed: int):
+    """G(n, p) with a clique planted on n // 3 of its vertices."""
+    rng = np.random.default_rng(seed)
+    a = np.triu(rng.random((n, n)) < p, 1)
+    c = rng.permutation(n)[: n // 3]
+    a[np.ix_(c, c)] = True
+    s, d = np.nonzero(np.triu(a, 1) | np.triu(a.T, 1))
+    return s.astype(np.uint32), d.astype(np.uint32), n
+
+
+@pytest.mark.parametrize("n", [6, 32, 33, 34, 64, 65, 66, 96, 97, 98, 128, 129, 130, 180])
+@pytest.mark.parametrize("p", [0.25, 0.85])
+def test_dense_graphs_match_oracle(ctx, n, p):
+    s, d, n = _dense(n, p, n)
+    og = OracleGraph(s, d, n)
+    og.orient("degen")
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degen")
+        for k in (4, 5, 6, 9):
+            if k > 6 and n > 66 and p > 0.5:
+                continue  # (the oracle's tree is large there)
+            want = og.count(k, "pivot", closed=True)
+            for mode, unit in (("pivot", "node"), ("pivot", "edge"), ("auto", "node")):
+                assert g.count(k, mode=mode, unit=unit) == want, (n, p, k, mode, unit)
+
+
+@pytest.mark.parametrize("n", [24, 33, 70, 140])
+def test_complete_graph_deep_k(ctx, n):
+    s, d = np.triu_indices(n, 1)
+    with kc.Graph.from_edges(ctx, s.astype(np.uint32), d.astype(np.uint32), n) as g:
+        g.orient("degree")
+        for k in (4, 8, 19, 20, 21, 22, 23):
+            for unit in ("node", "edge"):
+                assert g.count(k, mode="pivot", unit=unit) == math.comb(n, k), (n, k, unit)

@@ -142,160 +142,373 @@ __global__ void k_export_fill(const uint32_t* __restrict__ drp, const uint32_t* 
 }
 
 // ---- degeneracy peel: one cooperative persistent kernel -----------------------
+//
+// What bounds it is not bytes but the chain of sub-rounds (420 for R-MAT scale
+// 18, over 1,000 for a batch of 200 graphs), each a few dependent memory
+// latencies and a barrier; most hold a few vertices. So:
+//   * one barrier per sub-round: the vertices of a front are not marked as
+//     peeled before their neighbours are decremented. A peeled vertex's degree
+//     never exceeds the level, so a further decrement of it never yields
+//     level + 1 (the next front) or the end of the bucket's window, and a
+//     vertex below the level is a peeled one: no flags are kept;
+//   * one CTA of 1024 threads per SM, since a barrier costs by the CTA;
+//   * runs of small fronts (and short bucket scans) are done by one CTA alone
+//     with block barriers, the others waiting at the next grid barrier. Its
+//     edges are dealt out singly (a search in the front's length prefix);
+//   * a front is a list of row pieces of at most kPiece entries, so a hub's
+//     row (15,000 entries) is spread over many warps;
+//   * levels without vertices are skipped through the smallest degree seen.
+// R-MAT scale 18 (3.8M edges): 9.6 ms with two barriers per sub-round, flags
+// and four CTAs per SM, 3.7 ms now; scale 11 (16k edges) 0.78 ms, 0.27 ms now.
 
-constexpr uint32_t PEEL_WINDOW = 64;  // degree window of the candidate bucket
+constexpr uint32_t PEEL_WINDOW = 64;     // degree window of the candidate bucket
+constexpr uint32_t kPeelThreads = 1024;
+constexpr uint32_t kPiece = 128;         // row entries per front piece (four per lane of a warp)
+// One CTA takes a front of up to kSoloFront pieces with up to kSoloEdges
+// row entries (16 per thread: about the cost of a grid step), and bucket or
+// vertex scans of up to kSoloScan entries.
+constexpr uint32_t kSoloFront = 1024, kSoloEdges = 16384, kSoloScan = 8192;
 
 struct PeelArgs {
   const uint32_t* rp;
   const uint32_t* col;
   uint32_t n;
-  uint32_t init_prio;   // 2m: the priority the final batch keeps
-  int* deg;             // current degree among live vertices
+  int* deg;             // current degree (below the level: peeled)
   uint32_t* prio;
   uint32_t* level;
-  uint32_t* removed;    // 1 once peeled
-  uint32_t* inbucket;   // 1 while in the candidate bucket
   uint32_t* bucket_a;   // candidate bucket (ping-pong, capacity n)
   uint32_t* bucket_b;
-  uint32_t* front_a;    // frontier (ping-pong, capacity n)
-  uint32_t* front_b;
-  uint32_t* ctr;        // 4 phase slots x 4 counters, zeroed
+  uint2* front_a;       // frontier (ping-pong): [begin, end) in col of every row piece
+  uint2* front_b;
+  uint32_t* ctr;        // 4 phase slots x 4 counters, zeroed; then the solo CTA's state
+  uint32_t init_prio;   // 2m: the priority the final batch keeps
   uint32_t* out;        // [0] last level, [1] sub-rounds, [2] error
 };
+constexpr uint32_t kPeelSolo = 32;  // ctr: kPeelStateWords words left by the solo CTA
+constexpr uint32_t kPeelStateWords = 9;
 
-__global__ void k_peel_init(const uint32_t* __restrict__ rp, uint32_t n, uint32_t init_prio, int* deg,
-                            uint32_t* prio, uint32_t* level, uint32_t* removed, uint32_t* inbucket) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+__global__ void k_peel_init(const uint32_t* __restrict__ rp, uint32_t n, int* deg) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
     deg[v] = (int)(rp[v + 1] - rp[v]);
-    prio[v] = init_prio;
-    level[v] = 0;
-    removed[v] = 0;
-    inbucket[v] = 0;
-  }
 }
 
 // Appends x to list (for the lanes with pred) with one atomic per warp.
 __device__ __forceinline__ void warp_append(bool pred, uint32_t x, uint32_t* list, uint32_t* cnt) {
-  uint32_t m = __ballot_sync(0xffffffffu, pred);
+  const uint32_t m = __ballot_sync(0xffffffffu, pred);
   if (!m) return;
-  uint32_t leader = __ffs(m) - 1, base = 0;
+  const uint32_t leader = __ffs(m) - 1;
+  uint32_t base = 0;
   if (lane_id() == leader) base = atomicAdd(cnt, (uint32_t)__popc(m));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (pred) list[base + __popc(m & lanemask_lt())] = x;
 }
 
-// Every thread keeps an identical copy of the control state (level, sizes,
-// priority, phase), derived from counters read after a grid barrier, so all
-// threads take the same branches and reach the same barriers. Counters live in
-// four phase slots; a phase zeroes the slot two phases ahead, which every
-// thread has finished reading by then.
-__global__ void __launch_bounds__(256) k_peel(PeelArgs a) {
+// The lanes with pred put their vertex v into the front that sub-round
+// `priority` of level L will peel: level and priority are written now, the
+// row's pieces appended to `front` (the first kSoloFront of them to `sfront`
+// too, where there is one). cnt[0] counts pieces, cnt[1] vertices.
+__device__ __forceinline__ void front_append(const PeelArgs& a, bool pred, uint32_t v, uint32_t L, uint32_t priority,
+                                             uint2* front, uint2* sfront, uint32_t* cnt) {
+  const uint32_t m = __ballot_sync(0xffffffffu, pred);
+  if (!m) return;
+  uint32_t b = 0, e = 0, pieces = 0;
+  if (pred) {
+    b = a.rp[v];
+    e = a.rp[v + 1];
+    pieces = max(1u, (e - b + kPiece - 1u) / kPiece);  // (an isolated vertex is one empty piece)
+    a.level[v] = L;
+    a.prio[v] = priority;
+  }
+  uint32_t incl = pieces;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane_id() >= (uint32_t)o) incl += y;
+  }
+  uint32_t base = 0;
+  if (lane_id() == 31u) {
+    base = atomicAdd(&cnt[0], incl);
+    atomicAdd(&cnt[1], (uint32_t)__popc(m));
+  }
+  base = __shfl_sync(0xffffffffu, base, 31) + incl - pieces;
+  for (uint32_t i = 0; i < pieces; ++i) {
+    const uint2 pc = make_uint2(b + i * kPiece, min(e, b + (i + 1u) * kPiece));
+    front[base + i] = pc;
+    if (sfront != nullptr && base + i < kSoloFront) sfront[base + i] = pc;
+  }
+}
+
+// The control state. Every thread keeps an identical copy, derived from
+// counters read after a grid barrier (or from the state the solo CTA left), so
+// all threads take the same branches and reach the same barriers.
+struct PeelState {
+  uint32_t todo;        // vertices not yet peeled
+  uint32_t L;           // level
+  uint32_t bucket_end;  // the bucket holds the live vertices of degree in [L, bucket_end)
+  uint32_t bsize, fsize;  // bucket entries; vertices of the front
+  uint32_t pieces;        // row pieces of the front
+  uint32_t priority;    // sub-rounds done
+  uint32_t flips;       // bit 0: the bucket is in bucket_b, bit 1: the front is in front_b
+  uint32_t too_big;     // the front holds more edges than one CTA should take
+};
+
+__device__ __forceinline__ bool solo_takes(const PeelState& st, uint32_t n) {
+  if (st.fsize) return st.pieces <= kSoloFront && !st.too_big;
+  return (st.L < st.bucket_end ? st.bsize : n) <= kSoloScan;
+}
+
+// Block-wide exclusive scan of one value per thread; the total goes to *total.
+__device__ __forceinline__ uint32_t peel_scan(uint32_t v, uint32_t* wsum, uint32_t* total) {
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  if (lane == 31) wsum[w] = incl;
+  __syncthreads();
+  const uint32_t s = lane < kPeelThreads / 32 ? wsum[lane] : 0u;
+  uint32_t si = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, si, o);
+    if (lane >= (uint32_t)o) si += y;
+  }
+  *total = __shfl_sync(0xffffffffu, si, 31);
+  return incl - v + __shfl_sync(0xffffffffu, si - s, w);
+}
+
+// One CTA peels alone for as long as the next step is small (it takes at
+// least one step). Counters live in shared memory; lists in global memory.
+__device__ void peel_solo(const PeelArgs& a, PeelState& st) {
+  __shared__ uint32_t pre[kSoloFront], beg[kSoloFront], wsum[kPeelThreads / 32];
+  __shared__ uint2 sfront[kSoloFront];
+  __shared__ uint32_t cn[2], cb, cmin;  // next front (pieces, vertices), bucket, smallest degree above the level (complemented)
+  const uint32_t tid = threadIdx.x;
+  bool in_shared = false;  // the front is in sfront
+  while (st.todo > 0 && solo_takes(st, a.n)) {
+    uint32_t* bucket = (st.flips & 1u) ? a.bucket_b : a.bucket_a;
+    uint32_t* bucket2 = (st.flips & 1u) ? a.bucket_a : a.bucket_b;
+    uint2* front = (st.flips & 2u) ? a.front_b : a.front_a;
+    uint2* next = (st.flips & 2u) ? a.front_a : a.front_b;
+    if (tid == 0) { cn[0] = cn[1] = 0; cb = st.fsize ? st.bsize : 0u; cmin = 0; }
+    if (st.fsize) {  // a sub-round
+      if (st.fsize == st.todo) {  // the final batch
+        st.todo = 0;
+        break;
+      }
+      uint32_t len = 0, total = 0;
+      if (tid < st.pieces) {
+        const uint2 pc = in_shared ? sfront[tid] : front[tid];
+        beg[tid] = pc.x;
+        len = pc.y - pc.x;
+      }
+      const uint32_t ex = peel_scan(len, wsum, &total);
+      if (tid < st.pieces) pre[tid] = ex;
+      if (total > kSoloEdges) {
+        st.too_big = 1u;
+        __syncthreads();
+        return;
+      }
+      st.todo -= st.fsize;
+      __syncthreads();
+      uint32_t top = 1;
+      while (top < st.pieces) top <<= 1;
+      constexpr uint32_t kU = 8;  // edges in flight per thread
+      for (uint32_t i0 = 0; i0 < total; i0 += kU * kPeelThreads) {
+        uint32_t u[kU];
+        int cur[kU];
+#pragma unroll
+        for (uint32_t q = 0; q < kU; ++q) {
+          const uint32_t i = i0 + q * kPeelThreads + tid;
+          u[q] = 0xffffffffu;
+          if (i < total) {
+            uint32_t j = 0;  // the last piece with pre[j] <= i
+            for (uint32_t s = top >> 1; s; s >>= 1)
+              if (j + s < st.pieces && pre[j + s] <= i) j += s;
+            u[q] = a.col[beg[j] + (i - pre[j])];
+          }
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kU; ++q) cur[q] = u[q] != 0xffffffffu ? atomicSub(&a.deg[u[q]], 1) : -1;
+#pragma unroll
+        for (uint32_t q = 0; q < kU; ++q) {
+          if (i0 + q * kPeelThreads >= total) break;
+          const bool to_next = cur[q] == (int)st.L + 1;
+          front_append(a, to_next, u[q], st.L, st.priority + 1u, next, sfront, cn);
+          warp_append(!to_next && cur[q] == (int)st.bucket_end, u[q], bucket, &cb);
+        }
+      }
+      __syncthreads();
+      st.fsize = min(cn[1], a.n);
+      st.pieces = cn[0];
+      st.bsize = min(cb, a.n);
+      st.flips ^= 2u;
+      ++st.priority;
+      in_shared = true;
+      if (st.fsize == 0) ++st.L;
+    } else if (st.L < st.bucket_end) {  // the bucket's vertices at this level
+      in_shared = true;
+      __syncthreads();
+      uint32_t mn = 0;
+      for (uint32_t i0 = 0; i0 < st.bsize; i0 += kPeelThreads) {
+        const uint32_t i = i0 + tid;
+        const uint32_t v = i < st.bsize ? bucket[i] : 0u;
+        const int d = i < st.bsize ? __ldcg(a.deg + v) : -1;
+        front_append(a, d == (int)st.L, v, st.L, st.priority, front, sfront, cn);
+        warp_append(d > (int)st.L, v, bucket2, &cb);
+        if (d > (int)st.L) mn = max(mn, ~(uint32_t)d);
+      }
+      mn = __reduce_max_sync(0xffffffffu, mn);
+      if (lane_id() == 0 && mn) atomicMax(&cmin, mn);
+      __syncthreads();
+      st.fsize = min(cn[1], a.n);
+      st.pieces = cn[0];
+      st.bsize = min(cb, a.n);
+      st.flips ^= 1u;
+      if (st.fsize == 0) st.L = cmin ? min(~cmin, st.bucket_end) : st.bucket_end;
+    } else {  // a new window
+      __syncthreads();
+      uint32_t mn = 0;
+      for (uint32_t v0 = 0; v0 < a.n; v0 += kPeelThreads) {
+        const uint32_t v = v0 + tid;
+        const int d = v < a.n ? __ldcg(a.deg + v) : -1;
+        warp_append(d >= (int)st.L && d < (int)(st.L + PEEL_WINDOW), v, bucket, &cb);
+        if (d >= (int)st.L) mn = max(mn, ~(uint32_t)d);
+      }
+      mn = __reduce_max_sync(0xffffffffu, mn);
+      if (lane_id() == 0 && mn) atomicMax(&cmin, mn);
+      __syncthreads();
+      st.bsize = min(cb, a.n);
+      if (cmin == 0u) {  // no live vertex left, todo > 0: cannot happen for a valid CSR
+        if (tid == 0) a.out[2] = DEV_ERR_INPUT;
+        st.todo = 0;
+        break;
+      }
+      if (st.bsize == 0) st.L = ~cmin;  // every live vertex lies above the window
+      else st.bucket_end = st.L + PEEL_WINDOW;
+      if (st.bsize == 0) st.bucket_end = st.L;
+    }
+    st.too_big = 0;
+    __syncthreads();  // the counters are read before they are set again
+  }
+}
+
+__global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
   cg::grid_group grid = cg::this_grid();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t nthreads = gridDim.x * blockDim.x;
   const uint32_t lane = lane_id();
-  const uint32_t gw = tid >> 5, nw = nthreads >> 5;
-  uint32_t* bucket = a.bucket_a;
-  uint32_t* bucket2 = a.bucket_b;
-  uint32_t* front = a.front_a;
-  uint32_t* next = a.front_b;
-  uint64_t todo = a.n;
-  uint32_t L = 0, bucket_end = 0, bsize = 0, priority = 0, phase = 0, subrounds = 0;
+  const uint32_t gw = tid >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  PeelState st = {a.n, 0, 0, 0, 0, 0, 0, 0, 0};
+  // Counters live in four phase slots; a phase zeroes the slot two phases
+  // ahead, which every thread has finished reading by then.
+  uint32_t phase = 0;
   auto slot = [&](uint32_t ph) { return a.ctr + (ph & 3u) * 4u; };
-  auto begin_phase = [&]() {
+  while (st.todo > 0) {
+    if (solo_takes(st, a.n)) {
+      if (blockIdx.x == 0) {
+        peel_solo(a, st);
+        if (tid == 0) {
+          uint32_t* o = a.ctr + kPeelSolo;
+          o[0] = st.todo; o[1] = st.L; o[2] = st.bucket_end; o[3] = st.bsize;
+          o[4] = st.fsize; o[5] = st.pieces; o[6] = st.priority; o[7] = st.flips; o[8] = st.too_big;
+        }
+      }
+      grid.sync();
+      const uint32_t* o = a.ctr + kPeelSolo;
+      st = {__ldcg(o),     __ldcg(o + 1), __ldcg(o + 2), __ldcg(o + 3), __ldcg(o + 4),
+            __ldcg(o + 5), __ldcg(o + 6), __ldcg(o + 7), __ldcg(o + 8)};
+      continue;  // (the next step is a grid step, whose barrier comes before the state is written again)
+    }
+    uint32_t* bucket = (st.flips & 1u) ? a.bucket_b : a.bucket_a;
+    uint32_t* bucket2 = (st.flips & 1u) ? a.bucket_a : a.bucket_b;
+    uint2* front = (st.flips & 2u) ? a.front_b : a.front_a;
+    uint2* next = (st.flips & 2u) ? a.front_a : a.front_b;
     if (tid == 0) {
       uint32_t* z = slot(phase + 2);
       z[0] = z[1] = z[2] = z[3] = 0;
     }
-  };
-  while (todo > 0) {
-    if (L > a.n) {  // cannot happen for a valid CSR; never spin
-      if (tid == 0) a.out[2] = DEV_ERR_INPUT;
-      break;
-    }
-    if (L == bucket_end) {
-      begin_phase();
-      uint32_t* c = slot(phase);
+    uint32_t* c = slot(phase++);  // front pieces, front vertices, bucket, smallest degree (complemented)
+    st.too_big = 0;
+    if (st.fsize) {  // a sub-round
+      const bool last = st.fsize == st.todo;  // the final batch
+      st.todo -= st.fsize;
+      if (last) break;
+      for (uint32_t i = gw; i < st.pieces; i += nw) {
+        const uint2 pc = front[i];
+        uint32_t u[kPiece / 32u];
+        int cur[kPiece / 32u];
+#pragma unroll
+        for (uint32_t q = 0; q < kPiece / 32u; ++q) {
+          const uint32_t j = pc.x + q * 32u + lane;
+          u[q] = j < pc.y ? a.col[j] : 0xffffffffu;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kPiece / 32u; ++q) cur[q] = u[q] != 0xffffffffu ? atomicSub(&a.deg[u[q]], 1) : -1;
+#pragma unroll
+        for (uint32_t q = 0; q < kPiece / 32u; ++q) {
+          const bool to_next = cur[q] == (int)st.L + 1;
+          front_append(a, to_next, u[q], st.L, st.priority + 1u, next, nullptr, c);
+          warp_append(!to_next && cur[q] == (int)st.bucket_end, u[q], bucket + st.bsize, &c[2]);
+        }
+      }
+      grid.sync();
+      st.pieces = __ldcg(c);
+      st.fsize = min(__ldcg(c + 1), a.n);
+      st.bsize = min(st.bsize + __ldcg(c + 2), a.n);
+      st.flips ^= 2u;
+      ++st.priority;
+      if (st.fsize == 0) ++st.L;
+    } else if (st.L < st.bucket_end) {  // the bucket's vertices at this level, and the bucket compacted
+      uint32_t mn = 0;
+      for (uint32_t i0 = gw * 32; i0 < st.bsize; i0 += nw * 32) {
+        const uint32_t i = i0 + lane;
+        const uint32_t v = i < st.bsize ? bucket[i] : 0u;
+        const int d = i < st.bsize ? __ldcg(a.deg + v) : -1;
+        front_append(a, d == (int)st.L, v, st.L, st.priority, front, nullptr, c);
+        warp_append(d > (int)st.L, v, bucket2, &c[2]);
+        if (d > (int)st.L) mn = max(mn, ~(uint32_t)d);
+      }
+      mn = __reduce_max_sync(0xffffffffu, mn);
+      if (lane == 0 && mn) atomicMax(&c[3], mn);
+      grid.sync();
+      st.pieces = __ldcg(c);
+      st.fsize = min(__ldcg(c + 1), a.n);
+      st.bsize = min(__ldcg(c + 2), a.n);
+      st.flips ^= 1u;
+      const uint32_t m = __ldcg(c + 3);
+      if (st.fsize == 0) st.L = m ? min(~m, st.bucket_end) : st.bucket_end;
+    } else {  // a new window
+      uint32_t mn = 0;
       for (uint32_t v0 = gw * 32; v0 < a.n; v0 += nw * 32) {
-        uint32_t v = v0 + lane;
-        bool in = false;
-        if (v < a.n && !a.removed[v]) {
-          int d = a.deg[v];
-          in = d >= (int)L && d < (int)(L + PEEL_WINDOW);
-          a.inbucket[v] = in ? 1u : 0u;
-        }
-        warp_append(in, v, bucket, &c[0]);
+        const uint32_t v = v0 + lane;
+        const int d = v < a.n ? __ldcg(a.deg + v) : -1;
+        warp_append(d >= (int)st.L && d < (int)(st.L + PEEL_WINDOW), v, bucket, &c[2]);
+        if (d >= (int)st.L) mn = max(mn, ~(uint32_t)d);
       }
+      mn = __reduce_max_sync(0xffffffffu, mn);
+      if (lane == 0 && mn) atomicMax(&c[3], mn);
       grid.sync();
-      bsize = min(c[0], a.n);
-      bucket_end = L + PEEL_WINDOW;
-      ++phase;
-    }
-    // frontier of level L, and compaction of the bucket
-    begin_phase();
-    uint32_t* c = slot(phase);
-    for (uint32_t i0 = gw * 32; i0 < bsize; i0 += nw * 32) {
-      uint32_t i = i0 + lane;
-      uint32_t v = i < bsize ? bucket[i] : 0;
-      bool live = i < bsize && !a.removed[v];
-      int d = live ? a.deg[v] : 0;
-      warp_append(live && d == (int)L, v, front, &c[0]);
-      warp_append(live && d != (int)L, v, bucket2, &c[1]);
-    }
-    grid.sync();
-    uint32_t fsize = min(c[0], a.n);
-    bsize = min(c[1], a.n);
-    { uint32_t* t = bucket; bucket = bucket2; bucket2 = t; }
-    ++phase;
-    while (fsize > 0) {
-      todo -= fsize;
-      for (uint32_t i = tid; i < fsize; i += nthreads) a.level[front[i]] = L;
-      if (todo == 0) break;  // the final batch keeps its initial priority
-      for (uint32_t i = tid; i < fsize; i += nthreads) {
-        a.prio[front[i]] = priority;
-        a.removed[front[i]] = 1u;
+      st.bsize = min(__ldcg(c + 2), a.n);
+      const uint32_t m = __ldcg(c + 3);
+      if (m == 0u) {  // no live vertex left, todo > 0: cannot happen for a valid CSR; never spin
+        if (tid == 0) a.out[2] = DEV_ERR_INPUT;
+        break;
       }
-      begin_phase();
-      grid.sync();
-      uint32_t* c2 = slot(phase);
-      for (uint32_t i = gw; i < fsize; i += nw) {
-        const uint32_t v = front[i];
-        const uint32_t b = a.rp[v], e = a.rp[v + 1];
-        for (uint32_t j0 = b; j0 < e; j0 += 32) {
-          uint32_t j = j0 + lane;
-          bool to_next = false, to_bucket = false;
-          uint32_t u = 0;
-          if (j < e) {
-            u = a.col[j];
-            if (!a.removed[u]) {
-              int cur = atomicSub(&a.deg[u], 1);
-              if (cur == (int)L + 1) {
-                to_next = true;
-              } else {
-                int now = cur - 1;
-                if (now > (int)L && now < (int)bucket_end) to_bucket = atomicExch(&a.inbucket[u], 1u) == 0u;
-              }
-            }
-          }
-          warp_append(to_next, u, next, &c2[0]);
-          warp_append(to_bucket, u, bucket + bsize, &c2[1]);
-        }
-      }
-      grid.sync();
-      fsize = min(c2[0], a.n);
-      bsize = min(bsize + c2[1], a.n);
-      { uint32_t* t = front; front = next; next = t; }
-      ++priority;
-      ++subrounds;
-      ++phase;
+      if (st.bsize == 0) st.L = ~m;  // every live vertex lies above the window
+      st.bucket_end = st.bsize == 0 ? st.L : st.L + PEEL_WINDOW;
     }
-    if (todo == 0) break;
-    ++L;
   }
   if (tid == 0) {
-    a.out[0] = L;
-    a.out[1] = subrounds;
+    a.out[0] = st.L;
+    a.out[1] = st.priority;
   }
+  // the final batch keeps its initial priority (every vertex has been put in
+  // a front, and what any CTA wrote there was ordered by the last barrier)
+  grid.sync();
+  for (uint32_t v = tid; v < a.n; v += nw * 32u)
+    if (__ldcg(a.prio + v) == st.priority) a.prio[v] = a.init_prio;
 }
 
 }  // namespace
@@ -309,29 +522,30 @@ kc_status run_peel(kc_graph* g, uint32_t* prio, uint32_t* level) {
   const uint32_t n = g->n;
   DevTemps t(s);
   int* deg = nullptr;
-  uint32_t *removed = nullptr, *inb = nullptr, *ba = nullptr, *bb = nullptr, *fa = nullptr, *fb = nullptr,
-           *ctr = nullptr;
+  uint32_t *ba = nullptr, *bb = nullptr, *ctr = nullptr;
+  uint2 *fa = nullptr, *fb = nullptr;
+  // a front holds at most every vertex: n pieces and one more per kPiece entries
+  const size_t front_cap = (size_t)n + 2 * g->m / kPiece;
   KC_CUDA(t.alloc(&deg, sizeof(int) * n));
-  KC_CUDA(t.alloc(&removed, sizeof(uint32_t) * n));
-  KC_CUDA(t.alloc(&inb, sizeof(uint32_t) * n));
   KC_CUDA(t.alloc(&ba, sizeof(uint32_t) * n));
   KC_CUDA(t.alloc(&bb, sizeof(uint32_t) * n));
-  KC_CUDA(t.alloc(&fa, sizeof(uint32_t) * n));
-  KC_CUDA(t.alloc(&fb, sizeof(uint32_t) * n));
-  KC_CUDA(t.alloc(&ctr, sizeof(uint32_t) * 32));
-  KC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 32, s));
+  KC_CUDA(t.alloc(&fa, sizeof(uint2) * front_cap));
+  KC_CUDA(t.alloc(&fb, sizeof(uint2) * front_cap));
+  constexpr uint32_t kCtrWords = kPeelSolo + kPeelStateWords;
+  KC_CUDA(t.alloc(&ctr, sizeof(uint32_t) * kCtrWords));
+  KC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrWords, s));
   const uint32_t init_prio = (uint32_t)std::min<uint64_t>(2 * g->m, 0xffffffffull);
-  k_peel_init<<<grid_for(n, ctx->sms), 256, 0, s>>>(g->rp, n, init_prio, deg, prio, level, removed, inb);
+  k_peel_init<<<grid_for(n, ctx->sms), 256, 0, s>>>(g->rp, n, deg);
   KC_CUDA(cudaGetLastError());
 
   PeelArgs a;
-  a.rp = g->rp; a.col = g->col; a.n = n; a.init_prio = init_prio;
-  a.deg = deg; a.prio = prio; a.level = level; a.removed = removed; a.inbucket = inb;
+  a.rp = g->rp; a.col = g->col; a.n = n; a.deg = deg; a.prio = prio; a.level = level;
   a.bucket_a = ba; a.bucket_b = bb; a.front_a = fa; a.front_b = fb; a.ctr = ctr; a.out = ctr + 16;
-  int per_sm = 0;
-  KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel, 256, 0));
-  per_sm = std::max(1, std::min(per_sm, 4));
-  dim3 grid(ctx->sms * per_sm), block(256);
+  a.init_prio = init_prio;
+  // at most one CTA per SM, each with enough vertices or row entries to be
+  // worth a barrier's arrival (a small graph is peeled by one CTA alone)
+  const uint64_t want = std::max<uint64_t>(ceil_div<uint64_t>(n, kSoloScan), ceil_div<uint64_t>(2 * g->m, kSoloEdges));
+  dim3 grid((uint32_t)std::min<uint64_t>((uint64_t)ctx->sms, std::max<uint64_t>(1, want))), block(kPeelThreads);
   void* args[] = {&a};
   KC_CUDA(cudaLaunchCooperativeKernel((void*)k_peel, grid, block, args, 0, s));
   uint32_t out[3] = {0, 0, 0};

@@ -348,6 +348,9 @@ constexpr uint32_t kTriangleMax = 128; // most candidates of an r = 3 node close
 constexpr uint32_t kSmallMax = 32;     // most candidates of an r > 3 node closed whole
 constexpr int kSmallStack = 16;        // close_small: pushed frames (r - 5 at most)
 constexpr uint32_t kSmallMaxR = 20;
+// several k: the largest r closed whole, and the words of its histogram
+constexpr uint32_t kSmallMaxRMulti = 15;
+constexpr uint32_t kHistWords = (kSmallMaxRMulti + 1u) * (kSmallMax + 1u);
 
 // r = 3: triangles + drop edges + C(drop, 2) vertices + C(drop, 3). Every lane
 // returns its share.
@@ -384,9 +387,23 @@ __device__ __forceinline__ unsigned __int128 binom_at(const unsigned long long* 
 // listing, above that by pivoting. Vertices adjacent to the whole set are
 // moved to the pivots at once (their branches are empty). Returns the lane's
 // share; pre[32] receives the most rows any lane visited.
+//
+// MK (several k in one walk): nothing is known of the smaller k, so instead of
+// binomials of one k the lanes count, in hist[h (kSmallMax + 1) + x], the
+// cliques of F by the h vertices they hold and the x pivots of F that may join
+// them: each stands for C(drop + x, k - held - h) cliques of every k. r belongs
+// to the largest k; the closed forms for r <= 3 hold for every smaller k too.
+// R-MAT of 55k edges, k = 3..15 in one walk: 11.5 ms with every node walked,
+// 4.2 ms now.
+template <bool MK>
 __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, uint32_t* pre, uint32_t nc, uint32_t r,
-                                                      uint32_t drop, const unsigned long long* binom, uint32_t cols) {
+                                                         uint32_t drop, const unsigned long long* binom, uint32_t cols,
+                                                         uint32_t* hist) {
   const uint32_t lane = lane_id();
+  auto leaf = [&](uint32_t held, uint32_t dd, uint32_t times) {
+    if (times && KC_IN_BOUNDS(held * (kSmallMax + 1u) + (dd - drop), kHistWords, nullptr))
+      atomicAdd(&hist[held * (kSmallMax + 1u) + (dd - drop)], times);
+  };
   const uint32_t mine = lane < nc ? adj[lane] & (0xfffffffeu << lane) : 0u;
   const uint32_t c = __popc(mine);
   uint32_t incl = c;
@@ -398,7 +415,9 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
   pre[lane] = incl - c;
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
   unsigned __int128 acc = 0;
-  if (lane == 0) {
+  if (MK) {
+    for (uint32_t i = lane; i < (r + 1u) * (kSmallMax + 1u); i += 32u) hist[i] = i == 0u ? 1u : (i == kSmallMax + 1u ? nc : 0u);
+  } else if (lane == 0) {
     acc = binom_at(binom, cols, drop, r);
     if (drop + 1u >= r) acc += (unsigned __int128)nc * binom_at(binom, cols, drop, r - 1u);
   }
@@ -418,11 +437,17 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
     for (;;) {
       // the node (P, rr, dd)
       const uint32_t n = __popc(P);
-      if (n + dd >= rr) {
+      if (MK || n + dd >= rr) {
         if (n == 0u) {
-          acc += binom_at(binom, cols, dd, rr);
+          if (MK) leaf(r - rr, dd, 1u);
+          else acc += binom_at(binom, cols, dd, rr);
         } else if (rr == 1u) {
-          acc += n + dd;
+          if (MK) {
+            leaf(r - rr, dd, 1u);
+            leaf(r - rr + 1u, dd, n);
+          } else {
+            acc += n + dd;
+          }
         } else if (rr <= 3u) {
           uint32_t e = 0, tri = 0;
           for (uint32_t x = P; x; x &= x - 1u) {
@@ -437,7 +462,12 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
               }
           }
           const unsigned long long d1 = dd, d2 = d1 * (d1 - 1ull) / 2ull;  // (0 for dd = 0)
-          if (rr == 2u) {
+          if (MK) {
+            leaf(r - rr, dd, 1u);
+            leaf(r - rr + 1u, dd, n);
+            leaf(r - rr + 2u, dd, e);
+            if (rr == 3u) leaf(r, dd, tri);
+          } else if (rr == 2u) {
             acc += e + d1 * n + (dd >= 2u ? d2 : 0ull);
           } else {
             acc += tri + d1 * e + (dd >= 2u ? d2 * n : 0ull) + (dd >= 3u ? d2 * (d1 - 2ull) / 3ull : 0ull);
@@ -454,7 +484,8 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
           dd += __popc(uni);
           P &= ~uni;
           if (P == 0u) {
-            acc += binom_at(binom, cols, dd, rr);
+            if (MK) leaf(r - rr, dd, 1u);
+            else acc += binom_at(binom, cols, dd, rr);
           } else if (KC_IN_BOUNDS(lv, kSmallStack, nullptr)) {
             const uint32_t piv = best & 0xffffu;
             sP[lv] = P;
@@ -500,7 +531,7 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
   uint32_t cost = 1u + (nc >> 5);
   if (r > 3u) {
     if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
-    t = close_small(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols);
+    t = close_small<false>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols, nullptr);
     __syncwarp();
     cost = 1u + (cmp[kPairPrefix + 32u] >> 5);
   } else if (nc <= 32u) {
@@ -518,9 +549,38 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
   return t;
 }
 
+// close_node for several k at once (nc <= 32, r <= kSmallMaxRMulti for the
+// largest k): the lane's own k has kr = k - held vertices to go (`open`: it is
+// still to be counted), and its whole count below the node is returned.
+__device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
+                                                           uint32_t nc, uint32_t* cmp, uint32_t r, uint32_t drop,
+                                                           const unsigned long long* binom, uint32_t cols,
+                                                           uint32_t kr, bool open) {
+  const uint32_t lane = lane_id();
+  uint32_t* hist = cmp + 2u * kPairPrefix;
+  if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
+  close_small<true>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols, hist);
+  __syncwarp();
+  unsigned __int128 t = 0;
+  const uint32_t words = (r + 1u) * (kSmallMax + 1u);
+  for (uint32_t i0 = 0; i0 < words; i0 += 32u) {
+    const uint32_t mine = i0 + lane < words ? hist[i0 + lane] : 0u;
+    for (uint32_t m = __ballot_sync(0xffffffffu, mine != 0u); m; m &= m - 1u) {
+      const uint32_t b = (uint32_t)__ffs(m) - 1u;
+      const uint32_t times = __shfl_sync(0xffffffffu, mine, b);
+      const uint32_t h = (i0 + b) / (kSmallMax + 1u), x = (i0 + b) - h * (kSmallMax + 1u);
+      if (open && kr >= h) t += (unsigned __int128)times * binom_at(binom, cols, drop + x, kr - h);
+    }
+  }
+  if (lane == 0) cmp[0] = 1u + (cmp[kPairPrefix + 32u] >> 5);
+  __syncwarp();
+  return t;
+}
+
 // Register budgets: orientation fits 56 registers without spills (four
 // 256-thread CTAs per SM); pivoting needs 80 (three), spilling below that.
-template <int MODE, bool LOCAL>
+// MK: several k in one walk (pivoting, one graph).
+template <int MODE, bool LOCAL, bool MK>
 __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountParams p) {
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t G = p.G;
@@ -535,7 +595,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   pt.pbase = (lane / p.P) * p.P;
   pt.pmask = p.P >= 32 ? 0xffffffffu : (((1u << p.P) - 1u) << pt.pbase);
   const uint32_t part = gt / p.P;
-  // Several k in one walk (pivoting, one graph, p.nk > 0): the walk goes to
+  // Several k in one walk (MK, p.nk of them): the walk goes to
   // the largest k, and lane `plane` of every partition keeps the count of
   // kset[plane]. A clique-tree node with `hold` held vertices, `drop` pivots
   // and candidate set C adds sum_j C(drop, j) cliques(G[C], k - hold - j);
@@ -544,7 +604,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // below a non-pivot step from a parent with k - hold = 3 is where k - hold
   // first reaches 2. A k that is still open at a leaf (no candidates) adds
   // C(drop, k - hold) there.
-  const bool mk = MODE == 1 && !LOCAL && p.nk != 0u;
+  constexpr bool mk = MK;
   const bool kon = mk && pt.plane < p.nk;
   const uint32_t kl = kon ? p.kset[pt.plane] : 0u;
 
@@ -557,7 +617,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   uint32_t* frames = (p.frames_global ? gb + p.goff_fr : sb + p.off_fr) + (size_t)part * p.pstride;
   uint32_t* cand = frames + p.off_cand;  // pivoting: the candidates of the node being entered
   // pivoting: the compact bitmap of a node counted whole (then its prefix table)
-  const bool compact = MODE == 1 && !LOCAL && p.compact != 0u && p.nk == 0u;
+  const bool compact = MODE == 1 && !LOCAL && p.compact != 0u;
   uint32_t* cmp = cand + ((p.dcap + 3u) & ~3u);
   // open-addressing hash of S: vertex -> local index (linear probing, load <= 1/2)
   const uint32_t hT = p.hash_T;
@@ -1168,15 +1228,18 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           }
         }
       }
-    } else if (MODE == 1 && compact && (d <= kSmallMax || (d <= kTriangleMax && k == (p.edge_units ? 5u : 4u))) &&
-               k <= kSmallMaxR) {
+    } else if (MODE == 1 && compact && (d <= kSmallMax || (!mk && d <= kTriangleMax && k == (p.edge_units ? 5u : 4u))) &&
+               k <= (mk ? kSmallMaxRMulti : kSmallMaxR)) {
       // ---- a unit counted whole (edge roots: their sum is the unit's count)
       const uint32_t r = k - (p.edge_units ? 2u : 1u);  // >= 3 here
       if (part == 0 && !helper) {
         st_nodes++;
         for (uint32_t i = pt.plane; i < d; i += 32u) cand[i] = i;
         __syncwarp();
-        lacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
+        if constexpr (MK)  // the k with k - hold0 <= 2 are closed already
+          uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r), kon && kl + r >= k + 3u);
+        else
+          lacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
         st_words += 32u * cmp[0];
       }
     } else {
@@ -1290,7 +1353,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         leaf_pinc = 0;
         // several k: this lane's k is still open here if its k - hold was
         // at least 3 at the parent
-        const bool kopen = kon && kl + (pchild ? 0u : 1u) >= hold + 3u;
+        bool kopen = kon && kl + (pchild ? 0u : 1u) >= hold + 3u;
         if (nc == 0u) {
           leaf_cnt = binom(drop, r);
           if (r >= 1u && drop >= 1u) leaf_pinc = binom(drop - 1u, r - 1u);
@@ -1309,7 +1372,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         }
         // a small node is counted whole: the walker that owns it copies G[F]
         // and counts it (see close_triangles and close_small)
-        auto small = [&](uint32_t n) { return compact && r >= 3u && n <= (r == 3u ? kTriangleMax : kSmallMax) && r <= kSmallMaxR; };
+        auto small = [&](uint32_t n) {
+          return compact && r >= 3u && n <= (!mk && r == 3u ? kTriangleMax : kSmallMax) &&
+                 r <= (mk ? kSmallMaxRMulti : kSmallMaxR);
+        };
         bool whole = small(nc);
         if (whole && !(above ? claim() : own)) return false;
         uint32_t best = 0, nw = 0;
@@ -1340,7 +1406,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         __syncwarp(pt.pmask);
         nw = narrow ? (uint32_t)__popc(nzm) : W;
         if (whole) {
-          lacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
+          if constexpr (MK)
+            uacc += close_node_multi(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols, kl - hold, kopen);
+          else
+            lacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
           const uint32_t cost = cmp[0];
           since_charge += cost;
           st_words += 32u * cost;
@@ -1395,8 +1464,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           return false;
         }
         // several k: a smaller k that reaches k - hold = 2 here is closed here
-        if (mk && own && kopen && kl == hold + 2u)
-          uacc += (unsigned __int128)(esum / 2u) + (unsigned __int128)drop * nc + binom(drop, 2u);
+        if (mk && kopen && kl == hold + 2u) {
+          if (own) uacc += (unsigned __int128)(esum / 2u) + (unsigned __int128)drop * nc + binom(drop, 2u);
+          kopen = false;
+        }
         if (univ && __any_sync(pt.pmask, um != 0u)) {
           const uint32_t nu = __reduce_add_sync(pt.pmask, (uint32_t)__popc(um));
           for (uint32_t x = um; x; x &= x - 1u) {
@@ -1408,7 +1479,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           nc -= nu;
           if (nc == 0u) {  // F was a clique: a leaf with all of it as pivots
             leaf_cnt = binom(drop, r);
-            if (own) uacc += mk ? ((kopen && kl >= hold + 3u) ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
+            if (own) uacc += mk ? (kopen ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
             return false;
           }
           if (narrow) nzm = __ballot_sync(pt.pmask, pt.plane < W && F[pt.plane] != 0u);
@@ -1593,7 +1664,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (budgeted && hdr[5]) {
       if (gt == 0) p.heavy[atomicAdd(p.heavy_count, 1u)] = unit;
     } else {
-      if (MODE == 1 && compact) {  // the lanes' shares: every lane of the partition gets their sum
+      if (MODE == 1 && !MK && compact) {  // the lanes' shares: every lane of the partition gets their sum
         if (__any_sync(pt.pmask, lacc != 0)) {
           for (uint32_t o = 1; o < pt.P; o <<= 1) {
             const unsigned long long lo = __shfl_xor_sync(pt.pmask, (unsigned long long)lacc, o);
@@ -1695,8 +1766,9 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   const size_t sB = (size_t)dcap * (pivot ? (W | 1u) : W);  // pivot rows use an odd stride
   // per walker: the frames, then (pivoting) the candidate list and, for local
   // counts, the drop list, else the compact bitmap of a node counted whole
-  bool compact = pivot && !lp.local && p.nk == 0;
-  const size_t sCmp = compact_words(dcap) + kPairPrefix;
+  const bool mk = pivot && p.nk != 0;
+  bool compact = pivot && !lp.local;
+  const size_t sCmp = mk ? 2 * kPairPrefix + kHistWords : compact_words(dcap) + kPairPrefix;
   const size_t frame_words = al4((size_t)depth * fw);
   auto pstride_of = [&]() {
     return frame_words + (pivot ? al4(dcap) * (lp.local ? 2 : 1) : 0) + (compact ? al4(sCmp) : 0);
@@ -1759,8 +1831,9 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   p.gbuf = nullptr;
 
   const size_t smem_bytes = (size_t)gpb * p.group_words * 4;
-  auto kern = lp.mode == KC_MODE_ORIENT ? (lp.local ? k_count_bitmap<0, true> : k_count_bitmap<0, false>)
-                                         : (lp.local ? k_count_bitmap<1, true> : k_count_bitmap<1, false>);
+  auto kern = !pivot ? (lp.local ? k_count_bitmap<0, true, false> : k_count_bitmap<0, false, false>)
+              : lp.local ? k_count_bitmap<1, true, false>
+              : mk ? k_count_bitmap<1, false, true> : k_count_bitmap<1, false, false>;
   // Several classes launch the same kernel with different shared-memory sizes;
   // the attribute is per function, so it is set to the device maximum.
   // (the kernel's static shared memory counts against the same per-block limit)

@@ -47,3 +47,24 @@ def test_complete_graph_deep_k(ctx, n):
         for k in (4, 8, 19, 20, 21, 22, 23):
             for unit in ("node", "edge"):
                 assert g.count(k, mode="pivot", unit=unit) == math.comb(n, k), (n, k, unit)
+
+
+@pytest.mark.parametrize("n", [6, 32, 33, 34, 66, 97])
+@pytest.mark.parametrize("p", [0.25, 0.85])
+def test_several_k(ctx, n, p):
+    s, d, n = _dense(n, p, n + 1)
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degen")
+        for ks in ([3, 4, 5], list(range(3, 10)), [4, 16], [5, 17, 6]):
+            want = [g.count(k, mode="pivot") for k in ks]
+            for unit in ("node", "edge"):
+                assert g.count_multi(ks, unit=unit) == want, (n, p, ks, unit)
+
+
+@pytest.mark.parametrize("n", [24, 33, 70, 140])
+def test_several_k_complete_graph(ctx, n):
+    s, d = np.triu_indices(n, 1)
+    with kc.Graph.from_edges(ctx, s.astype(np.uint32), d.astype(np.uint32), n) as g:
+        g.orient("degree")
+        for ks in (list(range(3, 17)), list(range(3, 34)), [15, 18]):
+            assert g.count_multi(ks) == [math.comb(n, k) for k in ks], (n, ks)

@@ -26,6 +26,7 @@
 //   * edge units are grouped by source when N+(u) fits a shared-memory bitmap:
 //     the unit u builds G[N+(u)] once and its out-edges are the root branches.
 #include <algorithm>
+#include <type_traits>
 
 #include "count_kernels.cuh"
 #include "dev_common.cuh"
@@ -65,15 +66,16 @@ __device__ __forceinline__ uint32_t valid_mask(uint32_t d, uint32_t w) {  // bit
 }
 
 constexpr int kLaneStack = 16;  // lane-DFS levels: t - 2 <= 16, i.e. k <= 19 (node units)
-constexpr uint32_t kGatherRun = 8;    // warp gather: consecutive out-list words per lane per iteration
-constexpr uint32_t kSpanWords = 256;  // warp gather: membership map of up to 8192 rank labels
-
-// Offset (words) of a warp unit's gather row table inside the hash / map
-// region, which holds the hash (2 hT words) or the membership map and its
-// prefix (2 kSpanWords words).
-__host__ __device__ constexpr uint32_t gather_rows_at(uint32_t hT) {
-  return hT > kSpanWords ? 2u * hT : 2u * kSpanWords;
+// Gather tables (shared memory, needed until the bitmap stands): the member
+// map of up to kSpanWords * 32 rank labels with its prefix, or, for a wider S,
+// a hash (hT keys, 16-bit local indices) behind a filter of one bit per hash
+// value; then the row table (start and length of every row).
+constexpr uint32_t kSpanWords = 256;
+__host__ __device__ constexpr uint32_t filter_words(uint32_t G) { return G == 32u ? 256u : 1024u; }
+__host__ __device__ constexpr uint32_t gather_rows_at(uint32_t hT, uint32_t G) {
+  return hT + hT / 2u + filter_words(G) > 2u * kSpanWords ? hT + hT / 2u + filter_words(G) : 2u * kSpanWords;
 }
+constexpr uint32_t kRowLanes = 8;  // gather: lanes that read one row together
 
 template <int NW>
 __device__ __forceinline__ void load_row(const uint32_t* B, uint32_t v, uint32_t (&r)[NW]) {
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // open-addressing hash of S: vertex -> local index (linear probing, load <= 1/2)
   const uint32_t hT = p.hash_T;
   uint32_t* hkey = sb + p.off_H;
-  uint32_t* hval = hkey + hT;
+  uint16_t* hval = reinterpret_cast<uint16_t*>(hkey + hT);
 
   // class bounds come from device memory: clamp them so no unit index can leave the queue
   const uint32_t ubeg = min(p.bounds[2 * p.cls], p.n_units_max);
@@ -880,134 +882,109 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (LOCAL)
       for (uint32_t i = gt; i < (MODE == 0 ? d : 2u * d); i += G) loc[i] = 0ull;
     const uint32_t hshift = hT ? 33u - (uint32_t)__ffs(hT) : 0u;  // 32 - log2(hT)
-    // A warp unit whose S spans at most kSpanWords * 32 rank labels finds
-    // local indices in a membership map of that span instead of the hash:
-    // bit x - S[0] is set for every x of S, and mpre[w] counts the members in
-    // the words below w, so x's local index (or, for a non-member, the index
-    // it would take) is mpre[w] + popc(map[w] & bits below x). Every row
-    // word lies in [S[0], ...): DAG out-lists hold only higher ranks.
+    // An S that spans at most kSpanWords * 32 rank labels (every graph of up to
+    // 8,192 vertices) has a member map of that span: bit x - S[0] is set for
+    // every x of S, and mpre[w] counts the members in the words below w, so
+    // x's local index is mpre[w] + popc(map[w] & bits below x). A wider S has a
+    // hash behind a filter: almost every gathered word is not in S, and the
+    // filter (one bit per hash value, at most 3% of them set) turns those away
+    // with one read, where a probe of the half-full hash takes two to five.
     const uint32_t s0 = S[0], last = S[d - 1];
-    const bool wmap = G == 32 && hT != 0u && last - s0 < kSpanWords * 32u;
+    const bool wmap = hT != 0u && last - s0 < kSpanWords * 32u;
     uint32_t* map = hkey;
     uint32_t* mpre = hkey + kSpanWords;
-    if (wmap) {
+    const uint32_t fw = filter_words(G);
+    const uint32_t fshift = G == 32u ? 19u : 17u;  // 32 - log2(32 fw)
+    uint32_t* filter = hkey + hT + hT / 2u;
+    uint32_t* rbase = hkey + gather_rows_at(hT, G);
+    uint32_t* rlen = rbase + p.dcap;
+    if (hT) {
       const uint32_t nmw = ((last - s0) >> 5) + 1u;
-      for (uint32_t w = lane; w < nmw; w += 32u) map[w] = 0u;
-      __syncwarp();
-      for (uint32_t i = lane; i < d; i += 32u) {
-        const uint32_t o = S[i] - s0;
-        if (KC_IN_BOUNDS(o >> 5, kSpanWords, p.err)) atomicOr(&map[o >> 5], 1u << (o & 31u));
+      if (wmap) {
+        for (uint32_t w = gt; w < nmw; w += G) map[w] = 0u;
+      } else {
+        for (uint32_t i = gt; i < hT; i += G) hkey[i] = 0xffffffffu;
+        for (uint32_t i = gt; i < fw; i += G) filter[i] = 0u;
       }
-      __syncwarp();
-      uint32_t carry = 0;
-      for (uint32_t w0 = 0; w0 < nmw; w0 += 32u) {
-        const uint32_t w = w0 + lane;
-        const uint32_t c = w < nmw ? (uint32_t)__popc(map[w]) : 0u;
-        uint32_t incl = c;
-#pragma unroll
-        for (uint32_t o = 1; o < 32u; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += y;
-        }
-        if (w < nmw) mpre[w] = carry + incl - c;
-        carry += __shfl_sync(0xffffffffu, incl, 31);
+      for (uint32_t j = gt; j < d; j += G) {
+        const uint32_t x = S[j], b = p.rp[x];
+        rbase[j] = b;
+        rlen[j] = p.rp[x + 1] - b;
       }
-    } else if (hT) {
-      for (uint32_t i = gt; i < hT; i += G) hkey[i] = 0xffffffffu;
       gsync();
       for (uint32_t i = gt; i < d; i += G) {
         const uint32_t x = S[i];
-        uint32_t h = (x * 0x9e3779b1u) >> hshift;
-        while (atomicCAS(&hkey[h], 0xffffffffu, x) != 0xffffffffu) h = (h + 1u) & (hT - 1u);
-        hval[h] = i;
+        if (wmap) {
+          const uint32_t o = x - s0;
+          if (KC_IN_BOUNDS(o >> 5, kSpanWords, p.err)) atomicOr(&map[o >> 5], 1u << (o & 31u));
+        } else {
+          const uint32_t hx = x * 0x9e3779b1u;
+          atomicOr(&filter[hx >> (fshift + 5u)], 1u << ((hx >> fshift) & 31u));
+          uint32_t h = hx >> hshift;
+          while (atomicCAS(&hkey[h], 0xffffffffu, x) != 0xffffffffu) h = (h + 1u) & (hT - 1u);
+          hval[h] = (uint16_t)i;
+        }
+      }
+      if (wmap) {
+        gsync();
+        if (wig == 0) {
+          uint32_t carry = 0;
+          for (uint32_t w0 = 0; w0 < nmw; w0 += 32u) {
+            const uint32_t w = w0 + lane;
+            const uint32_t c = w < nmw ? (uint32_t)__popc(map[w]) : 0u;
+            uint32_t incl = c;
+#pragma unroll
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+              const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += y;
+            }
+            if (w < nmw) mpre[w] = carry + incl - c;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+          }
+        }
       }
     }
     gsync();
     lap(0);
-    if (G == 32 && hT) {
-      // Warp unit: the out-lists of S's rows are read as one flat array,
-      // 32 kGatherRun words per iteration with every lane's loads in flight
-      // together, so the unit's whole gather costs a few memory latencies
-      // instead of one per word of its longest row. The row table (start of
-      // each row in col, exclusive prefix of the row lengths, rpre[d] = total)
-      // follows the hash / map region; word f belongs to the last row j with
-      // rpre[j] <= f.
-      uint32_t* rbase = hkey + gather_rows_at(hT);
-      uint32_t* rpre = rbase + p.dcap;
-      uint32_t carry = 0;
-      for (uint32_t j0 = 0; j0 < d; j0 += 32u) {
-        const uint32_t j = j0 + lane;
-        uint32_t b = 0, len = 0;
-        if (j < d) {
-          const uint32_t x0 = S[j];
-          b = p.rp[x0];
-          len = p.rp[x0 + 1] - b;
-        }
-        uint32_t incl = len;
+    if (hT) {
+      // The out-lists of S's rows: kRowLanes lanes read a row, so a warp has
+      // four rows in hand, and every lane tests U words of its row per step
+      // (8, or 4 when no row of the four is longer than 32). What a step costs
+      // is issue, so the test is one table read per word, and only the words
+      // found to be members, one or two of a lane's U, pay for the local index
+      // and the bitmap's atomic. Before, a lane's words were eight consecutive
+      // ones of all rows joined, with a search for the row of every word: about
+      // 47 lane instructions a word. Batch of 2,500 mixed graphs (3.5e9 words):
+      // counting 26.8 ms before, 21.0 ms now; its gather's share of the unit
+      // groups' cycles fell from 8.8e10 to 6.0e10.
+      const uint32_t sub = lane / kRowLanes, ll = lane % kRowLanes, span = last - s0;
+      auto step = [&](auto ucount, const uint32_t* row, uint32_t len, uint32_t off, uint32_t j) {
+        constexpr uint32_t U = decltype(ucount)::value;
+        uint32_t xs[U], hit = 0;
 #pragma unroll
-        for (uint32_t o = 1; o < 32u; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += y;
+        for (uint32_t q = 0; q < U; ++q) {
+          const uint32_t i = off + q * kRowLanes + ll;
+          xs[q] = i < len ? __ldg(row + i) : 0xffffffffu;
         }
-        if (j < d) {
-          rbase[j] = b;
-          rpre[j] = carry + incl - len;
-        }
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      const uint32_t total = carry;
-      if (lane == 0) rpre[d] = total;
-      __syncwarp();
-      st_bytes += 4ull * (total + d);
-      // Each lane takes kGatherRun consecutive words of the flat array per
-      // iteration (lane L: words f0 + L kGatherRun ...), so one row search
-      // serves the run: its first word's row is jb (the row of the previous
-      // iteration's last word) plus the number of the next 32 row starts at or
-      // below it (a search over one start per lane), or, past 32 rows, a
-      // binary search of the rest; the later words of the run move forward
-      // over row starts one at a time. Almost every gathered word is not in S:
-      // a non-member costs one map (or hash) read, and only members pay for
-      // their local index and the bitmap atomic.
-      uint32_t jb = 0;
-      for (uint32_t f0 = 0; f0 < total; f0 += 32u * kGatherRun) {
-        const uint32_t t = jb + 1u + lane;
-        const uint32_t cand = t <= d ? rpre[t] : 0xffffffffu;
-        const uint32_t cand_last = __shfl_sync(0xffffffffu, cand, 31);
-        const uint32_t fl = f0 + lane * kGatherRun;
-        uint32_t c = 0;
+        if (wmap) {
 #pragma unroll
-        for (uint32_t sft = 16; sft; sft >>= 1)
-          if (__shfl_sync(0xffffffffu, cand, c + sft - 1u) <= fl) c += sft;
-        uint32_t j = jb + c;
-        if (c == 31u && cand_last <= fl) {
-          uint32_t hi = d;
-          j = jb + 32u;
-          while (hi - j > 1u) {
-            const uint32_t mid = (j + hi) >> 1;
-            if (rpre[mid] <= fl) j = mid;
-            else hi = mid;
+          for (uint32_t q = 0; q < U; ++q) {
+            const uint32_t o = xs[q] - s0;
+            if (o <= span) hit |= ((map[o >> 5] >> (o & 31u)) & 1u) << q;
+          }
+        } else {
+#pragma unroll
+          for (uint32_t q = 0; q < U; ++q) {
+            const uint32_t hx = xs[q] * 0x9e3779b1u;
+            if (xs[q] <= last) hit |= ((filter[hx >> (fshift + 5u)] >> ((hx >> fshift) & 31u)) & 1u) << q;
           }
         }
-        uint32_t xs[kGatherRun], js[kGatherRun];
-#pragma unroll
-        for (uint32_t q = 0; q < kGatherRun; ++q) {
-          const uint32_t f = fl + q;
-          xs[q] = 0xffffffffu;
-          if (f < total) {
-            while (rpre[j + 1u] <= f) ++j;  // rpre[d] = total > f
-            if (KC_IN_BOUNDS(j, d, p.err)) xs[q] = __ldg(p.col + rbase[j] + (f - rpre[j]));
-          }
-          js[q] = j;
-        }
-        jb = __shfl_sync(0xffffffffu, j, 31);
-#pragma unroll
-        for (uint32_t q = 0; q < kGatherRun; ++q) {
-          const uint32_t x = xs[q];
-          if (x > last) continue;  // past every vertex of S (also the padding)
+        for (; hit; hit &= hit - 1u) {
+          const uint32_t x = __ldg(row + off + ((uint32_t)__ffs(hit) - 1u) * kRowLanes + ll);
           uint32_t lo = 0xffffffffu;
           if (wmap) {
-            const uint32_t o = x - s0, mw = map[o >> 5];
-            if ((mw >> (o & 31u)) & 1u) lo = mpre[o >> 5] + (uint32_t)__popc(mw & ((1u << (o & 31u)) - 1u));
+            const uint32_t o = x - s0;
+            lo = mpre[o >> 5] + (uint32_t)__popc(map[o >> 5] & ((1u << (o & 31u)) - 1u));
           } else {
             uint32_t h = (x * 0x9e3779b1u) >> hshift;
             for (uint32_t hk; (hk = hkey[h]) != 0xffffffffu; h = (h + 1u) & (hT - 1u))
@@ -1015,40 +992,38 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
                 lo = hval[h];
                 break;
               }
+            if (lo == 0xffffffffu) continue;
           }
-          if (lo == 0xffffffffu) continue;
-          const uint32_t jr = js[q];
-          if (KC_IN_BOUNDS(jr * Ws + (lo >> 5), d * Ws, p.err)) atomicOr(&B[jr * Ws + (lo >> 5)], 1u << (lo & 31u));
-          if (sym && KC_IN_BOUNDS(lo * Ws + (jr >> 5), d * Ws, p.err))
-            atomicOr(&B[lo * Ws + (jr >> 5)], 1u << (jr & 31u));
+          if (KC_IN_BOUNDS(j * Ws + (lo >> 5), d * Ws, p.err)) atomicOr(&B[j * Ws + (lo >> 5)], 1u << (lo & 31u));
+          if (sym && KC_IN_BOUNDS(lo * Ws + (j >> 5), d * Ws, p.err))
+            atomicOr(&B[lo * Ws + (j >> 5)], 1u << (j & 31u));
+        }
+      };
+      for (uint32_t j0 = wig * (32u / kRowLanes); j0 < d; j0 += nwg * (32u / kRowLanes)) {
+        const uint32_t j = j0 + sub;
+        const uint32_t len = j < d ? rlen[j] : 0u;
+        const uint32_t* row = p.col + (j < d ? rbase[j] : 0u);
+        const uint32_t most = __reduce_max_sync(0xffffffffu, len);
+        if (p.stats) st_bytes += 4ull * __reduce_add_sync(0xffffffffu, ll == 0u && j < d ? len + 1u : 0u);
+        if (most <= 4u * kRowLanes) {
+          step(std::integral_constant<uint32_t, 4>{}, row, len, 0u, j);
+        } else {
+          for (uint32_t off = 0; off < most; off += 8u * kRowLanes)
+            step(std::integral_constant<uint32_t, 8>{}, row, len, off, j);
         }
       }
     } else {
       for (uint32_t j = wig; j < d; j += nwg) {
         const uint32_t x0 = S[j];
         const uint32_t b = p.rp[x0], e = p.rp[x0 + 1];
-        uint32_t i0 = b;
-        for (; i0 < e; i0 += 32) {
+        for (uint32_t i0 = b; i0 < e; i0 += 32) {
           const uint32_t i = i0 + lane;
           const uint32_t x = i < e ? __ldg(p.col + i) : 0xffffffffu;
           const bool inr = x <= last;
           if (!__any_sync(0xffffffffu, inr)) break;
           if (inr) {
-            uint32_t lo = 0xffffffffu;
-            if (hT) {
-              // the hash holds every vertex of S; x may be absent (a miss)
-              uint32_t h = (x * 0x9e3779b1u) >> hshift;
-              for (uint32_t key; (key = hkey[h]) != 0xffffffffu; h = (h + 1u) & (hT - 1u))
-                if (key == x) { lo = hval[h]; break; }
-            } else {
-              uint32_t a = j + 1, c = d;
-              while (a < c) {
-                const uint32_t mid = (a + c) >> 1;
-                if (S[mid] < x) a = mid + 1; else c = mid;
-              }
-              if (a < d && S[a] == x) lo = a;
-            }
-            if (lo != 0xffffffffu && KC_IN_BOUNDS(lo, d, p.err)) {
+            const uint32_t lo = j + 1u + lower_bound_u32(S + j + 1u, d - j - 1u, x);
+            if (lo < d && S[lo] == x && KC_IN_BOUNDS(lo, d, p.err)) {
               atomicOr(&B[j * Ws + (lo >> 5)], 1u << (lo & 31u));
               if (sym) atomicOr(&B[lo * Ws + (j >> 5)], 1u << (j & 31u));
             }
@@ -1776,16 +1751,15 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   size_t pstride = pstride_of();
   size_t sFr = lane ? 0 : al4((size_t)nparts * pstride);
   const size_t limit_words = ((size_t)ctx->max_smem_optin - kStaticSmemBytes) / 4;
-  // hash of S for the bitmap build: 2*hT words, hT the power of two >= 2 dcap
-  // (load at most 1/2)
+  // hash of S for the bitmap build: hT the power of two >= 2 dcap (load at
+  // most 1/2)
   uint32_t hT = 0;
   if (dcap <= 2048) {
     hT = 64;
     while (hT < 2u * dcap) hT <<= 1;
   }
-  // warp units keep their gather's row table (start and prefix of each row,
-  // 2 dcap + 1 words) behind the hash or the membership map
-  const size_t sRow = G == 32 ? al4(2 * (size_t)dcap + 1) : 0;
+  // the gather's row table (start and length of each row) follows its tables
+  const size_t sRow = al4(2 * (size_t)dcap);
   bool bitmap_global = lp.force_global_bitmap;
   bool frames_global = false;
   // The hash is needed only while the bitmap is built and the frames only
@@ -1795,7 +1769,7 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   auto group_words = [&]() {
     return hdr + sS + sR0 + (bitmap_global ? 0 : al4(sB)) + sLoc +
            std::max<size_t>(frames_global ? 0 : sFr,
-                            !hT ? 0 : (G == 32 ? gather_rows_at(hT) + sRow : 2 * (size_t)hT));
+                            !hT ? 0 : gather_rows_at(hT, G) + sRow);
   };
   if (compact && (size_t)gpb * group_words() > limit_words) {  // the frames come before the compact bitmaps
     compact = false;

@@ -671,11 +671,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // Work budget: a unit whose traversal exceeds p.budget nodes stops, drops
   // its partial count and is appended to the heavy list, which a CTA-wide
   // pass counts afterwards. Nodes are charged to hdr[4] in steps of 64 and
-  // hdr[5] flags the stop; each partition keeps the unit's count in uacc
-  // until the unit is known to have finished.
+  // hdr[5] flags the stop; each partition (pivoting: its lanes' sum) keeps the
+  // unit's count in uacc until the unit is known to have finished.
   const bool budgeted = p.budget != 0;
   unsigned __int128 uacc = 0;
-  unsigned __int128 lacc = 0;  // pivoting: this lane's share of the nodes counted whole
   uint32_t since_charge = 0;
   auto over_budget = [&]() -> bool {  // partition-uniform
     uint32_t stop = 0;
@@ -770,7 +769,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (timing) tc = clk32();
     const uint32_t unit = p.queue[pos];
     uacc = 0;
-    lacc = 0;
     since_charge = 0;
     uint32_t src, d;
     if (!p.edge_units) {
@@ -1214,7 +1212,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         if constexpr (MK)  // the k with k - hold0 <= 2 are closed already
           uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r), kon && kl + r >= k + 3u);
         else
-          lacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
+          uacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
         st_words += 32u * cmp[0];
       }
     } else {
@@ -1328,18 +1326,21 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         leaf_pinc = 0;
         // several k: this lane's k is still open here if its k - hold was
         // at least 3 at the parent
+        // the walker's own adds: every lane its k, else (one k) lane 0 alone, as
+        // nodes counted whole add each lane's share
+        const bool adds = mk || LOCAL || pt.plane == 0u;
         bool kopen = kon && kl + (pchild ? 0u : 1u) >= hold + 3u;
         if (nc == 0u) {
           leaf_cnt = binom(drop, r);
           if (r >= 1u && drop >= 1u) leaf_pinc = binom(drop - 1u, r - 1u);
-          if (own) uacc += mk ? (kopen ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
+          if (own && adds) uacc += mk ? (kopen ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
           return false;
         }
         if (hold + drop + nc < (mk ? p.kset[0] : k)) return false;
         if (r <= 1u) {  // (never with several k: an open k has k - hold >= 2 here)
           leaf_cnt = (r == 0u) ? (unsigned __int128)1u : (unsigned __int128)(nc + drop);
           leaf_pinc = (r == 1u && drop >= 1u) ? 1u : 0u;
-          if (own && !mk) uacc += leaf_cnt;
+          if (own && adds && !mk) uacc += leaf_cnt;
           if (lc && own && r == 1u)  // each candidate c completes one clique
             for (uint32_t w = pt.plane; w < W; w += pt.P)
               for (uint32_t x = F[w]; x; x &= x - 1u) loc2_add(w * 32u + (uint32_t)__ffs(x) - 1u, 1u);
@@ -1384,7 +1385,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           if constexpr (MK)
             uacc += close_node_multi(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols, kl - hold, kopen);
           else
-            lacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
+            uacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
           const uint32_t cost = cmp[0];
           since_charge += cost;
           st_words += 32u * cost;
@@ -1435,7 +1436,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         if (r == 2u) {  // edges of G[F] + drop * |F| + C(drop, 2)
           leaf_cnt = (unsigned __int128)(esum / 2u) + (unsigned __int128)drop * nc + binom(drop, 2u);
           leaf_pinc = drop >= 1u ? (unsigned __int128)(nc + drop - 1u) : 0u;
-          if (own) uacc += mk ? ((kopen && kl == hold + 2u) ? leaf_cnt : (unsigned __int128)0u) : leaf_cnt;
+          if (own && adds) uacc += mk ? ((kopen && kl == hold + 2u) ? leaf_cnt : (unsigned __int128)0u) : leaf_cnt;
           return false;
         }
         // several k: a smaller k that reaches k - hold = 2 here is closed here
@@ -1454,7 +1455,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           nc -= nu;
           if (nc == 0u) {  // F was a clique: a leaf with all of it as pivots
             leaf_cnt = binom(drop, r);
-            if (own) uacc += mk ? (kopen ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
+            if (own && adds) uacc += mk ? (kopen ? binom(drop, kl - hold) : (unsigned __int128)0u) : leaf_cnt;
             return false;
           }
           if (narrow) nzm = __ballot_sync(pt.pmask, pt.plane < W && F[pt.plane] != 0u);
@@ -1528,105 +1529,135 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         }
       };
 
-      for (uint32_t v = 0; v < d; ++v) {
+      // One loop and one call site of `enter` (its code is large, and three
+      // copies of it kept the warps waiting for instructions, the top stall of
+      // dense units): a step forms the candidate set of the next node (a root
+      // branch, a branch of the top frame, or the top frame's pivot branch in
+      // that frame's own slot), enters it, and pushes or drops its frame.
+      enum Step { kRoot, kBranch, kPivot };
+      int lv = -1;  // top frame
+      uint32_t v = 0;  // root branches below v are done
+      for (;;) {
         if (budgeted && over_budget()) break;
-        if (!((R0[v >> 5] >> (v & 31u)) & 1u)) continue;
-        if (L == 1u && !claim()) continue;
-        const bool own1 = L == 1u || top_owner;
-        const uint32_t hold = hold0 + (v != p0 ? 1u : 0u), drop = (v == p0) ? 1u : 0u;
-        if (own1) st_nodes++;
-        if (hold > k) continue;
-        uint32_t* F0 = frames;
-        for (uint32_t w = pt.plane; w < W; w += pt.P) F0[w] = B[v * Ws + w] & ~(R0[w] & low_mask(v, w));
-        __syncwarp(pt.pmask);
-        if (!enter(F0, hold, drop, own1, v == p0, L > 1u)) {
-          if (lc && own1 && pt.plane == 0) {
-            const unsigned __int128 x = (v != p0) ? leaf_cnt : leaf_pinc;
-            if (x) loc2_add(v, x);
+        Step step;
+        uint32_t* F;
+        uint32_t hold, drop, held;  // held: the vertex that the node's branch holds
+        bool own, above;
+        if (lv < 0) {
+          // the next root branch
+          while (v < d) {
+            const uint32_t x = R0[v >> 5] >> (v & 31u);
+            if (x) {
+              v += (uint32_t)__ffs(x) - 1u;
+              break;
+            }
+            v = (v | 31u) + 1u;
           }
+          if (v >= d) break;
+          held = v++;
+          if (L == 1u && !claim()) continue;
+          step = kRoot;
+          own = L == 1u || top_owner;
+          above = L > 1u;
+          hold = hold0 + (held != p0 ? 1u : 0u);
+          drop = (held == p0) ? 1u : 0u;
+          if (own) st_nodes++;
+          if (hold > k) continue;
+          F = frames;
+          for (uint32_t w = pt.plane; w < W; w += pt.P) F[w] = B[held * Ws + w] & ~(R0[w] & low_mask(held, w));
           __syncwarp(pt.pmask);
-          continue;
-        }
-        if (lc) {
-          ndl = 0;
-          if (pt.plane == 0) {
-            fr_open(F0, v != p0 ? v : 0xffffffffu);
-            if (v == p0) dl[0] = p0;  // the root pivot is a pivot of this whole subtree
-          }
-          ndl = (v == p0) ? 1u : 0u;
-          __syncwarp(pt.pmask);
-        }
-        int lv = 0;
-        while (lv >= 0) {
-          if (budgeted && over_budget()) break;
-          uint32_t* F = frames + (size_t)lv * p.fw;
+        } else {
+          F = frames + (size_t)lv * p.fw;
           uint32_t wi = 0;
           const int vb = part_next_bit(F + W, F[2 * W + 3], W, pt, &wi);
-          const uint32_t fh = F[2 * W], fd = F[2 * W + 1], fp = F[2 * W + 2];
+          hold = F[2 * W];
+          drop = F[2 * W + 1];
+          held = F[2 * W + 2];
           if (vb < 0) {
             // every other branch is done: the pivot's branch replaces the frame
-            const bool own = (uint32_t)lv + 1u >= L || top_owner;
+            step = kPivot;
+            own = (uint32_t)lv + 1u >= L || top_owner;
+            above = (uint32_t)lv + 1u < L;
             if (own) st_nodes++;
             __syncwarp(pt.pmask);
-            if (lc) {  // fp joins this frame's pivots
+            if (lc) {  // the pivot joins this frame's pivots
               if (pt.plane == 0) {
-                dl[ndl] = fp;
+                dl[ndl] = held;
                 const unsigned __int128 tp = fr_get(F, 10);
-                if (tp) loc2_add(fp, (unsigned __int128)0 - tp);
+                if (tp) loc2_add(held, (unsigned __int128)0 - tp);
               }
               ++ndl;
             }
-            for (uint32_t w = pt.plane; w < W; w += pt.P) F[w] &= B[fp * Ws + w];
+            ++drop;
+            for (uint32_t w = pt.plane; w < W; w += pt.P) F[w] &= B[held * Ws + w];
             __syncwarp(pt.pmask);
-            if (!enter(F, fh, fd + 1u, own, true, (uint32_t)lv + 1u < L)) {
-              if (lc) {
-                if (pt.plane == 0) {
-                  if (own) fr_take(F);
-                  fr_close(F, lv);
-                }
-                __syncwarp(pt.pmask);
-                ndl = F[2 * W + 5];
-                __syncwarp(pt.pmask);
-              }
-              --lv;
-            }
-            continue;
-          }
-          const uint32_t u = (uint32_t)vb;
-          __syncwarp(pt.pmask);
-          if (pt.plane == 0) {
-            F[W + wi] &= ~(1u << (u & 31u));
-            F[2 * W + 3] = wi;
-          }
-          const uint32_t h2 = fh + 1u;  // u is not the pivot
-          bool descend = h2 <= k;
-          if (descend && (uint32_t)(lv + 1) >= p.depth) {
-            if (pt.plane == 0) set_error(p.err, DEV_ERR_STACK);
-            descend = false;
-          }
-          bool own = (uint32_t)lv + 2u > L || top_owner;
-          if (descend && (uint32_t)lv + 2u == L) own = descend = claim();
-          if (own) st_nodes++;
-          uint32_t* Fc = F + p.fw;
-          if (descend)
-            for (uint32_t w = pt.plane; w < W; w += pt.P) Fc[w] = F[w] & B[u * Ws + w];
-          __syncwarp(pt.pmask);
-          if (pt.plane == 0) F[u >> 5] &= ~(1u << (u & 31u));  // later siblings exclude u
-          __syncwarp(pt.pmask);
-          if (descend && enter(Fc, h2, fd, own, false, (uint32_t)lv + 2u < L)) {
-            if (lc) {
-              if (pt.plane == 0) fr_open(Fc, u);
-              __syncwarp(pt.pmask);
-            }
-            ++lv;
-          } else if (descend && lc && own) {
-            // the child ended at once: u holds its cliques, this frame takes them too
+          } else {
+            step = kBranch;
+            held = (uint32_t)vb;
+            __syncwarp(pt.pmask);
             if (pt.plane == 0) {
-              if (leaf_cnt) loc2_add(u, leaf_cnt);
-              fr_take(F);
+              F[W + wi] &= ~(1u << (held & 31u));
+              F[2 * W + 3] = wi;
+            }
+            ++hold;  // the branch is not the pivot's
+            bool descend = hold <= k;
+            if (descend && (uint32_t)(lv + 1) >= p.depth) {
+              if (pt.plane == 0) set_error(p.err, DEV_ERR_STACK);
+              descend = false;
+            }
+            own = (uint32_t)lv + 2u > L || top_owner;
+            above = (uint32_t)lv + 2u < L;
+            if (descend && (uint32_t)lv + 2u == L) own = descend = claim();
+            if (own) st_nodes++;
+            uint32_t* Fc = F + p.fw;
+            if (descend)
+              for (uint32_t w = pt.plane; w < W; w += pt.P) Fc[w] = F[w] & B[held * Ws + w];
+            __syncwarp(pt.pmask);
+            if (pt.plane == 0) F[held >> 5] &= ~(1u << (held & 31u));  // later siblings exclude it
+            __syncwarp(pt.pmask);
+            if (!descend) continue;
+            F = Fc;
+          }
+        }
+        const bool pushed = enter(F, hold, drop, own, step == kRoot ? held == p0 : step == kPivot, above);
+        if (!lc) {
+          if (step == kPivot) lv -= pushed ? 0 : 1;
+          else lv += pushed ? 1 : 0;
+        } else if (step == kRoot) {
+          if (pushed) {
+            if (pt.plane == 0) {
+              ndl = 0;
+              fr_open(F, held != p0 ? held : 0xffffffffu);
+              if (held == p0) dl[0] = p0;  // the root pivot is a pivot of this whole subtree
+            }
+            ndl = (held == p0) ? 1u : 0u;
+            lv = 0;
+          } else if (own && pt.plane == 0) {
+            const unsigned __int128 x = (held != p0) ? leaf_cnt : leaf_pinc;
+            if (x) loc2_add(held, x);
+          }
+          __syncwarp(pt.pmask);
+        } else if (step == kPivot) {
+          if (!pushed) {
+            if (pt.plane == 0) {
+              if (own) fr_take(F);
+              fr_close(F, lv);
             }
             __syncwarp(pt.pmask);
+            ndl = F[2 * W + 5];
+            __syncwarp(pt.pmask);
+            --lv;
           }
+        } else {
+          if (pushed) {
+            if (pt.plane == 0) fr_open(F, held);
+            ++lv;
+          } else if (own && pt.plane == 0) {
+            // the child ended at once: it holds its cliques, the parent's frame takes them too
+            if (leaf_cnt) loc2_add(held, leaf_cnt);
+            fr_take(F - p.fw);
+          }
+          __syncwarp(pt.pmask);
         }
       }
       // this walker has been through every cut node: all of them are taken
@@ -1639,14 +1670,11 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     if (budgeted && hdr[5]) {
       if (gt == 0) p.heavy[atomicAdd(p.heavy_count, 1u)] = unit;
     } else {
-      if (MODE == 1 && !MK && compact) {  // the lanes' shares: every lane of the partition gets their sum
-        if (__any_sync(pt.pmask, lacc != 0)) {
-          for (uint32_t o = 1; o < pt.P; o <<= 1) {
-            const unsigned long long lo = __shfl_xor_sync(pt.pmask, (unsigned long long)lacc, o);
-            const unsigned long long hi = __shfl_xor_sync(pt.pmask, (unsigned long long)(lacc >> 64), o);
-            lacc += ((unsigned __int128)hi << 64) | lo;
-          }
-          uacc += lacc;
+      if (MODE == 1 && !LOCAL && !MK && __any_sync(pt.pmask, uacc != 0)) {  // the lanes' shares, summed in every lane
+        for (uint32_t o = 1; o < pt.P; o <<= 1) {
+          const unsigned long long lo = __shfl_xor_sync(pt.pmask, (unsigned long long)uacc, o);
+          const unsigned long long hi = __shfl_xor_sync(pt.pmask, (unsigned long long)(uacc >> 64), o);
+          uacc += ((unsigned __int128)hi << 64) | lo;
         }
       }
       acc += uacc;

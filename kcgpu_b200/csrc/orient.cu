@@ -21,13 +21,10 @@
 // orientation's total order, so every out-list holds larger labels only and
 // the induced-subgraph bitmaps of the counting stage are upper-triangular.
 #include <algorithm>
-#include <cooperative_groups.h>
 
 #include "dev_common.cuh"
 #include "engine.h"
 #include "prims.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace kc {
 
@@ -182,6 +179,7 @@ struct PeelArgs {
   uint2* front_b;
   uint32_t* ctr;        // 4 phase slots x 4 counters, zeroed; then the solo CTA's state
   uint32_t init_prio;   // 2m: the priority the final batch keeps
+  uint32_t* bar;        // grid barrier: arrivals so far, zeroed
   uint32_t* out;        // [0] last level, [1] sub-rounds, [2] error
 };
 constexpr uint32_t kPeelSolo = 32;  // ctr: kPeelStateWords words left by the solo CTA
@@ -395,12 +393,35 @@ __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
   }
 }
 
+// Barrier over the cooperative grid: one release-add per CTA on a counter that
+// only grows, and an acquire-load spin, which costs @BAR@ us where the
+// library's (two full fences per CTA) took 9 us. The spin is bounded: a CTA
+// that waits for a minute records a timeout, and every CTA leaves the kernel
+// at its next barrier. The whole CTA returns false then.
+constexpr uint32_t kPeelSpins = 1u << 26;
+
+__device__ __forceinline__ bool grid_barrier(const PeelArgs& a, uint32_t& target) {
+  target += gridDim.x;
+  int ok = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    uint32_t seen = 0, spins = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+    } while (seen < target && ++spins < kPeelSpins);
+    ok = seen >= target;
+    if (!ok) set_error(a.out + 2, DEV_ERR_TIMEOUT);
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
 __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
-  cg::grid_group grid = cg::this_grid();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = lane_id();
   const uint32_t gw = tid >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   PeelState st = {a.n, 0, 0, 0, 0, 0, 0, 0, 0};
+  uint32_t bar = 0;
   // Counters live in four phase slots; a phase zeroes the slot two phases
   // ahead, which every thread has finished reading by then.
   uint32_t phase = 0;
@@ -415,7 +436,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
           o[4] = st.fsize; o[5] = st.pieces; o[6] = st.priority; o[7] = st.flips; o[8] = st.too_big;
         }
       }
-      grid.sync();
+      if (!grid_barrier(a, bar)) return;
       const uint32_t* o = a.ctr + kPeelSolo;
       st = {__ldcg(o),     __ldcg(o + 1), __ldcg(o + 2), __ldcg(o + 3), __ldcg(o + 4),
             __ldcg(o + 5), __ldcg(o + 6), __ldcg(o + 7), __ldcg(o + 8)};
@@ -453,7 +474,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
           warp_append(!to_next && cur[q] == (int)st.bucket_end, u[q], bucket + st.bsize, &c[2]);
         }
       }
-      grid.sync();
+      if (!grid_barrier(a, bar)) return;
       st.pieces = __ldcg(c);
       st.fsize = min(__ldcg(c + 1), a.n);
       st.bsize = min(st.bsize + __ldcg(c + 2), a.n);
@@ -472,7 +493,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
       }
       mn = __reduce_max_sync(0xffffffffu, mn);
       if (lane == 0 && mn) atomicMax(&c[3], mn);
-      grid.sync();
+      if (!grid_barrier(a, bar)) return;
       st.pieces = __ldcg(c);
       st.fsize = min(__ldcg(c + 1), a.n);
       st.bsize = min(__ldcg(c + 2), a.n);
@@ -489,7 +510,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
       }
       mn = __reduce_max_sync(0xffffffffu, mn);
       if (lane == 0 && mn) atomicMax(&c[3], mn);
-      grid.sync();
+      if (!grid_barrier(a, bar)) return;
       st.bsize = min(__ldcg(c + 2), a.n);
       const uint32_t m = __ldcg(c + 3);
       if (m == 0u) {  // no live vertex left, todo > 0: cannot happen for a valid CSR; never spin
@@ -506,7 +527,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
   }
   // the final batch keeps its initial priority (every vertex has been put in
   // a front, and what any CTA wrote there was ordered by the last barrier)
-  grid.sync();
+  if (!grid_barrier(a, bar)) return;
   for (uint32_t v = tid; v < a.n; v += nw * 32u)
     if (__ldcg(a.prio + v) == st.priority) a.prio[v] = a.init_prio;
 }
@@ -531,7 +552,7 @@ kc_status run_peel(kc_graph* g, uint32_t* prio, uint32_t* level) {
   KC_CUDA(t.alloc(&bb, sizeof(uint32_t) * n));
   KC_CUDA(t.alloc(&fa, sizeof(uint2) * front_cap));
   KC_CUDA(t.alloc(&fb, sizeof(uint2) * front_cap));
-  constexpr uint32_t kCtrWords = kPeelSolo + kPeelStateWords;
+  constexpr uint32_t kCtrWords = 128 + 1;  // the barrier's counter on a line of its own
   KC_CUDA(t.alloc(&ctr, sizeof(uint32_t) * kCtrWords));
   KC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrWords, s));
   const uint32_t init_prio = (uint32_t)std::min<uint64_t>(2 * g->m, 0xffffffffull);
@@ -542,6 +563,7 @@ kc_status run_peel(kc_graph* g, uint32_t* prio, uint32_t* level) {
   a.rp = g->rp; a.col = g->col; a.n = n; a.deg = deg; a.prio = prio; a.level = level;
   a.bucket_a = ba; a.bucket_b = bb; a.front_a = fa; a.front_b = fb; a.ctr = ctr; a.out = ctr + 16;
   a.init_prio = init_prio;
+  a.bar = ctr + 128;
   // at most one CTA per SM, each with enough vertices or row entries to be
   // worth a barrier's arrival (a small graph is peeled by one CTA alone)
   const uint64_t want = std::max<uint64_t>(ceil_div<uint64_t>(n, kSoloScan), ceil_div<uint64_t>(2 * g->m, kSoloEdges));

@@ -156,15 +156,16 @@ __global__ void k_export_fill(const uint32_t* __restrict__ drp, const uint32_t* 
 //     row (15,000 entries) is spread over many warps;
 //   * levels without vertices are skipped through the smallest degree seen.
 // R-MAT scale 18 (3.8M edges): 9.6 ms with two barriers per sub-round, flags
-// and four CTAs per SM, 3.7 ms now; scale 11 (16k edges) 0.78 ms, 0.27 ms now.
+// and four CTAs per SM, 2.6 ms now; scale 11 (16k edges) 0.78 ms, 0.27 ms now.
 
 constexpr uint32_t PEEL_WINDOW = 64;     // degree window of the candidate bucket
 constexpr uint32_t kPeelThreads = 1024;
 constexpr uint32_t kPiece = 128;         // row entries per front piece (four per lane of a warp)
-// One CTA takes a front of up to kSoloFront pieces with up to kSoloEdges
-// row entries (16 per thread: about the cost of a grid step), and bucket or
-// vertex scans of up to kSoloScan entries.
-constexpr uint32_t kSoloFront = 1024, kSoloEdges = 16384, kSoloScan = 8192;
+// One CTA takes a front of up to kSoloFront pieces with up to kSoloEdges row
+// entries, and bucket or vertex scans of up to kSoloScan entries: one SM makes
+// about one random access per cycle, so 4,096 of them cost what a grid step's
+// barrier does.
+constexpr uint32_t kSoloFront = 1024, kSoloEdges = 4096, kSoloScan = 4096;
 
 struct PeelArgs {
   const uint32_t* rp;
@@ -313,7 +314,7 @@ __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
       __syncthreads();
       uint32_t top = 1;
       while (top < st.pieces) top <<= 1;
-      constexpr uint32_t kU = 8;  // edges in flight per thread
+      constexpr uint32_t kU = kSoloEdges / kPeelThreads;  // edges per thread, all in flight
       for (uint32_t i0 = 0; i0 < total; i0 += kU * kPeelThreads) {
         uint32_t u[kU];
         int cur[kU];
@@ -393,25 +394,31 @@ __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
   }
 }
 
-// Barrier over the cooperative grid: one release-add per CTA on a counter that
-// only grows, and an acquire-load spin, which costs @BAR@ us where the
-// library's (two full fences per CTA) took 9 us. The spin is bounded: a CTA
-// that waits for a minute records a timeout, and every CTA leaves the kernel
-// at its next barrier. The whole CTA returns false then.
+// Barrier over the cooperative grid (a release-add and an acquire spin per
+// CTA, 2.4k cycles), after which thread 0 of every CTA reads `words` words at
+// src for its CTA: with every warp of 148 CTAs reading the counters itself,
+// one L2 line served 40,000 requests, which took 15k cycles. The spin is
+// bounded: a CTA that waits for a minute records a timeout, and every CTA
+// leaves the kernel at its next barrier; the whole CTA returns false then.
 constexpr uint32_t kPeelSpins = 1u << 26;
 
-__device__ __forceinline__ bool grid_barrier(const PeelArgs& a, uint32_t& target) {
+__device__ __forceinline__ bool grid_barrier(const PeelArgs& a, uint32_t& target, const uint32_t* src, uint32_t words,
+                                             uint32_t* got) {
   target += gridDim.x;
   int ok = 1;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-    uint32_t seen = 0, spins = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
-    } while (seen < target && ++spins < kPeelSpins);
-    ok = seen >= target;
-    if (!ok) set_error(a.out + 2, DEV_ERR_TIMEOUT);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+      uint32_t seen = 0, spins = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+      } while (seen < target && ++spins < kPeelSpins);
+      ok = seen >= target;
+      if (!ok) set_error(a.out + 2, DEV_ERR_TIMEOUT);
+    }
+    __syncwarp();
+    if (threadIdx.x < words) got[threadIdx.x] = __ldcg(src + threadIdx.x);
   }
   return __syncthreads_and(ok) != 0;
 }
@@ -422,6 +429,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
   const uint32_t gw = tid >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   PeelState st = {a.n, 0, 0, 0, 0, 0, 0, 0, 0};
   uint32_t bar = 0;
+  __shared__ uint32_t got[kPeelStateWords];  // what the last barrier brought
   // Counters live in four phase slots; a phase zeroes the slot two phases
   // ahead, which every thread has finished reading by then.
   uint32_t phase = 0;
@@ -436,10 +444,8 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
           o[4] = st.fsize; o[5] = st.pieces; o[6] = st.priority; o[7] = st.flips; o[8] = st.too_big;
         }
       }
-      if (!grid_barrier(a, bar)) return;
-      const uint32_t* o = a.ctr + kPeelSolo;
-      st = {__ldcg(o),     __ldcg(o + 1), __ldcg(o + 2), __ldcg(o + 3), __ldcg(o + 4),
-            __ldcg(o + 5), __ldcg(o + 6), __ldcg(o + 7), __ldcg(o + 8)};
+      if (!grid_barrier(a, bar, a.ctr + kPeelSolo, kPeelStateWords, got)) return;
+      st = {got[0], got[1], got[2], got[3], got[4], got[5], got[6], got[7], got[8]};
       continue;  // (the next step is a grid step, whose barrier comes before the state is written again)
     }
     uint32_t* bucket = (st.flips & 1u) ? a.bucket_b : a.bucket_a;
@@ -474,10 +480,10 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
           warp_append(!to_next && cur[q] == (int)st.bucket_end, u[q], bucket + st.bsize, &c[2]);
         }
       }
-      if (!grid_barrier(a, bar)) return;
-      st.pieces = __ldcg(c);
-      st.fsize = min(__ldcg(c + 1), a.n);
-      st.bsize = min(st.bsize + __ldcg(c + 2), a.n);
+      if (!grid_barrier(a, bar, c, 4, got)) return;
+      st.pieces = got[0];
+      st.fsize = min(got[1], a.n);
+      st.bsize = min(st.bsize + got[2], a.n);
       st.flips ^= 2u;
       ++st.priority;
       if (st.fsize == 0) ++st.L;
@@ -493,12 +499,12 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
       }
       mn = __reduce_max_sync(0xffffffffu, mn);
       if (lane == 0 && mn) atomicMax(&c[3], mn);
-      if (!grid_barrier(a, bar)) return;
-      st.pieces = __ldcg(c);
-      st.fsize = min(__ldcg(c + 1), a.n);
-      st.bsize = min(__ldcg(c + 2), a.n);
+      if (!grid_barrier(a, bar, c, 4, got)) return;
+      st.pieces = got[0];
+      st.fsize = min(got[1], a.n);
+      st.bsize = min(got[2], a.n);
       st.flips ^= 1u;
-      const uint32_t m = __ldcg(c + 3);
+      const uint32_t m = got[3];
       if (st.fsize == 0) st.L = m ? min(~m, st.bucket_end) : st.bucket_end;
     } else {  // a new window
       uint32_t mn = 0;
@@ -510,9 +516,9 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
       }
       mn = __reduce_max_sync(0xffffffffu, mn);
       if (lane == 0 && mn) atomicMax(&c[3], mn);
-      if (!grid_barrier(a, bar)) return;
-      st.bsize = min(__ldcg(c + 2), a.n);
-      const uint32_t m = __ldcg(c + 3);
+      if (!grid_barrier(a, bar, c, 4, got)) return;
+      st.bsize = min(got[2], a.n);
+      const uint32_t m = got[3];
       if (m == 0u) {  // no live vertex left, todo > 0: cannot happen for a valid CSR; never spin
         if (tid == 0) a.out[2] = DEV_ERR_INPUT;
         break;
@@ -527,7 +533,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
   }
   // the final batch keeps its initial priority (every vertex has been put in
   // a front, and what any CTA wrote there was ordered by the last barrier)
-  if (!grid_barrier(a, bar)) return;
+  if (!grid_barrier(a, bar, a.ctr, 0, got)) return;
   for (uint32_t v = tid; v < a.n; v += nw * 32u)
     if (__ldcg(a.prio + v) == st.priority) a.prio[v] = a.init_prio;
 }
@@ -566,7 +572,7 @@ kc_status run_peel(kc_graph* g, uint32_t* prio, uint32_t* level) {
   a.bar = ctr + 128;
   // at most one CTA per SM, each with enough vertices or row entries to be
   // worth a barrier's arrival (a small graph is peeled by one CTA alone)
-  const uint64_t want = std::max<uint64_t>(ceil_div<uint64_t>(n, kSoloScan), ceil_div<uint64_t>(2 * g->m, kSoloEdges));
+  const uint64_t want = std::max<uint64_t>(ceil_div<uint64_t>(n, kSoloScan), ceil_div<uint64_t>(2 * g->m, 4 * kSoloEdges));
   dim3 grid((uint32_t)std::min<uint64_t>((uint64_t)ctx->sms, std::max<uint64_t>(1, want))), block(kPeelThreads);
   void* args[] = {&a};
   KC_CUDA(cudaLaunchCooperativeKernel((void*)k_peel, grid, block, args, 0, s));

@@ -224,7 +224,7 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
 // scores, reductions) with most lanes idle, and almost all nodes of a tree are
 // small and near its leaves. Two kinds are therefore counted whole: r = 3 with
 // at most 128 candidates (triangles, edges and vertices of G[F]) and r in
-// 4..20 with at most 32 candidates (a lane per pair of adjacent candidates).
+// 4..19 with at most 32 candidates (a lane per subproblem).
 // Both first copy G[F] into a compact bitmap of nc rows and ceil(nc / 32)
 // words. Larger nodes are worth splitting further: their branches are what
 // the walkers share. R-MAT scale 17, k = 5 (edge units): 37.8M tree nodes,
@@ -348,8 +348,9 @@ __host__ __device__ constexpr uint32_t compact_words(uint32_t n) {
 constexpr uint32_t kPairPrefix = 36;   // close_small: exclusive prefix of the row lengths
 constexpr uint32_t kTriangleMax = 128; // most candidates of an r = 3 node closed whole
 constexpr uint32_t kSmallMax = 32;     // most candidates of an r > 3 node closed whole
-constexpr int kSmallStack = 16;        // close_small: pushed frames (r - 5 at most)
-constexpr uint32_t kSmallMaxR = 20;
+constexpr int kSmallStack = 16;        // close_small: a lane's own frames (r - 3 at most)
+constexpr uint32_t kSmallMaxR = 19;
+constexpr uint32_t kQueueCap = 236;    // close_small: nodes on its shared stack
 // several k: the largest r closed whole, and the words of its histogram
 constexpr uint32_t kSmallMaxRMulti = 15;
 constexpr uint32_t kHistWords = (kSmallMaxRMulti + 1u) * (kSmallMax + 1u);
@@ -381,14 +382,20 @@ __device__ __forceinline__ unsigned __int128 binom_at(const unsigned long long* 
 }
 
 // r >= 3 with at most 32 candidates: adj holds their rows (one word each,
-// symmetric). The empty set and single candidates are closed; every pair
-// i < j of adjacent candidates is a task (pairs, not vertices: a dense node's
-// first vertices hold most of its cliques), taken by the lanes in turn, with
-// the common neighbours above j as its candidate set X and r - 2 vertices to
-// go. A lane counts its tasks alone, with sets in registers: r = 1 to 3 by
-// listing, above that by pivoting. Vertices adjacent to the whole set are
-// moved to the pivots at once (their branches are empty). Returns the lane's
-// share; pre[32] receives the most rows any lane visited.
+// symmetric). The lanes count subproblems (set, vertices to go, pivots) side by
+// side, with sets in registers, the last three levels by listing:
+//   * r <= 4: a task is a pair i < j of adjacent candidates, with the common
+//     neighbours above j as its set and r - 2 vertices to go (pairs, not
+//     vertices: a dense node's first vertices hold most of its cliques);
+//   * r > 4: the tasks are clique-tree nodes on a stack in shared memory. Up to
+//     32 of them are taken at a time; a lane closes its node or pushes its
+//     branches. Splitting by pivots keeps a near-clique's tree small, where
+//     pairs would walk it once per pair (R-MAT of 21k edges, k = 8: 1.1 ms for
+//     the units of up to 32 vertices by pairs, 0.06 ms). Lanes whose branches no
+//     longer fit walk their nodes to the end on stacks of their own.
+// Vertices adjacent to the whole set are moved to the pivots at once (their
+// branches are empty). Returns the lane's share; pre[32] receives the steps
+// (rows visited, the most of any lane per round).
 //
 // MK (several k in one walk): nothing is known of the smaller k, so instead of
 // binomials of one k the lanes count, in hist[h (kSmallMax + 1) + x], the
@@ -396,129 +403,217 @@ __device__ __forceinline__ unsigned __int128 binom_at(const unsigned long long* 
 // them: each stands for C(drop + x, k - held - h) cliques of every k. r belongs
 // to the largest k; the closed forms for r <= 3 hold for every smaller k too.
 // R-MAT of 55k edges, k = 3..15 in one walk: 11.5 ms with every node walked,
-// 4.2 ms now.
+// 4.2 ms by pairs, 1.5 ms now.
 template <bool MK>
 __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, uint32_t* pre, uint32_t nc, uint32_t r,
                                                          uint32_t drop, const unsigned long long* binom, uint32_t cols,
-                                                         uint32_t* hist) {
+                                                         uint2* queue, uint32_t* hist) {
   const uint32_t lane = lane_id();
-  auto leaf = [&](uint32_t held, uint32_t dd, uint32_t times) {
+  const uint32_t mine = lane < nc ? adj[lane] : 0u;
+  unsigned __int128 acc = 0;
+  uint32_t it = 0, steps = 0;
+  auto put = [&](uint32_t held, uint32_t dd, uint32_t times) {
     if (times && KC_IN_BOUNDS(held * (kSmallMax + 1u) + (dd - drop), kHistWords, nullptr))
       atomicAdd(&hist[held * (kSmallMax + 1u) + (dd - drop)], times);
   };
-  const uint32_t mine = lane < nc ? adj[lane] & (0xfffffffeu << lane) : 0u;
-  const uint32_t c = __popc(mine);
-  uint32_t incl = c;
-#pragma unroll
-  for (uint32_t o = 1; o < 32u; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  pre[lane] = incl - c;
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  unsigned __int128 acc = 0;
+  // a node (P, rr vertices to go, dd pivots) without candidates, or with rr <= 3
+  auto leaf = [&](uint32_t rr, uint32_t dd) {
+    if (MK) put(r - rr, dd, 1u);
+    else acc += binom_at(binom, cols, dd, rr);
+  };
+  auto listed = [&](uint32_t P, uint32_t rr, uint32_t dd) {
+    const uint32_t n = __popc(P);
+    uint32_t e = 0, tri = 0;
+    if (rr >= 2u)
+      for (uint32_t x = P; x; x &= x - 1u) {
+        const uint32_t u = (uint32_t)__ffs(x) - 1u;
+        const uint32_t X = (x & (x - 1u)) & adj[u];
+        e += __popc(X);
+        ++it;
+        if (rr == 3u)
+          for (uint32_t y = X; y; y &= y - 1u) {
+            tri += __popc((y & (y - 1u)) & adj[__ffs(y) - 1]);
+            ++it;
+          }
+      }
+    if (MK) {
+      put(r - rr, dd, 1u);
+      put(r - rr + 1u, dd, n);
+      if (rr >= 2u) put(r - rr + 2u, dd, e);
+      if (rr == 3u) put(r, dd, tri);
+    } else {
+      const unsigned long long d1 = dd, d2 = dd >= 2u ? d1 * (d1 - 1ull) / 2ull : 0ull;
+      if (rr == 1u) acc += n + d1;
+      else if (rr == 2u) acc += e + d1 * n + d2;
+      else acc += tri + d1 * e + d2 * n + (dd >= 3u ? d2 * (d1 - 2ull) / 3ull : 0ull);
+    }
+  };
   if (MK) {
-    for (uint32_t i = lane; i < (r + 1u) * (kSmallMax + 1u); i += 32u) hist[i] = i == 0u ? 1u : (i == kSmallMax + 1u ? nc : 0u);
-  } else if (lane == 0) {
-    acc = binom_at(binom, cols, drop, r);
-    if (drop + 1u >= r) acc += (unsigned __int128)nc * binom_at(binom, cols, drop, r - 1u);
+    for (uint32_t i = lane; i < (r + 1u) * (kSmallMax + 1u); i += 32u) hist[i] = 0u;
+    __syncwarp();
   }
-  __syncwarp();
-  uint32_t it = 0;
-  uint32_t sP[kSmallStack], sR[kSmallStack], sX[kSmallStack];  // set, branches left, pivot and drop
-  for (uint32_t t = lane; t < total; t += 32u) {
-    uint32_t i = 0;  // pre[i] <= t < pre[i + 1]
+  if (r <= 4u) {
+    const uint32_t up = mine & (0xfffffffeu << lane);
+    const uint32_t c = __popc(up);
+    uint32_t incl = c;
 #pragma unroll
-    for (uint32_t s = 16; s; s >>= 1)
-      if (pre[i + s] <= t) i += s;
-    const uint32_t ui = adj[i] & (0xfffffffeu << i);
-    const uint32_t j = select_bit(ui, t - pre[i]);
-    uint32_t P = ui & adj[j] & (0xfffffffeu << j);
-    uint32_t rr = r - 2u, dd = drop;
-    int lv = 0;
-    for (;;) {
-      // the node (P, rr, dd)
-      const uint32_t n = __popc(P);
-      if (MK || n + dd >= rr) {
-        if (n == 0u) {
-          if (MK) leaf(r - rr, dd, 1u);
-          else acc += binom_at(binom, cols, dd, rr);
-        } else if (rr == 1u) {
-          if (MK) {
-            leaf(r - rr, dd, 1u);
-            leaf(r - rr + 1u, dd, n);
-          } else {
-            acc += n + dd;
-          }
-        } else if (rr <= 3u) {
-          uint32_t e = 0, tri = 0;
-          for (uint32_t x = P; x; x &= x - 1u) {
-            const uint32_t u = (uint32_t)__ffs(x) - 1u;
-            const uint32_t X = (x & (x - 1u)) & adj[u];
-            e += __popc(X);
-            ++it;
-            if (rr == 3u)
-              for (uint32_t y = X; y; y &= y - 1u) {
-                tri += __popc((y & (y - 1u)) & adj[__ffs(y) - 1]);
-                ++it;
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    pre[lane] = incl - c;
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (lane == 0) {  // the empty set and the single candidates
+      if (MK) {
+        put(0u, drop, 1u);
+        put(1u, drop, nc);
+      } else {
+        acc = binom_at(binom, cols, drop, r);
+        if (drop + 1u >= r) acc += (unsigned __int128)nc * binom_at(binom, cols, drop, r - 1u);
+      }
+    }
+    __syncwarp();
+    for (uint32_t t = lane; t < total; t += 32u) {
+      uint32_t i = 0;  // pre[i] <= t < pre[i + 1]
+#pragma unroll
+      for (uint32_t s = 16; s; s >>= 1)
+        if (pre[i + s] <= t) i += s;
+      const uint32_t ui = adj[i] & (0xfffffffeu << i);
+      const uint32_t j = select_bit(ui, t - pre[i]);
+      listed(ui & adj[j] & (0xfffffffeu << j), r - 2u, drop);
+    }
+    steps = __reduce_max_sync(0xffffffffu, it);
+  } else {
+    // the root: its scores are the row lengths
+    const uint32_t s0 = __popc(mine);
+    const uint32_t uni0 = __ballot_sync(0xffffffffu, lane < nc && s0 + 1u == nc);
+    const uint32_t P0 = (nc < 32u ? (1u << nc) - 1u : 0xffffffffu) & ~uni0;
+    const uint32_t d0 = drop + (uint32_t)__popc(uni0);
+    uint32_t top = 0;
+    if (P0 == 0u) {
+      if (lane == 0) leaf(r, d0);
+    } else {
+      const bool in = (P0 >> lane) & 1u;
+      const uint32_t piv = __reduce_max_sync(0xffffffffu, in ? (s0 << 8) | lane : 0u) & 31u;
+      const uint32_t R = P0 & ~__shfl_sync(0xffffffffu, mine, piv) & ~(1u << piv);
+      const uint32_t below = R & lanemask_lt();
+      if ((R >> lane) & 1u) queue[__popc(below)] = make_uint2(P0 & ~below & mine, ((r - 1u) << 16) | d0);
+      if (lane == piv) queue[__popc(R)] = make_uint2(P0 & ~R & mine, (r << 16) | (d0 + 1u));
+      top = (uint32_t)__popc(R) + 1u;
+    }
+    __syncwarp();
+    uint32_t sP[kSmallStack], sR[kSmallStack], sX[kSmallStack];  // set, branches left, (rr, pivot, dd)
+    while (top) {
+      const uint32_t cnt = min(top, 32u);
+      top -= cnt;
+      uint32_t P = 0, rr = 0, dd = 0, R = 0, piv = 0;
+      bool work = lane < cnt;
+      if (work) {
+        const uint2 q = queue[top + lane];
+        P = q.x;
+        rr = q.y >> 16;
+        dd = q.y & 0xffffu;
+      }
+      int lv = 0;
+      for (bool own = false;; own = true) {  // own: on the lane's own stack
+        uint32_t kids = 0;
+        bool fresh = !own;
+        while (work) {
+          bool open = false;
+          if (fresh) {
+            const uint32_t n = __popc(P);
+            if (MK || n + dd >= rr) {
+              if (n == 0u) {
+                leaf(rr, dd);
+              } else if (rr <= 3u) {
+                listed(P, rr, dd);
+              } else {
+                uint32_t best = 0, uni = 0;  // best: 1 + score, in the high half, of a non-universal candidate
+                for (uint32_t x = P; x; x &= x - 1u) {
+                  const uint32_t u = (uint32_t)__ffs(x) - 1u;
+                  const uint32_t s = __popc(P & adj[u]);
+                  if (s + 1u == n) uni |= 1u << u;
+                  else best = max(best, ((s + 1u) << 16) | u);
+                  ++it;
+                }
+                dd += __popc(uni);
+                P &= ~uni;
+                if (P == 0u) {
+                  leaf(rr, dd);
+                } else {
+                  open = true;
+                  piv = best & 31u;
+                  R = P & ~adj[piv] & ~(1u << piv);
+                }
               }
+            }
           }
-          const unsigned long long d1 = dd, d2 = d1 * (d1 - 1ull) / 2ull;  // (0 for dd = 0)
-          if (MK) {
-            leaf(r - rr, dd, 1u);
-            leaf(r - rr + 1u, dd, n);
-            leaf(r - rr + 2u, dd, e);
-            if (rr == 3u) leaf(r, dd, tri);
-          } else if (rr == 2u) {
-            acc += e + d1 * n + (dd >= 2u ? d2 : 0ull);
-          } else {
-            acc += tri + d1 * e + (dd >= 2u ? d2 * n : 0ull) + (dd >= 3u ? d2 * (d1 - 2ull) / 3ull : 0ull);
+          if (open && !own) {
+            kids = (uint32_t)__popc(R) + 1u;
+            break;
           }
-        } else {
-          uint32_t best = 0, uni = 0;  // best: 1 + score, in the high half, of a non-universal candidate
-          for (uint32_t x = P; x; x &= x - 1u) {
-            const uint32_t u = (uint32_t)__ffs(x) - 1u;
-            const uint32_t s = __popc(P & adj[u]);
-            if (s + 1u == n) uni |= 1u << u;
-            else best = max(best, ((s + 1u) << 16) | u);
-            ++it;
-          }
-          dd += __popc(uni);
-          P &= ~uni;
-          if (P == 0u) {
-            if (MK) leaf(r - rr, dd, 1u);
-            else acc += binom_at(binom, cols, dd, rr);
-          } else if (KC_IN_BOUNDS(lv, kSmallStack, nullptr)) {
-            const uint32_t piv = best & 0xffffu;
+          if (open && KC_IN_BOUNDS(lv, kSmallStack, nullptr)) {
             sP[lv] = P;
-            sR[lv] = P & ~adj[piv] & ~(1u << piv);
+            sR[lv] = R;
             sX[lv] = (rr << 24) | (piv << 16) | dd;
             ++lv;
           }
+          if (lv == 0) break;
+          // the next branch: the candidates outside the pivot's neighbourhood,
+          // then the pivot's own branch in its parent's frame
+          const uint32_t x = sX[lv - 1];
+          R = sR[lv - 1];
+          P = sP[lv - 1];
+          rr = x >> 24;
+          dd = x & 0xffffu;
+          if (R) {
+            const uint32_t u = (uint32_t)__ffs(R) - 1u;
+            sR[lv - 1] = R & (R - 1u);
+            sP[lv - 1] = P & ~(1u << u);
+            P &= adj[u];
+            --rr;
+          } else {
+            --lv;
+            P &= adj[(x >> 16) & 31u];
+            ++dd;
+          }
+          fresh = true;
         }
-      }
-      // the next branch: the candidates outside the pivot's neighbourhood,
-      // then the pivot's own branch in its parent's frame
-      if (lv == 0) break;
-      const uint32_t R = sR[lv - 1], x = sX[lv - 1];
-      P = sP[lv - 1];
-      rr = x >> 24;
-      dd = x & 0xffffu;
-      if (R) {
-        const uint32_t u = (uint32_t)__ffs(R) - 1u;
-        sR[lv - 1] = R & (R - 1u);
-        sP[lv - 1] = P & ~(1u << u);
-        P &= adj[u];
-        --rr;
-      } else {
-        --lv;
-        P &= adj[(x >> 16) & 31u];
-        ++dd;
+        __syncwarp();  // every node of the round has been read
+        steps += __reduce_max_sync(0xffffffffu, it) + 2u;
+        it = 0;
+        if (own || !__any_sync(0xffffffffu, kids != 0u)) break;
+        // the branches that fit go on the stack, in lane order
+        uint32_t incl = kids;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const bool fits = top + incl <= kQueueCap;
+        if (kids && fits) {
+          uint2* q = queue + top + (incl - kids);
+          *q++ = make_uint2(P & ~R & adj[piv], (rr << 16) | (dd + 1u));
+          for (uint32_t x = R; x; x &= x - 1u) {
+            const uint32_t u = (uint32_t)__ffs(x) - 1u;
+            *q++ = make_uint2(P & adj[u], ((rr - 1u) << 16) | dd);
+            P &= ~(1u << u);
+          }
+        }
+        top += __reduce_max_sync(0xffffffffu, fits ? incl : 0u);
+        work = kids != 0u && !fits;
+        if (work) {
+          sP[0] = P;
+          sR[0] = R;
+          sX[0] = (rr << 24) | (piv << 16) | dd;
+          lv = 1;
+        }
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, work)) break;
       }
     }
   }
-  it = __reduce_max_sync(0xffffffffu, it);
-  if (lane == 0) pre[32] = it;
+  if (lane == 0) pre[32] = steps;
   return acc;
 }
 
@@ -533,9 +628,10 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
   uint32_t cost = 1u + (nc >> 5);
   if (r > 3u) {
     if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
-    t = close_small<false>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols, nullptr);
+    t = close_small<false>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols,
+                           reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), nullptr);
     __syncwarp();
-    cost = 1u + (cmp[kPairPrefix + 32u] >> 5);
+    cost = 1u + (cmp[kPairPrefix + 32u] >> 4);
   } else if (nc <= 32u) {
     t = close_triangles<1, 1>(B, Ws, cand, nc, cmp, drop);
   } else if (nc <= 64u) {
@@ -559,9 +655,10 @@ __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, ui
                                                            const unsigned long long* binom, uint32_t cols,
                                                            uint32_t kr, bool open) {
   const uint32_t lane = lane_id();
-  uint32_t* hist = cmp + 2u * kPairPrefix;
+  uint32_t* hist = cmp + 2u * kPairPrefix + 2u * kQueueCap;
   if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
-  close_small<true>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols, hist);
+  close_small<true>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols,
+                    reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), hist);
   __syncwarp();
   unsigned __int128 t = 0;
   const uint32_t words = (r + 1u) * (kSmallMax + 1u);
@@ -574,7 +671,7 @@ __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, ui
       if (open && kr >= h) t += (unsigned __int128)times * binom_at(binom, cols, drop + x, kr - h);
     }
   }
-  if (lane == 0) cmp[0] = 1u + (cmp[kPairPrefix + 32u] >> 5);
+  if (lane == 0) cmp[0] = 1u + (cmp[kPairPrefix + 32u] >> 4);
   __syncwarp();
   return t;
 }
@@ -1771,7 +1868,8 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   // counts, the drop list, else the compact bitmap of a node counted whole
   const bool mk = pivot && p.nk != 0;
   bool compact = pivot && !lp.local;
-  const size_t sCmp = mk ? 2 * kPairPrefix + kHistWords : compact_words(dcap) + kPairPrefix;
+  // (rows and prefix, then the stack of small nodes; triangles use the same words for wider rows)
+  const size_t sCmp = std::max<size_t>(2 * kPairPrefix + 2 * kQueueCap + (mk ? kHistWords : 0), compact_words(dcap));
   const size_t frame_words = al4((size_t)depth * fw);
   auto pstride_of = [&]() {
     return frame_words + (pivot ? al4(dcap) * (lp.local ? 2 : 1) : 0) + (compact ? al4(sCmp) : 0);

@@ -273,7 +273,12 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
   // edges (u, v) are the root branches, each with the subproblem
   // N+(u) ∩ N+(v), the row of v. Orientation listing walks exactly those
   // branches for a node unit, so there the grouped form is the node form.
-  const bool grouped = req.unit == KC_UNIT_EDGE && req.encoding == KC_ENC_BITMAP && g->max_out <= 1024;
+  // The list encoding is the encoding of the units above 1024 vertices, where
+  // a bitmap's |S|^2 bits no longer fit shared memory; below that G[S] is held
+  // as bitmaps in either encoding (R-MAT scale 14, k = 4, units of up to 121
+  // vertices: lists took 5.2 ms, bitmaps take 0.31 ms).
+  const bool lists = req.encoding == KC_ENC_LIST && g->max_out > 1024;
+  const bool grouped = req.unit == KC_UNIT_EDGE && g->max_out <= 1024;
   pl->edge = req.unit == KC_UNIT_EDGE && !grouped;
   pl->edge_roots = grouped;
   pl->d_out = d_out;
@@ -296,7 +301,7 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
   // queue, then the heavy list), an active-unit word per CTA per launch, and
   // the exited CTAs of each class launch.
   const bool helping = ctx->tail_help && req.help && req.mode != KC_MODE_ORIENT &&
-                       req.encoding == KC_ENC_BITMAP && req.d_local == nullptr;
+                       !lists && req.d_local == nullptr;
   const size_t exit_at = 2 * (size_t)nu + (size_t)(kNumClasses + 1) * kHelpMaxGrid;
   if (helping) {
     pl->help_words = exit_at + kNumClasses;
@@ -305,12 +310,11 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
   // Per-launch algorithm: orientation or pivot as requested; KC_MODE_AUTO
   // lists small units by orientation (cheap when their neighbourhood holds few
   // cliques) and counts large units and over-budget units with the pivot.
-  const bool budget_ok = req.encoding == KC_ENC_BITMAP;
   auto launch_mode = [&](bool warp_group, bool heavy_pass) -> uint32_t {
     if (req.mode != KC_MODE_AUTO) return req.mode;
     // orientation listing only where a budget can hand a clique-heavy unit
-    // on to the pivot; without one (list encoding) AUTO pivots everywhere
-    return (warp_group && !heavy_pass && budget_ok) ? (uint32_t)KC_MODE_ORIENT : (uint32_t)KC_MODE_PIVOT;
+    // on to the pivot
+    return (warp_group && !heavy_pass) ? (uint32_t)KC_MODE_ORIENT : (uint32_t)KC_MODE_PIVOT;
   };
   bool any_budget = false;
   for (int c = 0; c <= kNumClasses; ++c) {
@@ -320,7 +324,7 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
     const bool warp_group = !heavy_pass && kClasses[c].G == 32;
     LaunchPlan lp;
     lp.mode = launch_mode(warp_group, heavy_pass);
-    lp.encoding = req.encoding;
+    lp.encoding = lists && c == 0 ? (uint32_t)KC_ENC_LIST : (uint32_t)KC_ENC_BITMAP;
     lp.edge = pl->edge;
     lp.dcap = heavy_pass ? std::max<uint32_t>(1, std::min<uint32_t>(kWarpClassMax, pl->max_size))
                          : (uint32_t)std::max<int64_t>(1, std::min<int64_t>(kClasses[c].hi, pl->max_size));
@@ -365,7 +369,7 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
                                           : nullptr;
     p.time_limit_ns = ctx->time_limit_ns;
     p.t0 = reinterpret_cast<const unsigned long long*>(pl->scratch + kStartWord);
-    if (warp_group && budget_ok) {
+    if (warp_group) {
       p.budget = lp.mode == KC_MODE_PIVOT ? kPivotUnitBudget : kUnitBudget;
       p.heavy = pl->heavy;
       p.heavy_count = pl->scratch + kHeavyBounds + 1;

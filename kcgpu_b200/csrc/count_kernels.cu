@@ -223,14 +223,15 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
 // costs a warp about 1.5 us of latency per tree node (frame, candidate list,
 // scores, reductions) with most lanes idle, and almost all nodes of a tree are
 // small and near its leaves. Two kinds are therefore counted whole: r = 3 with
-// at most 128 candidates (triangles, edges and vertices of G[F]) and r in
-// 4..19 with at most 32 candidates (a lane per subproblem).
+// at most 128 candidates (the triangles of G[F]) and r up to 19 with at most 32
+// candidates (a lane per subproblem).
 // Both first copy G[F] into a compact bitmap of nc rows and ceil(nc / 32)
 // words. Larger nodes are worth splitting further: their branches are what
 // the walkers share. R-MAT scale 17, k = 5 (edge units): 37.8M tree nodes,
 // 37.1 ms before; 1.4M, 6.3 ms now. Chung-Lu 1M + planted cliques, k = 6
-// (node units): 76.7M, 145 ms before; 3.7M, 48 ms now. R-MAT of 21k edges,
-// k = 8, built, oriented and counted: 3.5 ms before, 1.6 ms now.
+// (node units): 76.7M, 145 ms before; 3.7M, 48 ms now (r = 4 closed the same
+// way, a triangle count per vertex, took 42 ms where this had come to 30).
+// R-MAT of 21k edges, k = 8, built, oriented and counted: 3.5 ms before, 1.6 ms.
 
 // The compact bitmap of the candidates cand[0, nc) (ascending): bit i of row j
 // is set when cand[i] and cand[j] are adjacent (UPPER: and i > j). The lanes
@@ -249,23 +250,26 @@ __device__ __forceinline__ void compact_rows(const uint32_t* B, uint32_t Ws, con
     cw[t] = c >> 5;
     cb[t] = i < nc ? (1u << (c & 31u)) : 0u;
   }
-#pragma unroll 4
-  for (uint32_t j = 0; j < nc; ++j) {
-    const uint32_t* row = B + cand[j] * Ws;
-    uint32_t m[ST];
 #pragma unroll
-    for (int t = 0; t < ST; ++t) {
-      m[t] = 0u;
-      if (t < NW) {
-        m[t] = __ballot_sync(0xffffffffu, (row[cw[t < NW ? t : 0]] & cb[t < NW ? t : 0]) != 0u);
-        if (UPPER)
-          m[t] &= (uint32_t)t > (j >> 5) ? 0xffffffffu : ((uint32_t)t == (j >> 5) ? 0xfffffffeu << (j & 31u) : 0u);
+  for (int jb = 0; jb < NW; ++jb) {  // rows 32 jb .. 32 jb + 31
+    const uint32_t je = min(nc, (uint32_t)jb * 32u + 32u);
+#pragma unroll 4
+    for (uint32_t j = (uint32_t)jb * 32u; j < je; ++j) {
+      const uint32_t* row = B + cand[j] * Ws;
+      uint32_t m[ST];
+#pragma unroll
+      for (int t = 0; t < ST; ++t) {
+        m[t] = 0u;
+        if (t < NW && (!UPPER || t >= jb)) {
+          m[t] = __ballot_sync(0xffffffffu, (row[cw[t < NW ? t : 0]] & cb[t < NW ? t : 0]) != 0u);
+          if (UPPER && t == jb) m[t] &= 0xfffffffeu << (j & 31u);
+        }
       }
-    }
-    if (lane == 0) {
-      if constexpr (ST == 4) *reinterpret_cast<uint4*>(out + j * 4u) = make_uint4(m[0], m[1], m[2], m[3]);
-      else if constexpr (ST == 2) *reinterpret_cast<uint2*>(out + j * 2u) = make_uint2(m[0], m[1]);
-      else out[j] = m[0];
+      if (lane == 0) {
+        if constexpr (ST == 4) *reinterpret_cast<uint4*>(out + j * 4u) = make_uint4(m[0], m[1], m[2], m[3]);
+        else if constexpr (ST == 2) *reinterpret_cast<uint2*>(out + j * 2u) = make_uint2(m[0], m[1]);
+        else out[j] = m[0];
+      }
     }
   }
   __syncwarp();
@@ -287,54 +291,67 @@ struct BitCount {
   __device__ __forceinline__ uint32_t total() const { return 4u * fours + 2u * __popc(twos) + __popc(ones); }
 };
 
-// Triangles of a graph of nc <= 32 NW vertices whose upper rows (ST words
-// each, zero rows up to a multiple of four) are in up: lane i keeps rows i,
-// i + 32, .., every row j is broadcast to all lanes, and a lane whose row holds
-// j adds the common upper neighbours. No divergence and no bank conflicts,
-// about nc^2 / 64 words per lane whatever the density. Returns the lane's
-// share of the triangles and, in edges, of the edges.
+// The upper rows i, i + 32, .. (ST words each) of lane i, from up; returns the
+// lane's share of the edges.
 template <int NW, int ST>
-__device__ __forceinline__ uint32_t count_triangles(const uint32_t* up, uint32_t nc, uint32_t& edges) {
-  const uint32_t lane = lane_id();
-  uint32_t P[NW][ST];
-  edges = 0;
+__device__ __forceinline__ uint32_t own_rows(const uint32_t* up, uint32_t nc, uint32_t (&P)[NW][ST]) {
+  uint32_t edges = 0;
 #pragma unroll
   for (int g = 0; g < NW; ++g) {
-    const uint32_t i = (uint32_t)g * 32u + lane;
+    const uint32_t i = (uint32_t)g * 32u + lane_id();
 #pragma unroll
     for (int w = 0; w < ST; ++w) P[g][w] = 0u;
-    if (i < nc) {
-      if constexpr (ST > 1) {
-        load_row<ST>(up, i, P[g]);
-      } else {
-        P[g][0] = up[i];
-      }
-    }
+    if (i < nc) load_row<ST>(up, i, P[g]);
 #pragma unroll
     for (int w = g; w < NW; ++w) edges += __popc(P[g][w]);
   }
+  return edges;
+}
+
+// Four upper rows j0 .. j0 + 3 of block jb, the same for every lane.
+template <int ST>
+__device__ __forceinline__ void four_rows(const uint32_t* up, uint32_t j0, uint32_t (&U)[4][ST]) {
+  if constexpr (ST == 1) {
+    load_row<4>(up + j0, 0u, *reinterpret_cast<uint32_t(*)[4]>(&U[0][0]));
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) load_row<ST>(up, j0 + (uint32_t)q, U[q]);
+  }
+}
+
+// Common upper neighbours of the lane's row P (words from jb on) and of those
+// of the four rows U that it holds (bits j0 .. j0 + 3 of block jb).
+template <int NW, int ST>
+__device__ __forceinline__ void add_common(BitCount& bc, const uint32_t (&P)[ST], const uint32_t (&U)[4][ST], int jb,
+                                           uint32_t j0) {
+  uint32_t has[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) has[q] = 0u - ((P[jb] >> ((j0 + (uint32_t)q) & 31u)) & 1u);
+#pragma unroll
+  for (int w = 0; w < NW; ++w)
+    if (w >= jb)
+      bc.add4(P[w] & U[0][w] & has[0], P[w] & U[1][w] & has[1], P[w] & U[2][w] & has[2], P[w] & U[3][w] & has[3]);
+}
+
+// Triangles of a graph of nc <= 32 NW vertices whose upper rows (zero rows up
+// to a multiple of four) are in up: every row j is broadcast to all lanes, and
+// a lane whose rows hold j adds the common upper neighbours. No divergence and
+// no bank conflicts, about nc^2 / 64 words per lane whatever the density.
+// Returns the lane's share of the triangles and, in edges, of the edges.
+template <int NW, int ST>
+__device__ __forceinline__ uint32_t count_triangles(const uint32_t* up, uint32_t nc, uint32_t& edges) {
+  uint32_t P[NW][ST];
+  edges = own_rows<NW, ST>(up, nc, P);
   BitCount bc;
 #pragma unroll
   for (int jb = 0; jb < NW; ++jb) {  // rows 32 jb .. 32 jb + 31
     const uint32_t je = min(nc, (uint32_t)jb * 32u + 32u);
     for (uint32_t j0 = (uint32_t)jb * 32u; j0 < je; j0 += 4u) {
       uint32_t U[4][ST];
-      if constexpr (ST == 1) {
-        load_row<4>(up + j0, 0u, *reinterpret_cast<uint32_t(*)[4]>(&U[0][0]));
-      } else {
+      four_rows<ST>(up, j0, U);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) load_row<ST>(up, j0 + (uint32_t)q, U[q]);
-      }
-#pragma unroll
-      for (int g = 0; g <= jb; ++g) {
-        uint32_t has[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) has[q] = 0u - ((P[g][jb] >> ((j0 + (uint32_t)q) & 31u)) & 1u);
-#pragma unroll
-        for (int w = jb; w < NW; ++w)
-          bc.add4(P[g][w] & U[0][w] & has[0], P[g][w] & U[1][w] & has[1], P[g][w] & U[2][w] & has[2],
-                  P[g][w] & U[3][w] & has[3]);
-      }
+      for (int g = 0; g < NW; ++g)
+        if (g <= jb) add_common<NW, ST>(bc, P[g], U, jb, j0);
     }
   }
   return bc.total();
@@ -346,8 +363,8 @@ __host__ __device__ constexpr uint32_t compact_words(uint32_t n) {
   return n <= 32u ? 36u : (n <= 64u ? 64u * 2u : 128u * 4u);
 }
 constexpr uint32_t kPairPrefix = 36;   // close_small: exclusive prefix of the row lengths
-constexpr uint32_t kTriangleMax = 128; // most candidates of an r = 3 node closed whole
-constexpr uint32_t kSmallMax = 32;     // most candidates of an r > 3 node closed whole
+constexpr uint32_t kWideMax = 128;     // most candidates of an r = 3 node closed whole
+constexpr uint32_t kSmallMax = 32;     // most candidates of any other node closed whole
 constexpr int kSmallStack = 16;        // close_small: a lane's own frames (r - 3 at most)
 constexpr uint32_t kSmallMaxR = 19;
 constexpr uint32_t kQueueCap = 236;    // close_small: nodes on its shared stack
@@ -358,19 +375,16 @@ constexpr uint32_t kHistWords = (kSmallMaxRMulti + 1u) * (kSmallMax + 1u);
 // r = 3: triangles + drop edges + C(drop, 2) vertices + C(drop, 3). Every lane
 // returns its share.
 template <int NW, int ST>
-__device__ __forceinline__ unsigned long long close_triangles(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
-                                                           uint32_t nc, uint32_t* up, uint32_t drop) {
+__device__ __forceinline__ unsigned long long close_wide(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
+                                                         uint32_t nc, uint32_t* up, uint32_t drop) {
   const uint32_t pad = (nc + 3u) & ~3u;
   if (lane_id() < (pad - nc) * ST) up[nc * ST + lane_id()] = 0u;  // (nc is at most 32 NW, a multiple of four)
   compact_rows<NW, ST, true>(B, Ws, cand, nc, up);
   uint32_t edges = 0;
+  const unsigned long long d1 = drop, d2 = drop >= 2u ? d1 * (d1 - 1ull) / 2ull : 0ull;
   unsigned long long t = count_triangles<NW, ST>(up, nc, edges);
-  const unsigned long long d = drop;
-  t += d * edges;
-  if (lane_id() == 0) {
-    if (d >= 2ull) t += d * (d - 1ull) / 2ull * nc;
-    if (d >= 3ull) t += d * (d - 1ull) / 2ull * (d - 2ull) / 3ull;
-  }
+  t += d1 * edges;
+  if (lane_id() == 0) t += d2 * nc + (drop >= 3u ? d2 * (d1 - 2ull) / 3ull : 0ull);
   return t;
 }
 
@@ -618,7 +632,7 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
 }
 
 // A node counted whole (see above): its candidates are cand[0, nc), or, with
-// cand null, its symmetric rows of one word are B itself. One copy of this
+// cand null (r > 3, nc <= 32), its symmetric rows of one word are B itself. One copy of this
 // code serves every call site. The lane's share is returned and cmp[0] holds
 // the node's cost, in tree nodes of the work budget.
 __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t Ws, const uint32_t* cand, uint32_t nc,
@@ -626,20 +640,20 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
                                                      const unsigned long long* binom, uint32_t cols) {
   unsigned __int128 t;
   uint32_t cost = 1u + (nc >> 5);
-  if (r > 3u) {
+  if (r > 3u && nc <= kSmallMax) {
     if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
     t = close_small<false>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols,
                            reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), nullptr);
     __syncwarp();
     cost = 1u + (cmp[kPairPrefix + 32u] >> 4);
   } else if (nc <= 32u) {
-    t = close_triangles<1, 1>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<1, 1>(B, Ws, cand, nc, cmp, drop);
   } else if (nc <= 64u) {
-    t = close_triangles<2, 2>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<2, 2>(B, Ws, cand, nc, cmp, drop);
   } else if (nc <= 96u) {
-    t = close_triangles<3, 4>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<3, 4>(B, Ws, cand, nc, cmp, drop);
   } else {
-    t = close_triangles<4, 4>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<4, 4>(B, Ws, cand, nc, cmp, drop);
   }
   __syncwarp();
   if (lane_id() == 0) cmp[0] = cost;
@@ -1298,7 +1312,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           }
         }
       }
-    } else if (MODE == 1 && compact && (d <= kSmallMax || (!mk && d <= kTriangleMax && k == (p.edge_units ? 5u : 4u))) &&
+    } else if (MODE == 1 && compact && (d <= kSmallMax || (!mk && d <= kWideMax && k == (p.edge_units ? 5u : 4u))) &&
                k <= (mk ? kSmallMaxRMulti : kSmallMaxR)) {
       // ---- a unit counted whole (edge roots: their sum is the unit's count)
       const uint32_t r = k - (p.edge_units ? 2u : 1u);  // >= 3 here
@@ -1309,7 +1323,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         if constexpr (MK)  // the k with k - hold0 <= 2 are closed already
           uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r), kon && kl + r >= k + 3u);
         else
-          uacc += close_node(B, Ws, r > 3u ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
+          uacc += close_node(B, Ws, r > 3u && d <= kSmallMax ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
         st_words += 32u * cmp[0];
       }
     } else {
@@ -1444,9 +1458,9 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           return false;
         }
         // a small node is counted whole: the walker that owns it copies G[F]
-        // and counts it (see close_triangles and close_small)
+        // and counts it (see close_node)
         auto small = [&](uint32_t n) {
-          return compact && r >= 3u && n <= (!mk && r == 3u ? kTriangleMax : kSmallMax) &&
+          return compact && r >= 3u && n <= (!mk && r == 3u ? kWideMax : kSmallMax) &&
                  r <= (mk ? kSmallMaxRMulti : kSmallMaxR);
         };
         bool whole = small(nc);

@@ -504,7 +504,9 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
     const uint32_t P0 = (nc < 32u ? (1u << nc) - 1u : 0xffffffffu) & ~uni0;
     const uint32_t d0 = drop + (uint32_t)__popc(uni0);
     uint32_t top = 0;
-    if (P0 == 0u) {
+    if (!MK && __reduce_max_sync(0xffffffffu, s0) + 1u + drop < r) {
+      // no clique of F is large enough
+    } else if (P0 == 0u) {
       if (lane == 0) leaf(r, d0);
     } else {
       const bool in = (P0 >> lane) & 1u;
@@ -550,11 +552,13 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
                   else best = max(best, ((s + 1u) << 16) | u);
                   ++it;
                 }
+                const uint32_t most = uni ? n : best >> 16;  // no clique of P has more vertices
+                const bool enough = MK || most + dd >= rr;
                 dd += __popc(uni);
                 P &= ~uni;
                 if (P == 0u) {
                   leaf(rr, dd);
-                } else {
+                } else if (enough) {
                   open = true;
                   piv = best & 31u;
                   R = P & ~adj[piv] & ~(1u << piv);
@@ -1555,6 +1559,12 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
           if (own) uacc += (unsigned __int128)(esum / 2u) + (unsigned __int128)drop * nc + binom(drop, 2u);
           kopen = false;
         }
+        // no clique of G[F] has more vertices than the best score + 1 (one k: a
+        // node whose cliques and pivots together cannot reach k counts nothing)
+        if (!mk && !LOCAL) {
+          const uint32_t top = um != 0u ? nc - 1u : best >> 16;
+          if (__reduce_max_sync(pt.pmask, top) + 1u + drop < r) return false;
+        }
         if (univ && __any_sync(pt.pmask, um != 0u)) {
           const uint32_t nu = __reduce_add_sync(pt.pmask, (uint32_t)__popc(um));
           for (uint32_t x = um; x; x &= x - 1u) {
@@ -1646,6 +1656,16 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
       // branch, a branch of the top frame, or the top frame's pivot branch in
       // that frame's own slot), enters it, and pushes or drops its frame.
       enum Step { kRoot, kBranch, kPivot };
+      const bool direct = L == 1u && narrow;
+      uint32_t r0cnt = 0, r0incl = 0;  // lane w: branches in R0[w], and in R0[0, w]
+      if (direct) {
+        r0cnt = pt.plane < W ? (uint32_t)__popc(R0[pt.plane]) : 0u;
+        r0incl = r0cnt;
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(pt.pmask, r0incl, o);
+          if (pt.plane >= o) r0incl += y;
+        }
+      }
       int lv = -1;  // top frame
       uint32_t v = 0;  // root branches below v are done
       for (;;) {
@@ -1655,18 +1675,30 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         uint32_t hold, drop, held;  // held: the vertex that the node's branch holds
         bool own, above;
         if (lv < 0) {
-          // the next root branch
-          while (v < d) {
-            const uint32_t x = R0[v >> 5] >> (v & 31u);
-            if (x) {
-              v += (uint32_t)__ffs(x) - 1u;
-              break;
+          // the next root branch: with the cut at depth 1 and a bitmap row in a
+          // warp's lanes, a ticket is a branch number and its branch is found
+          // by the branches' prefix (stepping over the others' branches, 140 of
+          // them in a sparse unit, took a third of the walk); else in order
+          if (direct) {
+            const uint32_t t = mine;
+            if (t >= nr0) break;
+            mine = ticket();
+            const uint32_t w = (uint32_t)__popc(__ballot_sync(pt.pmask, r0incl <= t));
+            const uint32_t before = __shfl_sync(pt.pmask, r0incl - r0cnt, w);
+            held = w * 32u + select_bit(R0[w], t - before);
+          } else {
+            while (v < d) {
+              const uint32_t x = R0[v >> 5] >> (v & 31u);
+              if (x) {
+                v += (uint32_t)__ffs(x) - 1u;
+                break;
+              }
+              v = (v | 31u) + 1u;
             }
-            v = (v | 31u) + 1u;
+            if (v >= d) break;
+            held = v++;
+            if (L == 1u && !claim()) continue;
           }
-          if (v >= d) break;
-          held = v++;
-          if (L == 1u && !claim()) continue;
           step = kRoot;
           own = L == 1u || top_owner;
           above = L > 1u;

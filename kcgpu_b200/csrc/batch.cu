@@ -354,15 +354,18 @@ kc_status run_batch(kc_ctx* ctx, const uint32_t* src, const uint32_t* dst, Input
   if (st == KC_OK) {
     bool deep = false;
     for (auto& pl : plans) {
-      unsigned long long sv[kStatsCount] = {};
-      uint32_t err = count_error(pl, s, sv);
-      if (err == DEV_ERR_STACK) deep = true;
-      else if (err && st == KC_OK) st = device_error_status(err);
-      for (int q = 0; q < kStatsCount; ++q) trav[q] += sv[q];
-      heavy_units += count_heavy(pl, s);
-      units += count_units(pl, s);
-      kernels += 5;
-      for (int c = 0; c <= kNumClasses; ++c) kernels += pl.active[c] ? 1 : 0;
+      PassResult res;
+      const kc_status rs = count_readback(pl, s, &res, nullptr, 0);
+      if (rs != KC_OK) {
+        if (st == KC_OK) st = rs;
+        break;
+      }
+      if (res.err == DEV_ERR_STACK) deep = true;
+      else if (res.err && st == KC_OK) st = device_error_status(res.err);
+      for (int q = 0; q < kStatsCount; ++q) trav[q] += res.stats[q];
+      heavy_units += res.heavy;
+      units += res.units;
+      kernels += count_kernels(pl);
     }
     if (st == KC_OK && deep) {
       // a clique tree deeper than the fast stack: rerun every pass with full depth
@@ -374,8 +377,9 @@ kc_status run_batch(kc_ctx* ctx, const uint32_t* src, const uint32_t* dst, Input
         st = count_prepare(&U, req, dout, 1, &plans[i]);
         if (st == KC_OK) st = count_enqueue(plans[i], s);
         if (st == KC_OK) {
-          uint32_t err = count_error(plans[i], s, nullptr);
-          if (err) st = device_error_status(err);
+          PassResult res;
+          st = count_readback(plans[i], s, &res, nullptr, 0);
+          if (st == KC_OK && res.err) st = device_error_status(res.err);
         }
       }
     }

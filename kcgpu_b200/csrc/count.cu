@@ -50,30 +50,35 @@ const ClassSpec kClasses[kNumClasses] = {
 };
 __constant__ uint32_t kClassLo[kNumClasses - 1] = {1024, 128, 32};  // lower bounds of classes 0..2
 
-// Size class of every unit (kNumClasses = dropped: it cannot hold a k-clique).
+// Size class of unit i (kNumClasses = dropped: it cannot hold a k-clique).
+__device__ __forceinline__ uint32_t unit_class(uint32_t i, const uint32_t* __restrict__ drp,
+                                               const uint32_t* __restrict__ dcol, const uint32_t* __restrict__ erow,
+                                               int edge, const uint32_t* __restrict__ vgraph,
+                                               const uint32_t* __restrict__ gk, uint32_t k0) {
+  uint32_t s, src;
+  if (!edge) {
+    src = i;
+    s = drp[i + 1] - drp[i];
+  } else {
+    src = erow[i];
+    const uint32_t v = dcol[i];
+    s = min(drp[src + 1] - drp[src], drp[v + 1] - drp[v]);
+  }
+  const uint32_t k = gk ? gk[vgraph ? vgraph[src] : 0u] : k0;
+  bool keep;
+  if (k == 0xffffffffu || k == 0u) keep = false;  // graph not in this pass
+  else if (edge) keep = k >= 2u && s >= k - 2u;
+  else keep = s >= k - 1u;
+  if (!keep) return (uint32_t)kNumClasses;
+  return s > kClassLo[0] ? 0u : (s > kClassLo[1] ? 1u : (s > kClassLo[2] ? 2u : 3u));
+}
+
 __global__ void k_unit_class(const uint32_t* __restrict__ drp, const uint32_t* __restrict__ dcol,
                              const uint32_t* __restrict__ erow, uint32_t n_units, int edge,
                              const uint32_t* __restrict__ vgraph, const uint32_t* __restrict__ gk, uint32_t k0,
                              uint8_t* cls) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_units; i += gridDim.x * blockDim.x) {
-    uint32_t s, src;
-    if (!edge) {
-      src = i;
-      s = drp[i + 1] - drp[i];
-    } else {
-      src = erow[i];
-      const uint32_t v = dcol[i];
-      s = min(drp[src + 1] - drp[src], drp[v + 1] - drp[v]);
-    }
-    const uint32_t k = gk ? gk[vgraph ? vgraph[src] : 0u] : k0;
-    bool keep;
-    if (k == 0xffffffffu || k == 0u) keep = false;  // graph not in this pass
-    else if (edge) keep = k >= 2u && s >= k - 2u;
-    else keep = s >= k - 1u;
-    uint8_t c = (uint8_t)kNumClasses;
-    if (keep) c = s > kClassLo[0] ? 0 : (s > kClassLo[1] ? 1 : (s > kClassLo[2] ? 2 : 3));
-    cls[i] = c;
-  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_units; i += gridDim.x * blockDim.x)
+    cls[i] = (uint8_t)unit_class(i, drp, dcol, erow, edge, vgraph, gk, k0);
 }
 
 // Stable partition of the units by class, in two passes over chunks of
@@ -159,6 +164,94 @@ __global__ void k_class_bounds(const uint32_t* __restrict__ off, uint32_t n_chun
     bounds[2 * c] = cnt > shard ? b + shard : b;
     bounds[2 * c + 1] = cnt > shard ? (cnt - shard + n_shards - 1) / n_shards : 0u;
   }
+}
+
+// The queue of a small graph in one launch of one CTA: zeroes the plan's
+// scratch, classifies the units, partitions them (stable, as above) and writes
+// the class bounds. Up to kSmallQueue units (16 per thread, their classes kept
+// in registers) that takes less than the six launches it replaces cost in
+// launch gaps: G(2000, 0.01), k = 4: 105 us a count before, 37 us with this,
+// one read-back and no heavy pass where none can be needed.
+constexpr uint32_t kSmallThreads = 1024, kSmallRounds = 16, kSmallQueue = kSmallThreads * kSmallRounds;
+
+__global__ void __launch_bounds__(kSmallThreads) k_queue_small(const uint32_t* __restrict__ drp,
+                                                               const uint32_t* __restrict__ dcol,
+                                                               const uint32_t* __restrict__ erow, uint32_t n_units,
+                                                               int edge, const uint32_t* __restrict__ vgraph,
+                                                               const uint32_t* __restrict__ gk, uint32_t k0,
+                                                               uint32_t* queue, uint32_t* scratch, uint32_t shard,
+                                                               uint32_t n_shards) {
+  static_assert(kNumClasses == 4, "a class and `dropped` fit three bits");
+  constexpr uint32_t kWarps = kSmallThreads / 32;
+  __shared__ uint32_t total[kNumClasses], run[kNumClasses];
+  __shared__ uint32_t wc[kNumClasses][kWarps];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  for (uint32_t i = tid; i < kScratchWords; i += kSmallThreads) scratch[i] = 0;
+  if (tid < kNumClasses) total[tid] = 0;
+  __syncthreads();
+  unsigned long long mine = 0;  // three bits per round
+  const uint32_t rounds = (n_units + kSmallThreads - 1) / kSmallThreads;
+  for (uint32_t r = 0; r < rounds; ++r) {
+    const uint32_t i = r * kSmallThreads + tid;
+    const uint32_t c = i < n_units ? unit_class(i, drp, dcol, erow, edge, vgraph, gk, k0) : (uint32_t)kNumClasses;
+    mine |= (unsigned long long)c << (3u * r);
+#pragma unroll
+    for (int q = 0; q < kNumClasses; ++q) {
+      const uint32_t m = __ballot_sync(0xffffffffu, c == (uint32_t)q);
+      if (lane == 0 && m) atomicAdd(&total[q], (uint32_t)__popc(m));
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    *reinterpret_cast<unsigned long long*>(scratch + kStartWord) = global_ns();
+    uint32_t b = 0;
+    for (int c = 0; c < kNumClasses; ++c) {
+      const uint32_t cnt = total[c];
+      run[c] = b;
+      scratch[kClassBounds + 2 * c] = cnt > shard ? b + shard : b;
+      scratch[kClassBounds + 2 * c + 1] = cnt > shard ? (cnt - shard + n_shards - 1) / n_shards : 0u;
+      b += cnt;
+    }
+  }
+  for (uint32_t r = 0; r < rounds; ++r) {
+    const uint32_t c = (uint32_t)(mine >> (3u * r)) & 7u;
+    uint32_t rank = 0;
+#pragma unroll
+    for (int q = 0; q < kNumClasses; ++q) {
+      const uint32_t m = __ballot_sync(0xffffffffu, c == (uint32_t)q);
+      if (c == (uint32_t)q) rank = __popc(m & lanemask_lt());
+      if (lane == 0) wc[q][warp] = __popc(m);
+    }
+    __syncthreads();
+    if (warp < kNumClasses) {  // warp q: where every warp's units of class q go
+      const uint32_t v = wc[warp][lane];
+      uint32_t incl = v;
+#pragma unroll
+      for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const uint32_t base = run[warp];
+      wc[warp][lane] = base + incl - v;
+      if (lane == 31) run[warp] = base + incl;
+    }
+    __syncthreads();
+    if (c < (uint32_t)kNumClasses) queue[wc[c][warp] + rank] = r * kSmallThreads + tid;
+    __syncthreads();
+  }
+}
+
+// The most tree nodes orientation listing can visit in a unit of d vertices
+// for t-cliques: the j-subsets of d for j = 1 .. t - 1
+// (capped).
+uint64_t listing_bound(uint32_t d, uint32_t t) {
+  uint64_t sum = 0, c = 1;
+  for (uint32_t j = 1; j + 1 <= t && j <= d; ++j) {
+    c = c * (d - j + 1) / j;  // C(d, j)
+    sum += c;
+    if (sum > (1ull << 32)) break;
+  }
+  return sum;
 }
 
 uint32_t auto_part(uint32_t mode, uint32_t W) {
@@ -369,7 +462,8 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
                                           : nullptr;
     p.time_limit_ns = ctx->time_limit_ns;
     p.t0 = reinterpret_cast<const unsigned long long*>(pl->scratch + kStartWord);
-    if (warp_group) {
+    const uint32_t t_list = pl->edge ? (k_max >= 2 ? k_max - 2 : 0) : k_max - 1;
+    if (warp_group && (lp.mode == KC_MODE_PIVOT || listing_bound(lp.dcap, t_list) > kUnitBudget)) {
       p.budget = lp.mode == KC_MODE_PIVOT ? kPivotUnitBudget : kUnitBudget;
       p.heavy = pl->heavy;
       p.heavy_count = pl->scratch + kHeavyBounds + 1;
@@ -410,25 +504,38 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
 kc_status count_enqueue(const CountPlan& pl, cudaStream_t s) {
   kc_graph* g = pl.g;
   const int sms = pl.ctx->sms;
-  KC_CUDA(cudaMemsetAsync(pl.scratch, 0, sizeof(uint32_t) * kScratchWords, s));
   if (pl.help) KC_CUDA(cudaMemsetAsync(pl.help, 0, sizeof(uint32_t) * pl.help_words, s));
-  const uint32_t gq = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((pl.n_units + 255) / 256, (uint64_t)sms * 16));
-  if (pl.n_units)
+  if (pl.n_units <= kSmallQueue) {
+    k_queue_small<<<1, kSmallThreads, 0, s>>>(g->drp, g->dcol, g->erow, pl.n_units, pl.edge ? 1 : 0, g->vgraph,
+                                              pl.req.d_graph_k, pl.req.k, pl.queue, pl.scratch, pl.req.shard,
+                                              std::max(1u, pl.req.n_shards));
+  } else {
+    KC_CUDA(cudaMemsetAsync(pl.scratch, 0, sizeof(uint32_t) * kScratchWords, s));
+    const uint32_t gq = (uint32_t)std::min<uint64_t>((pl.n_units + 255) / 256, (uint64_t)sms * 16);
     k_unit_class<<<gq, 256, 0, s>>>(g->drp, g->dcol, g->erow, pl.n_units, pl.edge ? 1 : 0, g->vgraph,
                                     pl.req.d_graph_k, pl.req.k, pl.cls);
-  const uint32_t nc = pl.n_chunks;
-  if (pl.n_units) k_class_count<<<nc, kPartThreads, 0, s>>>(pl.cls, pl.n_units, nc, pl.ccnt);
-  else KC_CUDA(cudaMemsetAsync(pl.ccnt, 0, sizeof(uint32_t) * kNumClasses * (size_t)nc, s));
-  KC_CUDA(prim::scan_exclusive_u32(pl.ccnt, pl.ccnt, (size_t)kNumClasses * nc, s));
-  k_class_bounds<<<1, 32, 0, s>>>(pl.ccnt, nc, pl.scratch + kClassBounds,
-                                  reinterpret_cast<unsigned long long*>(pl.scratch + kStartWord), pl.req.shard,
-                                  std::max(1u, pl.req.n_shards));
-  if (pl.n_units) k_class_scatter<<<nc, kPartThreads, 0, s>>>(pl.cls, pl.n_units, nc, pl.ccnt, pl.queue);
+    const uint32_t nc = pl.n_chunks;
+    k_class_count<<<nc, kPartThreads, 0, s>>>(pl.cls, pl.n_units, nc, pl.ccnt);
+    KC_CUDA(prim::scan_exclusive_u32(pl.ccnt, pl.ccnt, (size_t)kNumClasses * nc, s));
+    k_class_bounds<<<1, 32, 0, s>>>(pl.ccnt, nc, pl.scratch + kClassBounds,
+                                    reinterpret_cast<unsigned long long*>(pl.scratch + kStartWord), pl.req.shard,
+                                    std::max(1u, pl.req.n_shards));
+    k_class_scatter<<<nc, kPartThreads, 0, s>>>(pl.cls, pl.n_units, nc, pl.ccnt, pl.queue);
+  }
   KC_CUDA(cudaGetLastError());
   // class launches side by side, then the heavy pass over the units they handed on
-  KC_CUDA(cudaEventRecord(pl.fork, s));
+  // (one class alone runs on s itself)
+  int classes = 0;
+  for (int c = 0; c < kNumClasses; ++c) classes += pl.active[c] ? 1 : 0;
+  if (classes > 1) KC_CUDA(cudaEventRecord(pl.fork, s));
   for (int c = 0; c < kNumClasses; ++c) {
     if (!pl.active[c]) continue;
+    if (classes == 1) {
+      if (pl.timed) KC_CUDA(cudaEventRecord(pl.tbeg[c], s));
+      KC_TRY(enqueue_launch(pl.launches[c], s));
+      if (pl.timed) KC_CUDA(cudaEventRecord(pl.tend[c], s));
+      break;
+    }
     KC_CUDA(cudaStreamWaitEvent(pl.side[c], pl.fork, 0));
     if (pl.timed) KC_CUDA(cudaEventRecord(pl.tbeg[c], pl.side[c]));
     KC_TRY(enqueue_launch(pl.launches[c], pl.side[c]));
@@ -450,41 +557,51 @@ kc_status device_error_status(uint32_t err) {
   return fail(KC_ERR_INTERNAL, "counting kernel reported device error %u", err);
 }
 
-uint32_t count_error(const CountPlan& pl, cudaStream_t s, unsigned long long* stats) {
+kc_status count_readback(const CountPlan& pl, cudaStream_t s, PassResult* r, unsigned long long* h_out, size_t n_out) {
   static_assert(kStatsWords + 2 * kStatsCount <= kClassBounds, "stats overlap the class bounds");
-  uint32_t h[kScratchWords];
-  cudaMemcpyAsync(h, pl.scratch, sizeof(h), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  if (stats) std::memcpy(stats, h + kStatsWords, kStatsCount * sizeof(unsigned long long));
-  return h[kErrWord];
+  static_assert(kScratchWords % 2 == 0 && kScratchWords * 4 + kPinOut * 8 <= kPinBytes, "page-locked buffer too small");
+  kc_ctx* ctx = pl.ctx;
+  if (n_out > kPinOut) return fail(KC_ERR_INTERNAL, "%zu counts to read back with a pass", n_out);
+  if (!ctx->pin) KC_CUDA(cudaHostAlloc(&ctx->pin, kPinBytes, cudaHostAllocDefault));
+  uint32_t* h = static_cast<uint32_t*>(ctx->pin);
+  unsigned long long* ho = reinterpret_cast<unsigned long long*>(h + kScratchWords);
+  KC_CUDA(cudaMemcpyAsync(h, pl.scratch, sizeof(uint32_t) * kScratchWords, cudaMemcpyDeviceToHost, s));
+  if (n_out) KC_CUDA(cudaMemcpyAsync(ho, pl.d_out, sizeof(unsigned long long) * n_out, cudaMemcpyDeviceToHost, s));
+  KC_CUDA(cudaStreamSynchronize(s));
+  r->err = h[kErrWord];
+  std::memcpy(r->stats, h + kStatsWords, sizeof(r->stats));
+  r->heavy = h[kHeavyBounds + 1];
+  r->units = 0;
+  for (int c = 0; c < kNumClasses; ++c) r->units += h[kClassBounds + 2 * c + 1];
+  if (n_out) std::memcpy(h_out, ho, sizeof(unsigned long long) * n_out);
+  return KC_OK;
 }
 
-uint32_t count_heavy(const CountPlan& pl, cudaStream_t s) {
-  uint32_t h = 0;
-  cudaMemcpyAsync(&h, pl.scratch + kHeavyBounds + 1, sizeof(h), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  return h;
+uint32_t count_kernels(const CountPlan& pl) {
+  uint32_t k = pl.n_units <= kSmallQueue ? 1u : 7u;  // the queue (its scan is three)
+  for (int c = 0; c <= kNumClasses; ++c) k += pl.active[c] ? 1u : 0u;
+  return k;
 }
 
-uint64_t count_units(const CountPlan& pl, cudaStream_t s) {
-  uint32_t b[2 * kNumClasses];
-  cudaMemcpyAsync(b, pl.scratch + kClassBounds, sizeof(b), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  uint64_t t = 0;
-  for (int c = 0; c < kNumClasses; ++c) t += b[2 * c + 1];
-  return t;
-}
-
-kc_status count_graph(kc_graph* g, const CountRequest& req, unsigned long long* d_out, kc_count_stats* stats) {
+kc_status count_graph(kc_graph* g, const CountRequest& req, unsigned long long* d_out, kc_count_stats* stats,
+                      unsigned long long* h_out) {
   kc_ctx* ctx = req.ctx ? req.ctx : g->ctx;
   cudaStream_t s = ctx->stream;
-  cudaEvent_t ev0, ev1;
-  cudaEventCreate(&ev0);
-  cudaEventCreate(&ev1);
+  struct Events {  // only for statistics
+    cudaEvent_t a = nullptr, b = nullptr;
+    ~Events() {
+      if (a) cudaEventDestroy(a);
+      if (b) cudaEventDestroy(b);
+    }
+  } ev;
+  if (stats) {
+    KC_CUDA(cudaEventCreate(&ev.a));
+    KC_CUDA(cudaEventCreate(&ev.b));
+  }
+  const size_t n_out = h_out ? 2 * (size_t)req.n_graphs * std::max(1u, req.nk) : 0;
   kc_status st = KC_OK;
   uint32_t kernels = 0;
-  uint64_t units = 0, heavy = 0;
-  unsigned long long sv[kStatsCount] = {};
+  PassResult res;
   double ms_launch[kNumClasses + 1] = {};
   uint32_t deep = 0;
   for (uint32_t boost = 0; boost < 2; ++boost) {
@@ -493,15 +610,12 @@ kc_status count_graph(kc_graph* g, const CountRequest& req, unsigned long long* 
     deep = boost;
     st = count_prepare(g, req, d_out, boost, &pl);
     if (st == KC_OK) {
-      if (boost == 0) cudaEventRecord(ev0, s);
+      if (stats && boost == 0) cudaEventRecord(ev.a, s);
       st = count_enqueue(pl, s);
-      cudaEventRecord(ev1, s);
+      if (stats) cudaEventRecord(ev.b, s);
     }
-    uint32_t err = 0;
+    if (st == KC_OK) st = count_readback(pl, s, &res, h_out, n_out);
     if (st == KC_OK) {
-      err = count_error(pl, s, sv);
-      units = count_units(pl, s);
-      heavy = count_heavy(pl, s);
       for (int c = 0; c <= kNumClasses; ++c) {
         float t = 0;
         if (pl.timed && pl.active[c] && cudaEventElapsedTime(&t, pl.tbeg[c], pl.tend[c]) == cudaSuccess)
@@ -509,38 +623,35 @@ kc_status count_graph(kc_graph* g, const CountRequest& req, unsigned long long* 
         else
           ms_launch[c] = 0;
       }
-      kernels = 5;
-      for (int c = 0; c <= kNumClasses; ++c) kernels += pl.active[c] ? 1 : 0;
+      kernels = count_kernels(pl);
     }
     count_release(&pl);
     if (st != KC_OK) break;
-    if (err == DEV_ERR_STACK && boost == 0 && req.mode != KC_MODE_ORIENT) {
+    if (res.err == DEV_ERR_STACK && boost == 0 && req.mode != KC_MODE_ORIENT) {
       // a clique tree deeper than the fast stack: rerun with the full depth
       KC_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long) * 2 * req.n_graphs * std::max(1u, req.nk), s));
       continue;
     }
-    if (err) st = device_error_status(err);
+    if (res.err) st = device_error_status(res.err);
     break;
   }
   if (stats && st == KC_OK) {
     float ms = 0;
-    cudaEventElapsedTime(&ms, ev0, ev1);
-    stats->units = units;
-    stats->tree_nodes = sv[0];
-    stats->word_ops = sv[1];
-    stats->gather_bytes = sv[2];
-    for (int q = 0; q < 3; ++q) stats->cycles[q] = sv[3 + q];
+    cudaEventElapsedTime(&ms, ev.a, ev.b);
+    stats->units = res.units;
+    stats->tree_nodes = res.stats[0];
+    stats->word_ops = res.stats[1];
+    stats->gather_bytes = res.stats[2];
+    for (int q = 0; q < 3; ++q) stats->cycles[q] = res.stats[3 + q];
     stats->ms_total = ms;
     stats->ms_traversal = ms;
     stats->max_unit_size = g->max_out;
     stats->kernels = kernels;
     for (int c = 0; c <= kNumClasses; ++c) stats->ms_launch[c] = ms_launch[c];
-    stats->heavy_units = heavy;
+    stats->heavy_units = res.heavy;
     stats->deep_retry = deep;
     stats->reserved = 0;
   }
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
   return st;
 }
 

@@ -1981,18 +1981,25 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
               : lp.local ? k_count_bitmap<1, true, false>
               : mk ? k_count_bitmap<1, false, true> : k_count_bitmap<1, false, false>;
   // Several classes launch the same kernel with different shared-memory sizes;
-  // the attribute is per function, so it is set to the device maximum.
+  // the attribute is per function, so it is set to the device maximum, once per
+  // context (and the occupancy is looked up once per launch shape).
   // (the kernel's static shared memory counts against the same per-block limit)
-  cudaFuncAttributes fa;
-  KC_CUDA(cudaFuncGetAttributes(&fa, kern));
-  if (fa.sharedSizeBytes > kStaticSmemBytes)
-    return fail(KC_ERR_INTERNAL, "counting kernel uses %zu bytes of static shared memory, planned for %zu",
-                fa.sharedSizeBytes, kStaticSmemBytes);
-  KC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               ctx->max_smem_optin - (int)fa.sharedSizeBytes));
-  int per_sm = 0;
-  KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem_bytes));
-  per_sm = std::max(1, per_sm);
+  if (ctx->kernel_static_smem.find((const void*)kern) == ctx->kernel_static_smem.end()) {
+    cudaFuncAttributes fa;
+    KC_CUDA(cudaFuncGetAttributes(&fa, kern));
+    if (fa.sharedSizeBytes > kStaticSmemBytes)
+      return fail(KC_ERR_INTERNAL, "counting kernel uses %zu bytes of static shared memory, planned for %zu",
+                  fa.sharedSizeBytes, kStaticSmemBytes);
+    KC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ctx->max_smem_optin - (int)fa.sharedSizeBytes));
+    ctx->kernel_static_smem[(const void*)kern] = (int)fa.sharedSizeBytes;
+  }
+  int& per_sm = ctx->occupancy[std::make_tuple((const void*)kern, block, smem_bytes)];
+  if (per_sm == 0) {
+    int found = 0;
+    KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&found, kern, block, smem_bytes));
+    per_sm = std::max(1, found);
+  }
   uint64_t grid = std::min<uint64_t>((uint64_t)ctx->sms * per_sm, ((uint64_t)p.n_units_max + gpb - 1) / gpb);
   grid = std::max<uint64_t>(1, grid);
   if (p.gbuf_words) {

@@ -165,12 +165,21 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
                         CountPlan* pl);
 kc_status count_enqueue(const CountPlan& pl, cudaStream_t s);
 void count_release(CountPlan* pl);
-// Reads the device error word (and the kStatsCount stats counters when stats != null).
-uint32_t count_error(const CountPlan& pl, cudaStream_t s, unsigned long long* stats);
+// What a pass left in its scratch.
+struct PassResult {
+  uint32_t err = 0;                            // device error word
+  unsigned long long stats[kStatsCount] = {};  // with statistics
+  uint64_t units = 0;                          // units queued
+  uint32_t heavy = 0;                          // units handed to the heavy pass
+};
+constexpr size_t kPinBytes = 1024;  // kc_ctx::pin: the scratch, then up to kPinOut counters
+constexpr size_t kPinOut = 64;      // (lo, hi) of 32 values of k
+// Waits for the pass and reads its scratch and, with it, n_out counters of its
+// output into h_out (page-locked staging: one synchronisation for all of it).
+kc_status count_readback(const CountPlan& pl, cudaStream_t s, PassResult* r, unsigned long long* h_out, size_t n_out);
+// Kernels one enqueue of the plan launches.
+uint32_t count_kernels(const CountPlan& pl);
 // The call's status for a non-zero device error word.
 kc_status device_error_status(uint32_t err);
-uint64_t count_units(const CountPlan& pl, cudaStream_t s);
-// Units the last enqueue handed to the heavy pass.
-uint32_t count_heavy(const CountPlan& pl, cudaStream_t s);
 
 }  // namespace kc

@@ -235,6 +235,7 @@ kc_status kc_ctx_destroy(kc_ctx* ctx) {
       if (ctx->tend[c]) cudaEventDestroy(ctx->tend[c]);
     }
     if (ctx->fork) cudaEventDestroy(ctx->fork);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->copy) {
       cudaStreamSynchronize(ctx->copy);
       cudaStreamDestroy(ctx->copy);
@@ -489,15 +490,12 @@ kc_status count_on(kc_ctx* run, kc_graph* g, const kc_params* p, kc_u128* out, k
   req.ctx = run;
   req.shard = shard;
   req.n_shards = n_shards;
-  kc_status st = kc::count_graph(g, req, d_out, (p->flags & KC_FLAG_STATS) ? stats : nullptr);
   unsigned long long h[2] = {0, 0};
+  const kc_status st = kc::count_graph(g, req, d_out, (p->flags & KC_FLAG_STATS) ? stats : nullptr, h);
   if (st == KC_OK) {
-    cudaError_t e = cudaMemcpyAsync(h, d_out, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) st = kc::cuda_fail(e, "count readback", __FILE__, __LINE__);
+    out->lo = h[0];
+    out->hi = h[1];
   }
-  out->lo = h[0];
-  out->hi = h[1];
   return st;
 }
 
@@ -542,14 +540,8 @@ kc_status count_multi_on(kc_ctx* run, kc_graph* g, const kc_params* p, const uin
   req.ctx = run;
   req.nk = nb;
   for (uint32_t i = 0; i < nb; ++i) req.kset[i] = big[i];
-  kc_status st = kc::count_graph(g, req, d_out, nullptr);
   std::vector<unsigned long long> h(2 * (size_t)nb, 0);
-  if (st == KC_OK) {
-    cudaError_t e = cudaMemcpyAsync(h.data(), d_out, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) st = kc::cuda_fail(e, "count readback", __FILE__, __LINE__);
-  }
-  if (st != KC_OK) return st;
+  KC_TRY(kc::count_graph(g, req, d_out, nullptr, h.data()));
   for (uint32_t i = 0; i < n_k; ++i) {
     if (ks[i] <= 2) continue;
     const size_t j = (size_t)(std::lower_bound(big.begin(), big.end(), ks[i]) - big.begin());
@@ -612,7 +604,7 @@ kc_status kc_count_local(kc_graph* g, const kc_params* p, kc_u128* per_vertex, k
   req.flags = 0;
   req.k_max = p->k;
   req.d_local = d_local;
-  kc_status st = kc::count_graph(g, req, d_out, nullptr);
+  kc_status st = kc::count_graph(g, req, d_out, nullptr, nullptr);
   std::vector<uint32_t> rank(n);
   unsigned long long h[2] = {0, 0};
   if (st == KC_OK) {

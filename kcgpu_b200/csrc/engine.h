@@ -2,7 +2,9 @@
 // and the stage entry points that the C ABI (engine.cu) strings together.
 #pragma once
 #include <cstdint>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -29,6 +31,11 @@ struct kc_ctx {
   kc::BlockCache cache;        // device blocks reused by allocations on `stream`
   uint64_t total_mem = 0;
   std::mutex mu;  // one call at a time per context
+  void* pin = nullptr;  // page-locked staging of a counting pass's read-back (created on first use)
+  // launch facts looked up once per context: kernels whose shared-memory limit
+  // is set, and CTAs per SM by (kernel, threads, shared memory)
+  std::map<const void*, int> kernel_static_smem;
+  std::map<std::tuple<const void*, uint32_t, size_t>, int> occupancy;
   // exact binomial table C(r, c) as (lo, hi) pairs, rows [0, brows], cols [0, bcols]
   unsigned long long* d_binom = nullptr;
   uint32_t brows = 0, bcols = 0;
@@ -126,9 +133,10 @@ struct CountRequest {
   bool help = true;
 };
 
-// Runs the counting stage; d_out holds n_graphs (lo, hi) pairs and must be zeroed.
+// Runs the counting stage; d_out holds n_graphs (lo, hi) pairs (nk of them with
+// several k) and must be zeroed. With h_out (one graph) they are read back too.
 kc_status count_graph(kc_graph* g, const CountRequest& req, unsigned long long* d_out,
-                      kc_count_stats* stats);
+                      kc_count_stats* stats, unsigned long long* h_out);
 // kc_count run by the context `run` (its stream, scratch and lock) on a graph
 // of the same device; the graph must be complete (see CountRequest::ctx).
 kc_status count_on(kc_ctx* run, kc_graph* g, const kc_params* p, kc_u128* out, kc_count_stats* stats,

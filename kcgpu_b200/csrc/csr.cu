@@ -144,7 +144,7 @@ kc_status build_csr(kc_graph* g, const uint32_t* d_src, const uint32_t* d_dst, u
   KC_CUDA(cudaGetLastError());
 
   KC_CUDA(tmp.alloc(&ucnt, sizeof(uint32_t) * ((size_t)n + 1)));
-  KC_CUDA(prim::segmented_sort_unique(off, adj, ucnt, n, h[1], s));
+  KC_CUDA(prim::segmented_sort_unique(off, adj, ucnt, n, h[1], n, s));
 
   // final offsets and compaction into the graph's own arrays
   KC_TRY(dev_alloc(g, (void**)&g->rp, sizeof(uint32_t) * ((size_t)n + 1)));

@@ -197,12 +197,17 @@ __global__ void __launch_bounds__(NT) k_radix_scatter(const unsigned long long* 
 
 // ---- segmented sort + dedup --------------------------------------------------
 
-enum RowClass { RC_TRIVIAL = 0, RC_WARP = 1, RC_B2K = 2, RC_B16K = 3, RC_B32K = 4, RC_HUGE = 5, RC_W256 = 6, RC_N = 7 };
+enum RowClass { RC_TRIVIAL = 0, RC_WARP = 1, RC_B2K = 2, RC_B16K = 3, RC_B32K = 4, RC_HUGE = 5, RC_W256 = 6, RC_W1K = 7, RC_N = 8 };
+
+// Rows above 1,024 entries whose values lie below this are sorted through a
+// bitmap of all values in shared memory (k_seg_bitmap), 128 KB at most.
+constexpr uint32_t kBitmapUniverse = 1u << 20;
 
 __device__ __forceinline__ int row_class(uint32_t len) {
   if (len <= 1) return RC_TRIVIAL;
   if (len <= 32) return RC_WARP;
   if (len <= 256) return RC_W256;
+  if (len <= 1024) return RC_W1K;
   if (len <= 2048) return RC_B2K;
   if (len <= 16384) return RC_B16K;
   if (len <= 32768) return RC_B32K;
@@ -260,8 +265,8 @@ __global__ void k_seg_warp(const uint32_t* __restrict__ off, uint32_t* data, uin
   }
 }
 
-// Warp per row for rows of 33..256 entries, sorted in registers: the row is
-// padded to N = 32 E entries (E = 2, 4 or 8) and held striped, element
+// Warp per row for rows of 33..1024 entries, sorted in registers: the row is
+// padded to N = 32 E entries (E = 2 to 32) and held striped, element
 // i = e * 32 + lane in register e of that lane, so loads and stores are
 // coalesced. Bitonic network: partners less than 32 apart are in other lanes
 // (one shuffle), farther partners are in another register of the same lane.
@@ -331,6 +336,72 @@ __global__ void __launch_bounds__(256) k_seg_warp_reg(const uint32_t* __restrict
     if (len <= 64) warp_sort_unique_row<2>(data, b, len, ucnt + r, lane);
     else if (len <= 128) warp_sort_unique_row<4>(data, b, len, ucnt + r, lane);
     else if (len <= 256) warp_sort_unique_row<8>(data, b, len, ucnt + r, lane);
+  }
+}
+
+// Rows of 257..1024 entries, in a kernel of their own for the registers. A CTA
+// per row sorting in shared memory took a barrier per stage (45 to 55 stages):
+// 155 us for R-MAT 18's rows of 257..2048, 21 us here.
+__global__ void __launch_bounds__(128) k_seg_warp_wide(const uint32_t* __restrict__ off, uint32_t* data, uint32_t* ucnt,
+                                                       const uint32_t* __restrict__ list, const uint32_t* count,
+                                                       uint32_t n_rows) {
+  const uint32_t lane = lane_id();
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t cnt = min(*count, n_rows);
+  for (uint32_t li = gw; li < cnt; li += nw) {
+    const uint32_t r = list[li];
+    const uint32_t b = off[r], len = off[r + 1] - b;
+    if (len <= 512) warp_sort_unique_row<16>(data, b, len, ucnt + r, lane);
+    else if (len <= 1024) warp_sort_unique_row<32>(data, b, len, ucnt + r, lane);
+  }
+}
+
+// CTA per row for rows above 1,024 entries with values below kBitmapUniverse:
+// every value sets its bit, and the bits in order are the sorted, distinct row.
+// Its cost is the row's plus universe / 32 words, where a bitonic sort of
+// 16,384 entries is 105 stages of barriers (0.3 ms on one CTA; R-MAT 18: the
+// long rows took 0.60 ms in two launches and a keyed radix sort of its largest
+// rows with a host synchronisation, 0.06 ms here).
+constexpr uint32_t kBitmapThreads = 1024;
+
+__global__ void __launch_bounds__(kBitmapThreads) k_seg_bitmap(const uint32_t* __restrict__ off, uint32_t* data,
+                                                               uint32_t* ucnt, const uint32_t* __restrict__ lists,
+                                                               const uint32_t* __restrict__ counts, uint32_t n_rows,
+                                                               uint32_t universe) {
+  extern __shared__ __align__(16) uint32_t bits[];
+  __shared__ uint32_t wsum[kBitmapThreads / 32];
+  const uint32_t tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+  const uint32_t words = (universe + 31u) / 32u;
+  const uint32_t per = (words + kBitmapThreads - 1u) / kBitmapThreads;  // words per thread, consecutive
+  const uint32_t c0 = min(counts[RC_B2K], n_rows), c1 = min(counts[RC_B16K], n_rows), c2 = min(counts[RC_B32K], n_rows),
+                 c3 = min(counts[RC_HUGE], n_rows);
+  for (uint32_t li = blockIdx.x; li < c0 + c1 + c2 + c3; li += gridDim.x) {
+    const uint32_t r = li < c0             ? lists[(size_t)RC_B2K * n_rows + li]
+                       : li < c0 + c1      ? lists[(size_t)RC_B16K * n_rows + (li - c0)]
+                       : li < c0 + c1 + c2 ? lists[(size_t)RC_B32K * n_rows + (li - c0 - c1)]
+                                           : lists[(size_t)RC_HUGE * n_rows + (li - c0 - c1 - c2)];
+    const uint32_t b = off[r], len = off[r + 1] - b;
+    for (uint32_t i = tid; i < words; i += kBitmapThreads) bits[i] = 0u;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = tid; i < len; i += kBitmapThreads) {
+      const uint32_t x = data[b + i];
+      if (x < universe) atomicOr(&bits[x >> 5], 1u << (x & 31u));  // (always; never index past the bitmap)
+    }
+    __syncthreads();
+    const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
+    uint32_t mine = 0;
+    for (uint32_t i = w0; i < w1; ++i) mine += __popc(bits[i]);
+    const uint32_t incl = warp_incl_scan(mine);
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    const uint32_t ws = warp_incl_scan(wsum[lane]);  // 32 warps
+    uint32_t pos = b + incl - mine + (w ? __shfl_sync(0xffffffffu, ws, w - 1) : 0u);
+    for (uint32_t i = w0; i < w1; ++i)
+      for (uint32_t x = bits[i]; x; x &= x - 1u) data[pos++] = i * 32u + (uint32_t)__ffs(x) - 1u;
+    if (tid == kBitmapThreads - 1u) ucnt[r] = pos - b;
+    __syncthreads();
   }
 }
 
@@ -435,7 +506,17 @@ __global__ void k_compact_rows(const uint32_t* __restrict__ off, const uint32_t*
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t r = gw; r < n_rows; r += nw) {
     const uint32_t b = off[r], nb = new_off[r], c = new_off[r + 1] - nb;
-    for (uint32_t i = lane; i < c; i += 32) dst[nb + i] = src[b + i];
+    // eight loads in flight per lane: a hub's row is one warp's (R-MAT 18:
+    // 407 us with one, 76 us)
+    uint32_t i = lane;
+    for (; i + 224u < c; i += 256u) {
+      uint32_t x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x[q] = src[b + i + 32u * q];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) dst[nb + i + 32u * q] = x[q];
+    }
+    for (; i < c; i += 32) dst[nb + i] = src[b + i];
   }
 }
 
@@ -487,7 +568,7 @@ cudaError_t radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, si
 }
 
 cudaError_t segmented_sort_unique(const uint32_t* off, uint32_t* data, uint32_t* ucount, uint32_t n_rows,
-                                  uint32_t max_len, cudaStream_t s) {
+                                  uint32_t max_len, uint32_t universe, cudaStream_t s) {
   if (n_rows == 0) return cudaSuccess;
   uint32_t* lists = nullptr;
   uint32_t* counts = nullptr;
@@ -511,22 +592,31 @@ cudaError_t segmented_sort_unique(const uint32_t* off, uint32_t* data, uint32_t*
                                             n_rows);
   k_seg_warp<<<sms * 8, 256, 0, s>>>(off, data, ucount, lists + (size_t)RC_WARP * n_rows, counts + RC_WARP,
                                      n_rows);
-  if (max_len > 32)
+  if (max_len > 256)
+    k_seg_warp_wide<<<sms * 8, 128, 0, s>>>(off, data, ucount, lists + (size_t)RC_W1K * n_rows, counts + RC_W1K, n_rows);
+  const bool bitmap = universe <= kBitmapUniverse;
+  if (max_len > 1024 && bitmap) {
+    const uint32_t bytes = (universe + 31u) / 32u * 4u;
+    if (bytes > 48u * 1024u)
+      cudaFuncSetAttribute(k_seg_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapUniverse / 8u));
+    k_seg_bitmap<<<sms * 2, kBitmapThreads, bytes, s>>>(off, data, ucount, lists, counts, n_rows, universe);
+  } else if (max_len > 1024) {
     k_seg_block<256><<<sms * 8, 256, 2048 * sizeof(uint32_t), s>>>(off, data, ucount,
                                                                   lists + (size_t)RC_B2K * n_rows, counts + RC_B2K,
                                                                   n_rows, 2048u);
-  if (max_len > 2048) {
-    cudaFuncSetAttribute(k_seg_block<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4);
-    k_seg_block<1024><<<sms, 1024, 16384 * sizeof(uint32_t), s>>>(off, data, ucount,
-                                                                 lists + (size_t)RC_B16K * n_rows, counts + RC_B16K,
-                                                                 n_rows, 16384u);
+    if (max_len > 2048) {
+      cudaFuncSetAttribute(k_seg_block<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4);
+      k_seg_block<1024><<<sms, 1024, 16384 * sizeof(uint32_t), s>>>(off, data, ucount,
+                                                                   lists + (size_t)RC_B16K * n_rows,
+                                                                   counts + RC_B16K, n_rows, 16384u);
+    }
+    if (max_len > 16384)
+      k_seg_block<1024><<<sms, 1024, 32768 * sizeof(uint32_t), s>>>(off, data, ucount,
+                                                                   lists + (size_t)RC_B32K * n_rows,
+                                                                   counts + RC_B32K, n_rows, 32768u);
   }
-  if (max_len > 16384)
-    k_seg_block<1024><<<sms, 1024, 32768 * sizeof(uint32_t), s>>>(off, data, ucount,
-                                                                 lists + (size_t)RC_B32K * n_rows, counts + RC_B32K,
-                                                                 n_rows, 32768u);
   e = cudaGetLastError();
-  if (e == cudaSuccess && max_len > 32768) {
+  if (e == cudaSuccess && max_len > 32768 && !bitmap) {
     // Rows beyond shared memory: read back how many, sort them with one keyed radix sort.
     uint32_t H = 0;
     unsigned long long T = 0;

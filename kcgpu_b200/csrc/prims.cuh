@@ -23,10 +23,12 @@ cudaError_t radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, si
 
 // Sorts every row [off[r], off[r+1]) of data ascending and removes duplicates
 // in place: the first ucount[r] entries of the row hold its distinct values.
-// max_len must bound the longest row. Rows longer than 32768 go through a
-// keyed radix sort; the others are sorted in registers or shared memory.
+// max_len must bound the longest row and universe the values (all below it).
+// Rows of up to 1024 entries are sorted in registers; longer ones through a
+// bitmap of the values where universe allows, else in shared memory, and past
+// 32768 entries by a keyed radix sort.
 cudaError_t segmented_sort_unique(const uint32_t* off, uint32_t* data, uint32_t* ucount, uint32_t n_rows,
-                                  uint32_t max_len, cudaStream_t s);
+                                  uint32_t max_len, uint32_t universe, cudaStream_t s);
 
 // Copies the first cnt[r] entries of row r of src (offsets off) into dst at
 // new_off[r], for every row.

@@ -1,0 +1,54 @@
+"""Row sorting, orientation and truss support at the edges of the row lengths
+their kernels are chosen by: 256/257, 512/513, 1024/1025 entries, rows past
+32,768, hubs whose rows one warp walks, a vertex range above and below the
+bitmaps' 2^20, and duplicate entries in every kind of row."""
+import numpy as np
+import pytest
+
+import kcgpu_b200 as kc
+from oracle.oracle import OracleGraph
+
+pytestmark = pytest.mark.gpu
+
+
+def _hubs(degrees, n: int, seed: int, noise: int):
+    """Vertex i of the first len(degrees) gets degrees[i] random neighbours
+    (with repeats on top), the rest a few random edges."""
+    rng = np.random.default_rng(seed)
+    s, d = [], []
+    for i, deg in enumerate(degrees):
+        nb = rng.choice(np.arange(len(degrees), n), size=deg, replace=False)
+        s += [np.full(deg, i), nb[: deg // 3]]
+        d += [nb, np.full(deg // 3, i)]
+    s.append(rng.integers(0, n, noise))
+    d.append(rng.integers(0, n, noise))
+    s, d = np.concatenate(s).astype(np.uint32), np.concatenate(d).astype(np.uint32)
+    order = rng.permutation(s.size)
+    return s[order], d[order], n
+
+
+CASES = {
+    "edges_of_ranges": lambda: _hubs([1, 2, 31, 32, 33, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2047,
+                                      2048, 2049], 6000, 1, 3000),
+    "longest_rows": lambda: _hubs([16_384, 16_385, 32_768, 32_769, 40_000], 60_000, 2, 60_000),
+    "at_the_bitmap_limit": lambda: _hubs([1500, 3000, 33_000], 1 << 20, 3, 40_000),
+    "past_the_bitmap_limit": lambda: _hubs([300, 1500, 3000, 17_000, 33_000], (1 << 20) + 1, 4, 40_000),
+    "dense_core": lambda: kc.gen_rmat(13, 16.0, seed=7).arrays(),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_rows_match_oracle(ctx, name):
+    s, d, n = CASES[name]()
+    og = OracleGraph(s, d, n)
+    want_rp, want_ci = og.csr()
+    want_sup = og.truss_support()
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        rp, ci = g.csr()
+        assert np.array_equal(rp, want_rp) and np.array_equal(ci, want_ci)
+        assert np.array_equal(g.truss_support(), want_sup)
+        for orientation in ("degree", "degen"):
+            og.orient(orientation)
+            want = og.dag()
+            got = g.orient(orientation).dag()
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), orientation

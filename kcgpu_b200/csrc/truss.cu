@@ -6,9 +6,15 @@
 // per edge u < v, in the row-major order of the symmetric CSR's upper
 // triangle.
 //
-// One warp per edge, grid-stride over the edges: the warp streams the shorter
-// adjacency list with coalesced loads and locates each element in the longer
-// one by binary search; the hits are counted with one ballot per 32 elements.
+// Every edge is counted at its longer end u (more neighbours; ties: the larger
+// id): the shorter row is streamed and each entry tested for membership in
+// N(u) with one read, of a bitmap of all vertices in shared memory (a CTA per
+// vertex of more than 32 neighbours) or by a search of the 32 in shared memory (a
+// warp per smaller vertex). Eight lanes read a row together. One warp per edge
+// with a search for the edge's row and a binary search per entry, both chains
+// of dependent L2 reads, took 2.03 ms on R-MAT scale 17 (1.26M edges); this takes
+// 0.72 ms. That form is still the one for graphs above kSupportBitmap vertices,
+// whose bitmap does not fit.
 #include <algorithm>
 
 #include "dev_common.cuh"
@@ -28,6 +34,130 @@ __global__ void k_upper_count(const uint32_t* __restrict__ rp, const uint32_t* _
   }
 }
 
+constexpr uint32_t kSupportBitmap = 1u << 20;  // 128 KB of bits
+constexpr uint32_t kSupportSmall = 32;
+constexpr uint32_t kRowLanes = 8;
+
+constexpr uint32_t kSupportChunk = 1024;
+
+// The tasks of the large vertices, in any order: (vertex, first neighbour) for
+// every kSupportChunk neighbours. A hub of 15,000 neighbours is 15 tasks, each
+// of which pays for setting the hub's bits; as one it was the launch's tail.
+__global__ void k_support_list(const uint32_t* __restrict__ rp, uint32_t n, uint2* list, uint32_t* count) {
+  for (uint32_t u0 = blockIdx.x * blockDim.x; u0 < n; u0 += gridDim.x * blockDim.x) {
+    const uint32_t u = u0 + threadIdx.x;
+    const uint32_t du = u < n ? rp[u + 1] - rp[u] : 0u;
+    const uint32_t tasks = du > kSupportSmall ? (du + kSupportChunk - 1u) / kSupportChunk : 0u;
+    if (!__any_sync(0xffffffffu, tasks != 0u)) continue;
+    uint32_t incl = tasks;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane_id() >= o) incl += y;
+    }
+    uint32_t base = 0;
+    if (lane_id() == 31u) base = atomicAdd(count, incl);
+    base = __shfl_sync(0xffffffffu, base, 31) + incl - tasks;
+    for (uint32_t i = 0; i < tasks; ++i) list[base + i] = make_uint2(u, i * kSupportChunk);
+  }
+}
+
+// Where the support of edge {u, v} goes: ju is v's position in row u, iv u's
+// position in row v.
+__device__ __forceinline__ uint32_t support_index(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ubase,
+                                                  uint32_t u, uint32_t v, uint32_t ju, uint32_t iv) {
+  const uint32_t w = min(u, v), j = u < v ? ju : iv;
+  return ubase[w] + j - ((rp[w + 1] - rp[w]) - (ubase[w + 1] - ubase[w]));
+}
+
+// The neighbours v of u (row [ub, ub + du)) whose rows are not longer, number
+// `first`, first + step, .. below `end`: the lanes of a group of kRowLanes stream row v and
+// count its members of N(u).
+template <class Member>
+__device__ __forceinline__ void support_of_rows(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ col,
+                                                const uint32_t* __restrict__ ubase, uint32_t u, uint32_t ub, uint32_t du,
+                                                uint32_t first, uint32_t end, uint32_t step, uint32_t* sup,
+                                                Member member) {
+  const uint32_t l = lane_id() % kRowLanes;
+  const uint32_t mask = 0xffu << (lane_id() / kRowLanes * kRowLanes);
+  for (uint32_t j = first; j < end; j += step) {
+    const uint32_t v = col[ub + j], b = rp[v], e = rp[v + 1];
+    if (e - b > du || (e - b == du && v > u)) continue;
+    uint32_t hits = 0, at = 0;  // at: u's position in row v
+    for (uint32_t i0 = b; i0 < e; i0 += 4u * kRowLanes) {
+      uint32_t x[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        const uint32_t i = i0 + q * kRowLanes + l;
+        x[q] = i < e ? col[i] : 0xffffffffu;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (x[q] == u) at = i0 + q * kRowLanes + l - b;
+        if (x[q] != 0xffffffffu && member(x[q])) ++hits;
+      }
+    }
+#pragma unroll
+    for (uint32_t o = 1; o < kRowLanes; o <<= 1) {
+      hits += __shfl_xor_sync(mask, hits, o);
+      at = max(at, __shfl_xor_sync(mask, at, o));
+    }
+    if (l == 0) sup[support_index(rp, ubase, u, v, j, at)] = hits;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_support_small(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ col,
+                                                       uint32_t n, const uint32_t* __restrict__ ubase, uint32_t* sup) {
+  __shared__ uint32_t rows[8][kSupportSmall];
+  uint32_t* su = rows[threadIdx.x >> 5];
+  const uint32_t lane = lane_id();
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t u = gw; u < n; u += nw) {
+    const uint32_t ub = rp[u], du = rp[u + 1] - ub;
+    if (du == 0u || du > kSupportSmall) continue;
+    __syncwarp();
+    su[lane] = lane < du ? col[ub + lane] : 0xffffffffu;
+    __syncwarp();
+    support_of_rows(rp, col, ubase, u, ub, du, lane / kRowLanes, du, 32u / kRowLanes, sup, [&](uint32_t x) {
+      uint32_t j = 0;  // the last entry <= x, or the first
+#pragma unroll
+      for (uint32_t s = 16; s; s >>= 1)
+        if (su[j + s] <= x) j += s;
+      return su[j] == x;
+    });
+  }
+}
+
+template <int BT>
+__global__ void __launch_bounds__(BT) k_support_big(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ col,
+                                                    uint32_t n, const uint32_t* __restrict__ ubase,
+                                                    const uint2* __restrict__ list, const uint32_t* count,
+                                                    uint32_t max_tasks, uint32_t* ticket, uint32_t* sup) {
+  extern __shared__ __align__(16) uint32_t bits[];
+  __shared__ uint32_t next;
+  const uint32_t words = (n + 31u) / 32u, cnt = min(*count, max_tasks);
+  for (uint32_t i = threadIdx.x; i < words; i += BT) bits[i] = 0u;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) next = atomicAdd(ticket, 1u);
+    __syncthreads();
+    if (next >= cnt) break;
+    const uint2 task = list[next];
+    const uint32_t u = task.x, ub = rp[u], du = rp[u + 1] - ub;
+    for (uint32_t i = threadIdx.x; i < du; i += BT) {
+      const uint32_t x = col[ub + i];
+      atomicOr(&bits[x >> 5], 1u << (x & 31u));
+    }
+    __syncthreads();
+    support_of_rows(rp, col, ubase, u, ub, du, task.y + threadIdx.x / kRowLanes, min(du, task.y + kSupportChunk),
+                    BT / kRowLanes, sup,
+                    [&](uint32_t x) { return (bits[x >> 5] >> (x & 31u)) & 1u; });
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < du; i += BT) bits[col[ub + i] >> 5] = 0u;
+  }
+}
+
+// One warp per edge, for graphs whose bitmap does not fit.
 __global__ void k_support(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ col, uint32_t n,
                           const uint32_t* __restrict__ ubase, uint32_t m, uint32_t* sup) {
   const uint32_t lane = lane_id();
@@ -77,8 +207,31 @@ kc_status truss_support(kc_graph* g, uint32_t* d_support) {
   const uint32_t g1 = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx->sms * 16));
   k_upper_count<<<g1, 256, 0, s>>>(g->rp, g->col, n, cnt);
   KC_CUDA(prim::scan_exclusive_u32(cnt, ubase, n, s));
-  const uint32_t g2 = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((g->m * 32 + 255) / 256, (uint64_t)ctx->sms * 32));
-  k_support<<<g2, 256, 0, s>>>(g->rp, g->col, n, ubase, (uint32_t)g->m, d_support);
+  if (n <= kSupportBitmap) {
+    uint32_t* ctl = nullptr;  // [0] tasks of the large vertices, [1] ticket
+    uint2* tasks = nullptr;
+    const uint32_t max_tasks = (uint32_t)(2 * g->m / kSupportSmall + 2 * g->m / kSupportChunk + 1);
+    KC_CUDA(t.alloc(&ctl, 2 * sizeof(uint32_t)));
+    KC_CUDA(t.alloc(&tasks, sizeof(uint2) * max_tasks));
+    KC_CUDA(cudaMemsetAsync(ctl, 0, 2 * sizeof(uint32_t), s));
+    k_support_list<<<g1, 256, 0, s>>>(g->rp, n, tasks, ctl);
+    const uint32_t gs = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n * 32 + 255) / 256, (uint64_t)ctx->sms * 16));
+    k_support_small<<<gs, 256, 0, s>>>(g->rp, g->col, n, ubase, d_support);
+    if (g->max_deg > kSupportSmall) {
+      const uint32_t bytes = (n + 31u) / 32u * 4u;
+      // four CTAs of 512 threads per SM while their bitmaps fit, else one of 1024
+      if (bytes <= 48u * 1024u) {
+        k_support_big<512><<<ctx->sms * 4, 512, bytes, s>>>(g->rp, g->col, n, ubase, tasks, ctl, max_tasks, ctl + 1, d_support);
+      } else {
+        KC_CUDA(cudaFuncSetAttribute(k_support_big<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(kSupportBitmap / 8u)));
+        k_support_big<1024><<<ctx->sms, 1024, bytes, s>>>(g->rp, g->col, n, ubase, tasks, ctl, max_tasks, ctl + 1, d_support);
+      }
+    }
+  } else {
+    const uint32_t g2 = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((g->m * 32 + 255) / 256, (uint64_t)ctx->sms * 32));
+    k_support<<<g2, 256, 0, s>>>(g->rp, g->col, n, ubase, (uint32_t)g->m, d_support);
+  }
   KC_CUDA(cudaGetLastError());
   return KC_OK;
 }

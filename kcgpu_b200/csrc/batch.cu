@@ -21,6 +21,7 @@
 #include <tuple>
 #include <vector>
 
+#include "bits.cuh"
 #include "count_kernels.cuh"
 #include "dev_common.cuh"
 #include "engine.h"
@@ -80,12 +81,15 @@ uint32_t grid_for(uint64_t work, int sms) {
 }
 
 void free_union(kc_graph* g) {
-  uint32_t** ps[] = {&g->rp, &g->col, &g->rank, &g->inv, &g->drp, &g->dcol, &g->erow, &g->prio, &g->level, &g->vgraph};
+  uint32_t** ps[] = {&g->rp,   &g->col,  &g->rank,  &g->inv,    &g->drp,      &g->dcol,
+                     &g->erow, &g->prio, &g->level, &g->vgraph, &g->bit_words, &g->dbit_words};
   for (uint32_t** p : ps) {
     if (*p) dfree(*p, g->ctx->stream);
     *p = nullptr;
   }
 }
+
+constexpr uint64_t kBitsPerEdge = 32, kBitsMaxBytes = 16ull << 30;
 
 struct Choice {
   uint32_t mode, unit, part, enc;
@@ -151,15 +155,31 @@ kc_status run_batch(kc_ctx* ctx, const uint32_t* src, const uint32_t* dst, Input
     }
   } release{&U, &plans, &cg, &cge, {e0, e1, e2, e3, e4, ec, eo}};
   uint32_t *ds = nullptr, *dd = nullptr, *dvoff = nullptr, *dnn = nullptr, *derr = nullptr, *vg = nullptr;
-  unsigned long long* deoff = nullptr;
+  unsigned long long *deoff = nullptr, *dboff = nullptr;
+  // Bit rows where they are worth their n^2 / 8 bytes per graph: at most
+  // kBitsPerEdge bytes per input edge (graphs of a density of about 1/128 and
+  // more, or small ones) and kBitsMaxBytes per set of rows.
+  std::vector<unsigned long long> boff((size_t)G + 1, 0);
+  bool bits = E > 0;
+  for (uint32_t g = 0; g < G; ++g) {
+    boff[g + 1] = boff[g] + (unsigned long long)n_nodes[g] * bit_row_words(n_nodes[g]);
+    bits = bits && n_nodes[g] <= kBitsMaxVertices;
+  }
+  bits = bits && boff[G] * 4 <= kBitsPerEdge * E && boff[G] * 4 <= kBitsMaxBytes && 2 * E < 0xffffffffull;
+  const bool in_place = bits && input == Input::kDevice;  // local ids are read where they lie
   if (input == Input::kDeviceOwned) {
     if (edge_off[0] != 0) return fail(KC_ERR_INTERNAL, "in-place batch input must start at edge 0");
     ds = const_cast<uint32_t*>(src);
     dd = const_cast<uint32_t*>(dst);
-  } else {
+  } else if (!in_place) {
     KC_CUDA(t.alloc(&ds, sizeof(uint32_t) * std::max<uint64_t>(1, E)));
     KC_CUDA(t.alloc(&dd, sizeof(uint32_t) * std::max<uint64_t>(1, E)));
   }
+  if (bits) {
+    KC_TRY(dev_alloc(&U, (void**)&U.bit_words, sizeof(uint32_t) * boff[G]));
+    KC_CUDA(t.alloc(&dboff, sizeof(unsigned long long) * ((size_t)G + 1)));
+  }
+  KC_CUDA(t.alloc(&vg, sizeof(uint32_t) * std::max<uint64_t>(1, N)));
   KC_CUDA(t.alloc(&deoff, sizeof(unsigned long long) * ((size_t)G + 1)));
   KC_CUDA(t.alloc(&dvoff, sizeof(uint32_t) * ((size_t)G + 1)));
   KC_CUDA(t.alloc(&dnn, sizeof(uint32_t) * G));
@@ -182,25 +202,34 @@ kc_status run_batch(kc_ctx* ctx, const uint32_t* src, const uint32_t* dst, Input
   KC_CUDA(cudaMemcpyAsync(deoff, eoff_rel.data(), sizeof(unsigned long long) * ((size_t)G + 1), cudaMemcpyHostToDevice, s));
   KC_CUDA(cudaMemcpyAsync(dvoff, voff.data(), sizeof(uint32_t) * ((size_t)G + 1), cudaMemcpyHostToDevice, s));
   KC_CUDA(cudaMemcpyAsync(dnn, n_nodes, sizeof(uint32_t) * G, cudaMemcpyHostToDevice, s));
+  if (bits)
+    KC_CUDA(cudaMemcpyAsync(dboff, boff.data(), sizeof(unsigned long long) * ((size_t)G + 1), cudaMemcpyHostToDevice, s));
   cudaEventRecord(e1, s);
-  k_globalize<<<std::min<uint32_t>(G, 65535), 256, 0, s>>>(gin_s, gin_d, ds, dd, deoff, dvoff, dnn, G, derr);
+  // graph of every original vertex: gives each graph a contiguous rank range
+  k_vertex_graph<<<std::min<uint32_t>(G, 65535), 256, 0, s>>>(dvoff, G, vg);
+  U.vgraph_orig = vg;
+  U.n_graphs = G;
   uint32_t herr = 0;
-  KC_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  KC_CUDA(cudaStreamSynchronize(s));
+  double th[6] = {t0, now_ms(), 0, 0, 0, 0};  // host phase boundaries (stats->host_ms)
+  kc_status st = KC_OK;
+  if (bits) {
+    U.n_bit_words = boff[G];
+    U.bits.words = U.bit_words;
+    U.bits.off = dboff;
+    U.bits.voff = dvoff;
+    st = build_bits(&U, gin_s, gin_d, E, deoff, G, (uint32_t)N, orientation == KC_ORIENT_DEGEN, derr, &herr);
+  } else {
+    k_globalize<<<std::min<uint32_t>(G, 65535), 256, 0, s>>>(gin_s, gin_d, ds, dd, deoff, dvoff, dnn, G, derr);
+    KC_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    KC_CUDA(cudaStreamSynchronize(s));
+  }
   if (herr) return fail(KC_ERR_INVALID_ARG, "graph %u has an endpoint not below its n_nodes", herr - 1);
-
-  double th[6] = {t0, 0, 0, 0, 0, 0};  // host phase boundaries (stats->host_ms)
   th[1] = now_ms();
-  kc_status st = build_csr(&U, ds, dd, E, (uint32_t)N);
+  if (!bits) st = build_csr(&U, ds, dd, E, (uint32_t)N);
   cudaEventRecord(ec, s);
   t.free_now(ds);
   t.free_now(dd);
-  // graph of every original vertex: gives each graph a contiguous rank range
   if (st == KC_OK) {
-    KC_CUDA(t.alloc(&vg, sizeof(uint32_t) * std::max<uint64_t>(1, N)));
-    k_vertex_graph<<<std::min<uint32_t>(G, 65535), 256, 0, s>>>(dvoff, G, vg);
-    U.vgraph_orig = vg;
-    U.n_graphs = G;
     st = orient_graph(&U, orientation);
     cudaEventRecord(eo, s);
     U.vgraph_orig = nullptr;

@@ -440,6 +440,7 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
     p.rp = g->drp;
     p.col = g->dcol;
     p.erow = g->erow;
+    p.bits = g->dbits;
     p.queue = heavy_pass ? pl->heavy : pl->queue;
     p.qstride = heavy_pass ? 1u : std::max(1u, req.n_shards);
     p.bounds = pl->scratch + (heavy_pass ? kHeavyBounds : kClassBounds);

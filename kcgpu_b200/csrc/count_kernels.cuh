@@ -18,6 +18,7 @@ struct CountParams {
   const uint32_t* bounds;    // device [begin, count] per size class
   uint32_t cls;              // this launch's class
   uint32_t n_units_max;      // host upper bound on the class size (grid sizing)
+  BitRows bits;              // a batch's out-lists as bit rows (col is then null), or none
   uint32_t edge_units;       // 0 node units, 1 edge units
   uint32_t edge_roots;       // node units whose root branches are their out-edges (edge units grouped by source)
   const uint32_t* vgraph;    // graph of every rank label, or null

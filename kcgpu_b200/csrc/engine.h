@@ -54,6 +54,15 @@ struct kc_ctx {
   cudaEvent_t pool_fork = nullptr;
 };
 
+namespace kc {
+// Adjacency bit rows of a batch's graphs (see bits.cuh); words null = none.
+struct BitRows {
+  const uint32_t* words = nullptr;
+  const unsigned long long* off = nullptr;  // first word of every graph
+  const uint32_t* voff = nullptr;           // first vertex of every graph, then the vertex count
+};
+}  // namespace kc
+
 struct kc_graph {
   kc_ctx* ctx = nullptr;
   uint32_t n = 0;
@@ -79,6 +88,11 @@ struct kc_graph {
   // graph's vertices get one contiguous range of rank labels (null otherwise)
   const uint32_t* vgraph_orig = nullptr;
   uint32_t n_graphs = 0;
+  // batch of small graphs: bit rows stand in for the CSR (col may be null) and
+  // for the DAG's out-lists (dcol is null while dbits stand), see bits.cuh
+  uint32_t *bit_words = nullptr, *dbit_words = nullptr;
+  uint64_t n_bit_words = 0;  // of each
+  kc::BitRows bits, dbits;
   uint64_t bytes = 0;
 };
 
@@ -90,6 +104,9 @@ namespace kc {
 // edges) runs as 3 chunks: 55.4k graphs/s end to end, against 51.1k in one
 // pass, 49.7k in 2 chunks and 54.2k in 4.
 constexpr uint64_t kDefaultBatchChunkEdges = 160ull << 20;
+
+// Batches of graphs of up to this many vertices can be built from bit rows.
+constexpr uint32_t kBitsMaxVertices = 8192;
 
 // A device allocation tracked against the graph's byte count.
 kc_status dev_alloc(kc_graph* g, void** p, size_t bytes);

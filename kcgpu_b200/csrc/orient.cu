@@ -22,6 +22,7 @@
 // the induced-subgraph bitmaps of the counting stage are upper-triangular.
 #include <algorithm>
 
+#include "bits.cuh"
 #include "dev_common.cuh"
 #include "engine.h"
 #include "prims.cuh"
@@ -657,7 +658,8 @@ kc_status orient_graph(kc_graph* g, uint32_t orientation) {
   KC_TRY(dev_alloc(g, (void**)&g->rank, sizeof(uint32_t) * std::max<size_t>(1, n)));
   KC_TRY(dev_alloc(g, (void**)&g->inv, sizeof(uint32_t) * std::max<size_t>(1, n)));
   KC_TRY(dev_alloc(g, (void**)&g->drp, sizeof(uint32_t) * ((size_t)n + 1)));
-  KC_TRY(dev_alloc(g, (void**)&g->dcol, sizeof(uint32_t) * std::max<uint64_t>(1, g->m)));
+  const bool bits = g->bits.words != nullptr;
+  if (!bits) KC_TRY(dev_alloc(g, (void**)&g->dcol, sizeof(uint32_t) * std::max<uint64_t>(1, g->m)));
   const int vbits = bits_for(n ? n - 1 : 0);
   DevTemps t(s);
   unsigned long long *keys = nullptr, *tmp = nullptr;
@@ -688,15 +690,23 @@ kc_status orient_graph(kc_graph* g, uint32_t orientation) {
   k_rank_from_sorted<<<grid_for(n, ctx->sms), 256, 0, s>>>(keys, n, (vbits >= 64) ? ~0ull : ((1ull << vbits) - 1),
                                                           g->rank, g->inv);
   const uint32_t gw = grid_for((uint64_t)n * 32, ctx->sms, 32);
-  k_out_degree<<<gw, 256, 0, s>>>(g->rp, g->col, n, g->rank, odeg);
+  if (bits) KC_TRY(bits_dag(g, odeg));
+  else k_out_degree<<<gw, 256, 0, s>>>(g->rp, g->col, n, g->rank, odeg);
   KC_CUDA(prim::scan_exclusive_u32(odeg, g->drp, n, s));
-  k_fill_dag<<<gw, 256, 0, s>>>(g->rp, g->col, n, g->rank, g->drp, g->dcol);
+  if (!bits) k_fill_dag<<<gw, 256, 0, s>>>(g->rp, g->col, n, g->rank, g->drp, g->dcol);
   if (n) k_max_row_len<<<grid_for(n, ctx->sms), 256, 0, s>>>(g->drp, n, mx);
   uint32_t max_out = 0;
   KC_CUDA(cudaMemcpyAsync(&max_out, mx, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   KC_CUDA(cudaStreamSynchronize(s));
+  // Units above 1024 vertices take lists: a batch that holds one drops its
+  // oriented bit rows.
+  if (bits && max_out > 1024u) {
+    KC_TRY(dev_alloc(g, (void**)&g->dcol, sizeof(uint32_t) * std::max<uint64_t>(1, g->m)));
+    KC_TRY(bits_dag_lists(g));
+    g->dbits = BitRows();
+  }
   // out-lists in rank order (values are distinct, so dedup keeps them all)
-  KC_CUDA(prim::segmented_sort_unique(g->drp, g->dcol, ucnt, n, max_out, n, s));
+  if (g->dcol) KC_CUDA(prim::segmented_sort_unique(g->drp, g->dcol, ucnt, n, max_out, n, s));
   KC_CUDA(cudaGetLastError());
   KC_CUDA(cudaStreamSynchronize(s));
   g->max_out = max_out;

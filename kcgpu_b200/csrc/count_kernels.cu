@@ -827,10 +827,21 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // unit's cut nodes holds a ticket past the last one, so every cut node is
   // taken: it sets bit 31 of the ticket, and no helper joins after that.
   const bool help = MODE == 1 && !LOCAL && p.help_ticket != nullptr;
+  // In the heavy pass, which starts with more CTAs than units, a CTA without a
+  // unit would look before the owners have a unit to show: an owner announces
+  // itself before it takes its ticket, and whoever finds only announcements
+  // looks again (kHelpPolls times at most, then it leaves).
+  const bool announce = help && p.class_exit == nullptr;
+  bool drained = false;
   const bool pairs = p.bits.words != nullptr;  // out-lists are bit rows
   for (;;) {
     if (gt == 0) {
+      if (announce && !drained) {
+        *(volatile uint32_t*)&p.help_active[blockIdx.x] = kHelpSetUp;
+        __threadfence();
+      }
       uint32_t tk = atomicAdd(p.ticket, 1u);
+      if (announce && !drained && tk >= ucnt) *(volatile uint32_t*)&p.help_active[blockIdx.x] = 0u;
       if (tk < ucnt && past_limit(p.time_limit_ns, p.t0)) {  // out of time: take no more units
         set_error(p.err, DEV_ERR_TIMEOUT);
         tk = 0xffffffffu;
@@ -847,6 +858,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
     bool helper = false;
     if (ui >= ucnt) {
       if (!help || ui == 0xffffffffu) break;
+      drained = true;
       // A CTA of a class launch helps only once the plan's other class
       // launches have finished (all their CTAs exited): while they run, its
       // slot serves them better than a share of another CTA's unit. The
@@ -865,15 +877,21 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
       if (wig == 0) {  // the first warp looks for a unit still being walked
         const uint32_t nb = gridDim.x;
         uint32_t pick = 0;
-        for (uint32_t i0 = 0; i0 < nb && pick == 0u; i0 += 32u) {
-          uint32_t c = 0;
-          if (i0 + lane < nb) {
-            const uint32_t b = (blockIdx.x + 1u + i0 + lane) % nb;
-            const uint32_t a = *(volatile const uint32_t*)&p.help_active[b];
-            if (a != 0u && !(*(volatile const uint32_t*)&p.help_ticket[a - 1u] & 0x80000000u)) c = a;
+        for (uint32_t poll = 0; poll < kHelpPolls; ++poll) {
+          uint32_t soon = 0;
+          for (uint32_t i0 = 0; i0 < nb && pick == 0u; i0 += 32u) {
+            uint32_t c = 0;
+            if (i0 + lane < nb) {
+              const uint32_t b = (blockIdx.x + 1u + i0 + lane) % nb;
+              const uint32_t a = *(volatile const uint32_t*)&p.help_active[b];
+              if (a == kHelpSetUp) soon = 1u;
+              else if (a != 0u && !(*(volatile const uint32_t*)&p.help_ticket[a - 1u] & 0x80000000u)) c = a;
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, c != 0u);
+            if (m) pick = __shfl_sync(0xffffffffu, c, __ffs(m) - 1);
           }
-          const uint32_t m = __ballot_sync(0xffffffffu, c != 0u);
-          if (m) pick = __shfl_sync(0xffffffffu, c, __ffs(m) - 1);
+          if (pick != 0u || !announce || !__any_sync(0xffffffffu, soon)) break;
+          __nanosleep(500);
         }
         if (lane == 0) hdr[6] = pick;
       }

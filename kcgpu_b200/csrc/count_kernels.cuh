@@ -114,13 +114,15 @@ constexpr uint32_t kWarpClassMax = 128;   // largest unit a warp group takes
 #endif
 constexpr uint32_t kUnitBudget = KC_UNIT_BUDGET;  // traversal nodes before a warp unit is handed on
 #ifndef KC_PIVOT_UNIT_BUDGET
-#define KC_PIVOT_UNIT_BUDGET 2048
+#define KC_PIVOT_UNIT_BUDGET 256
 #endif
-// the same for a warp unit walked by pivoting (a pivot node costs more: its
-// candidates are scored). Measured on R-MAT scale 16 (edge units, p8): k = 5
-// took 29.7 / 20.8 / 17.4 ms and k = 6 115 / 102 / 100 ms with 8192 / 2048 /
-// 1024; the serving mix was fastest with 2048.
+// the same for a warp unit walked by pivoting, in tree nodes (a node counted
+// whole is charged for its work): with 2048 a burst of 256 server requests
+// took 29.1 ms and k = 3..15 of a 55k-edge R-MAT 1.46 ms; 512: 25.1 and 1.50;
+// 256: 22.1 and 1.16. R-MAT 17 and Chung-Lu 1M did not move.
 constexpr uint32_t kPivotUnitBudget = KC_PIVOT_UNIT_BUDGET;
+constexpr uint32_t kHelpSetUp = 0xffffffffu;  // active-unit word of a CTA that is taking or setting up a unit
+constexpr uint32_t kHelpPolls = 4096;         // 0.5 us apart: the longest an idle CTA of the heavy pass looks on
 constexpr size_t kStaticSmemBytes = 64;
 constexpr uint32_t kHelpMaxGrid = 2048;   // most CTAs of a launch that takes part in tail helping   // static shared memory of the bitmap kernel (phase clocks), kept off the plan
 

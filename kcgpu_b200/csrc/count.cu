@@ -529,7 +529,11 @@ kc_status count_enqueue(const CountPlan& pl, cudaStream_t s) {
   int classes = 0;
   for (int c = 0; c < kNumClasses; ++c) classes += pl.active[c] ? 1 : 0;
   if (classes > 1) KC_CUDA(cudaEventRecord(pl.fork, s));
-  for (int c = 0; c < kNumClasses; ++c) {
+  // Warp units first: a CTA of a persistent launch keeps its slot until its
+  // queue is empty, so the warp launches' tails (single warps on their last
+  // units) then run beside the CTA launches instead of after them (Chung-Lu
+  // 1M, k = 6: 37.1 ms largest first, 32.5 to 35 ms so; batch of 400: 7.1, 6.7).
+  for (int c = kNumClasses - 1; c >= 0; --c) {
     if (!pl.active[c]) continue;
     if (classes == 1) {
       if (pl.timed) KC_CUDA(cudaEventRecord(pl.tbeg[c], s));

@@ -76,7 +76,10 @@ __global__ void k_bits_degree(BitRows b, const uint32_t* __restrict__ vg, uint32
   for (uint32_t v = gw; v < n; v += nw) {
     const BitRow r = bit_row(b, vg[v], v);
     uint32_t c = 0;
-    for (uint32_t w = lane; w < r.words; w += 32u) c += __popc(r.row[w]);
+    for (uint32_t w = lane * 4u; w < r.words; w += 128u) {
+      const uint4 x = *reinterpret_cast<const uint4*>(r.row + w);
+      c += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+    }
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) deg[v] = c;
     mx = max(mx, c);

@@ -327,7 +327,7 @@ __device__ __forceinline__ void add_common(BitCount& bc, const uint32_t (&P)[ST]
                                            uint32_t j0) {
   uint32_t has[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) has[q] = 0u - ((P[jb] >> ((j0 + (uint32_t)q) & 31u)) & 1u);
+  for (int q = 0; q < 4; ++q) has[q] = (uint32_t)((int32_t)(P[jb] << (31u - ((j0 + (uint32_t)q) & 31u))) >> 31);
 #pragma unroll
   for (int w = 0; w < NW; ++w)
     if (w >= jb)
@@ -1089,10 +1089,11 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
       if (wig == 0) {
         const uint32_t* own = rows + (size_t)(unit - v0) * rw;
         uint32_t carry = 0;
-        for (uint32_t w0 = first; w0 < rw; w0 += 32u) {
-          const uint32_t w = w0 + lane;
-          const uint32_t x = w < rw ? __ldg(own + w) : 0u;
-          const uint32_t c = __popc(x);
+        for (uint32_t w0 = first; w0 < rw; w0 += 128u) {
+          const uint32_t w = w0 + lane * 4u;
+          uint4 x = make_uint4(0u, 0u, 0u, 0u);
+          if (w < rw) x = __ldg(reinterpret_cast<const uint4*>(own + w));
+          const uint32_t c0 = __popc(x.x), c1 = __popc(x.y), c2 = __popc(x.z), c = c0 + c1 + c2 + __popc(x.w);
           uint32_t incl = c;
 #pragma unroll
           for (uint32_t o = 1; o < 32u; o <<= 1) {
@@ -1100,12 +1101,14 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
             if (lane >= o) incl += y;
           }
           uint32_t at = carry + incl - c;
-          if (w < rw && KC_IN_BOUNDS(w - first, kSpanWords, p.err)) {
-            map[w - first] = x;
-            mpre[w - first] = at;
+          if (w < rw && KC_IN_BOUNDS(w - first + 3u, kSpanWords, p.err)) {
+            *reinterpret_cast<uint4*>(map + (w - first)) = x;
+            *reinterpret_cast<uint4*>(mpre + (w - first)) = make_uint4(at, at + c0, at + c0 + c1, at + c0 + c1 + c2);
           }
-          for (uint32_t y = x; y; y &= y - 1u)
-            if (KC_IN_BOUNDS(at, d, p.err)) S[at++] = w * 32u + (uint32_t)__ffs(y) - 1u;
+#pragma unroll
+          for (uint32_t q = 0; q < 4; ++q)
+            for (uint32_t y = q == 0 ? x.x : q == 1 ? x.y : q == 2 ? x.z : x.w; y; y &= y - 1u)
+              if (KC_IN_BOUNDS(at, d, p.err)) S[at++] = (w + q) * 32u + (uint32_t)__ffs(y) - 1u;
           carry += __shfl_sync(0xffffffffu, incl, 31);
         }
       }

@@ -245,7 +245,7 @@ class Graph:
         out = (KcU128 * max(1, n))()
         tot = KcU128()
         check(lib().kc_count_local(self._h, C.byref(p), out, C.byref(tot)))
-        return [out[v].value() for v in range(n)]
+        return _u128_list(out, n)
 
     def kcore(self):
         n = self.info()["n"]

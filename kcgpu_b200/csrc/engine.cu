@@ -44,6 +44,13 @@ __global__ void k_expand_rows(const uint32_t* __restrict__ rp, uint32_t n, uint3
     for (uint32_t i = rp[u] + lane; i < rp[u + 1]; i += 32) src[i] = u;
 }
 
+// Local counts from rank labels to vertex ids.
+__global__ void k_by_vertex(const uint32_t* __restrict__ rank, const ulonglong2* __restrict__ by_rank, uint32_t n,
+                            ulonglong2* by_vertex) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    by_vertex[v] = by_rank[rank[v]];
+}
+
 struct CtxLock {
   kc_ctx* c;
   explicit CtxLock(kc_ctx* ctx) : c(ctx) {
@@ -576,8 +583,6 @@ kc_status kc_count_local(kc_graph* g, const kc_params* p, kc_u128* per_vertex, k
   kc::CtxLock lock(g->ctx);
   const uint32_t n = g->n;
   cudaStream_t s = g->ctx->stream;
-  std::vector<unsigned long long> loc(2 * (size_t)n, 0);
-  unsigned long long tot_lo = 0, tot_hi = 0;
   if (p->k <= 2) {
     // k = 1: every vertex once; k = 2: every vertex in deg(v) edges
     std::vector<uint32_t> rp((size_t)n + 1, 0);
@@ -590,9 +595,10 @@ kc_status kc_count_local(kc_graph* g, const kc_params* p, kc_u128* per_vertex, k
     return KC_OK;
   }
   kc::DevTemps t(s);
-  unsigned long long *d_out = nullptr, *d_local = nullptr;
+  unsigned long long *d_out = nullptr, *d_local = nullptr, *d_vertex = nullptr;
   KC_CUDA(t.alloc(&d_out, 2 * sizeof(unsigned long long)));
   KC_CUDA(t.alloc(&d_local, 2 * sizeof(unsigned long long) * std::max<uint32_t>(1, n)));
+  KC_CUDA(t.alloc(&d_vertex, 2 * sizeof(unsigned long long) * std::max<uint32_t>(1, n)));
   KC_CUDA(cudaMemsetAsync(d_out, 0, 2 * sizeof(unsigned long long), s));
   KC_CUDA(cudaMemsetAsync(d_local, 0, 2 * sizeof(unsigned long long) * std::max<uint32_t>(1, n), s));
   kc::CountRequest req;
@@ -604,22 +610,18 @@ kc_status kc_count_local(kc_graph* g, const kc_params* p, kc_u128* per_vertex, k
   req.flags = 0;
   req.k_max = p->k;
   req.d_local = d_local;
-  kc_status st = kc::count_graph(g, req, d_out, nullptr, nullptr);
-  std::vector<uint32_t> rank(n);
   unsigned long long h[2] = {0, 0};
-  if (st == KC_OK) {
-    cudaError_t e = cudaMemcpyAsync(h, d_out, sizeof(h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(loc.data(), d_local, sizeof(unsigned long long) * 2 * n, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(rank.data(), g->rank, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) st = kc::cuda_fail(e, "local count readback", __FILE__, __LINE__);
+  KC_TRY(kc::count_graph(g, req, d_out, nullptr, h));
+  if (n) {
+    // counters are indexed by rank label; the caller's array by vertex id
+    static_assert(sizeof(kc_u128) == sizeof(ulonglong2), "a count is two words");
+    kc::k_by_vertex<<<std::max(1u, std::min((n + 255u) / 256u, (uint32_t)g->ctx->sms * 16)), 256, 0, s>>>(
+        g->rank, reinterpret_cast<const ulonglong2*>(d_local), n, reinterpret_cast<ulonglong2*>(d_vertex));
+    KC_CUDA(cudaGetLastError());
+    KC_CUDA(cudaMemcpyAsync(per_vertex, d_vertex, sizeof(kc_u128) * n, cudaMemcpyDeviceToHost, s));
+    KC_CUDA(cudaStreamSynchronize(s));
   }
-  if (st != KC_OK) return st;
-  // counters are indexed by rank label; the caller's array by vertex id
-  for (uint32_t v = 0; v < n; ++v) per_vertex[v] = {loc[2 * (size_t)rank[v]], loc[2 * (size_t)rank[v] + 1]};
-  tot_lo = h[0];
-  tot_hi = h[1];
-  if (total) *total = {tot_lo, tot_hi};
+  if (total) *total = {h[0], h[1]};
   return KC_OK;
 }
 

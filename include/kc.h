@@ -66,6 +66,8 @@ typedef enum kc_orientation { KC_ORIENT_DEGREE = 0, KC_ORIENT_DEGEN = 1 } kc_ori
  * pivots every large unit; the count is the same in every mode. */
 typedef enum kc_mode { KC_MODE_ORIENT = 0, KC_MODE_PIVOT = 1, KC_MODE_AUTO = 2 } kc_mode;
 typedef enum kc_unit { KC_UNIT_NODE = 0, KC_UNIT_EDGE = 1 } kc_unit;
+/* Sorted lists are the encoding of units above 1024 vertices; smaller units are
+ * held as bitmaps in either encoding (faster, the same counts). */
 typedef enum kc_encoding { KC_ENC_BITMAP = 0, KC_ENC_LIST = 1 } kc_encoding;
 
 /* kc_params.flags */

@@ -44,8 +44,8 @@ UNIT = "graphs/s"
 # (both grow with the edges: the gather with the out-lists, the build with the
 # pairs it reads and the CSR it writes).
 DRAM_CAPTURE_EDGES = 53_548_148
-COUNT_DRAM_BYTES_CAPTURED = 298.2e6 + 1.7e6
-BUILD_DRAM_BYTES_CAPTURED = 6.21e9
+COUNT_DRAM_BYTES_CAPTURED = 510.6e6 + 4.2e6
+BUILD_DRAM_BYTES_CAPTURED = 2.30e9 + 0.78e9
 DRAM_SOURCE = ("profiles/build_kernels_batched1500_dram.md (ncu dram__bytes_read.sum + dram__bytes_write.sum, "
                "1,500-graph capture scaled by input edges)")
 
@@ -640,9 +640,9 @@ def main():
         peak_src = "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6650 GB/s (of fallback)"
         steps = max(1, args.steps)
         # Counting launch (k_count_bitmap, every counting kernel of a step).
-        # Its algorithmic HBM bytes are the out-lists gathered to build the
-        # induced subgraphs, 4 (|S| + sum of |N+(v)| over v in S) per unit,
-        # counted by the kernels; DRAM traffic per step comes from the ncu
+        # Its algorithmic HBM bytes are the out-lists read to build the induced
+        # subgraphs (here as bit rows: the words of every member's row from the
+        # member on), counted by the kernels; DRAM traffic per step comes from the ncu
         # capture summarised in profiles/ (most of the gather hits L2).
         gb_s = (trav["gather_bytes"] / steps) / (ms_count / 1e3) / 1e9
         sm_mhz = (clk.get("sm_mhz") or 1965.0)
@@ -669,7 +669,7 @@ def main():
         # orientation (8 m + 4 (n + 1)) and write the DAG (4 m + 4 (n + 1)).
         nv, mm = sizes.get("vertices", 0), sizes.get("edges_dedup", 0)
         build_bytes = 8 * E + 20 * mm + 12 * (nv + 1)
-        roofline_build = {"bound": "hbm", "kernel": "CSR build + degree orientation (csr.cu, prims.cu, orient.cu)",
+        roofline_build = {"bound": "hbm", "kernel": "bit-row build + degree orientation (bits.cu, prims.cu, orient.cu)",
                           "achieved": build_bytes / (ms_build / 1e3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                           "frac": build_bytes / (ms_build / 1e3) / 1e9 / hbm_peak, "peak_source": peak_src,
                           "algorithmic_bytes_per_step": build_bytes,

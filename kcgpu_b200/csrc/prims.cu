@@ -665,10 +665,12 @@ cudaError_t segmented_sort_unique(const uint32_t* off, uint32_t* data, uint32_t*
     k_seg_warp_wide<<<sms * 8, 128, 0, s>>>(off, data, ucount, lists + (size_t)RC_W1K * n_rows, counts + RC_W1K, n_rows);
   const bool bitmap = universe <= kBitmapUniverse;
   if (max_len > 1024 && bitmap) {
+    // (the limit is raised whatever the size: the 48 KB a launch may take without
+    // that hold the kernel's static shared memory too)
     const uint32_t bytes = (universe + 31u) / 32u * 4u;
-    if (bytes > 48u * 1024u)
-      cudaFuncSetAttribute(k_seg_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapUniverse / 8u));
-    k_seg_bitmap<<<sms * 2, kBitmapThreads, bytes, s>>>(off, data, ucount, lists, counts, n_rows, universe);
+    e = cudaFuncSetAttribute(k_seg_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapUniverse / 8u));
+    if (e == cudaSuccess)
+      k_seg_bitmap<<<sms * 2, kBitmapThreads, bytes, s>>>(off, data, ucount, lists, counts, n_rows, universe);
   } else if (max_len > 1024) {
     k_seg_block<256><<<sms * 8, 256, 2048 * sizeof(uint32_t), s>>>(off, data, ucount,
                                                                   lists + (size_t)RC_B2K * n_rows, counts + RC_B2K,
@@ -684,7 +686,7 @@ cudaError_t segmented_sort_unique(const uint32_t* off, uint32_t* data, uint32_t*
                                                                    lists + (size_t)RC_B32K * n_rows,
                                                                    counts + RC_B32K, n_rows, 32768u);
   }
-  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess && max_len > 32768 && !bitmap) {
     // Rows beyond shared memory: read back how many, sort them with one keyed radix sort.
     uint32_t H = 0;

@@ -220,7 +220,10 @@ kc_status truss_support(kc_graph* g, uint32_t* d_support) {
     if (g->max_deg > kSupportSmall) {
       const uint32_t bytes = (n + 31u) / 32u * 4u;
       // four CTAs of 512 threads per SM while their bitmaps fit, else one of 1024
+      // (the limit is raised for both: the 48 KB a launch may take without that
+      // hold the kernel's static shared memory too)
       if (bytes <= 48u * 1024u) {
+        KC_CUDA(cudaFuncSetAttribute(k_support_big<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024));
         k_support_big<512><<<ctx->sms * 4, 512, bytes, s>>>(g->rp, g->col, n, ubase, tasks, ctl, max_tasks, ctl + 1, d_support);
       } else {
         KC_CUDA(cudaFuncSetAttribute(k_support_big<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -2,6 +2,10 @@
 their kernels are chosen by: 256/257, 512/513, 1024/1025 entries, rows past
 32,768, hubs whose rows one warp walks, a vertex range above and below the
 bitmaps' 2^20, and duplicate entries in every kind of row."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -42,9 +46,7 @@ CASES = {
 }
 
 
-@pytest.mark.parametrize("name", sorted(CASES))
-def test_rows_match_oracle(ctx, name):
-    s, d, n = CASES[name]()
+def _check(ctx, s, d, n):
     og = OracleGraph(s, d, n)
     want_rp, want_ci = og.csr()
     want_sup = og.truss_support()
@@ -57,3 +59,27 @@ def test_rows_match_oracle(ctx, name):
             want = og.dag()
             got = g.orient(orientation).dag()
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), orientation
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_rows_match_oracle(ctx, name):
+    _check(ctx, *CASES[name]())
+
+
+# Vertex counts whose bitmaps end just below, at and above 48 KB, with and
+# without the kernels' static shared memory.
+AROUND_48K = (392_192, 392_193, 393_088, 393_089, 393_100, 393_200, 393_216, 393_217)
+
+
+def check_around_48k():
+    ctx = kc.Context(0)
+    for n in AROUND_48K:
+        _check(ctx, *_hubs([1500, 3000], n, n, 2000))
+    ctx.close()
+
+
+def test_bitmaps_around_48k_in_a_fresh_process():
+    """(A larger graph in the same process would raise the launch limit first.)"""
+    r = subprocess.run([sys.executable, "-c", "from tests.test_gpu_rows import check_around_48k; check_around_48k()"],
+                       cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-1000:] + r.stderr[-3000:]

@@ -187,7 +187,9 @@ __global__ void k_export_fill(const uint32_t* __restrict__ drp, const uint32_t* 
 //   * one CTA of 1024 threads per SM, since a barrier costs by the CTA;
 //   * runs of small fronts (and short bucket scans) are done by one CTA alone
 //     with block barriers, the others waiting at the next grid barrier. Its
-//     edges are dealt out singly (a search in the front's length prefix);
+//     edges are dealt out singly (a search in the front's length prefix). After
+//     kSoloSteps steps it comes to the barrier and starts again, so that no wait
+//     there is longer than that many steps;
 //   * a front is a list of row pieces of at most kPiece entries, so a hub's
 //     row (15,000 entries) is spread over many warps;
 //   * levels without vertices are skipped through the smallest degree seen.
@@ -202,6 +204,9 @@ constexpr uint32_t kPiece = 128;         // row entries per front piece (four pe
 // about one random access per cycle, so 4,096 of them cost what a grid step's
 // barrier does.
 constexpr uint32_t kSoloFront = 1024, kSoloEdges = 4096, kSoloScan = 4096;
+// Steps of one stretch of the solo CTA: 2 us each on a path (1M vertices are
+// 500,000 sub-rounds), so a stretch is some 10 ms, and its barrier 0.1% of it.
+constexpr uint32_t kSoloSteps = 4096;
 
 struct PeelArgs {
   const uint32_t* rp;
@@ -214,12 +219,15 @@ struct PeelArgs {
   uint32_t* bucket_b;
   uint2* front_a;       // frontier (ping-pong): [begin, end) in col of every row piece
   uint2* front_b;
-  uint32_t* ctr;        // 4 phase slots x 4 counters, zeroed; then the solo CTA's state
+  uint32_t* ctr;        // 4 phase slots x 4 counters, zeroed; then two slots for the solo CTA's state
   uint32_t init_prio;   // 2m: the priority the final batch keeps
   uint32_t* bar;        // grid barrier: arrivals so far, zeroed
   uint32_t* out;        // [0] last level, [1] sub-rounds, [2] error
 };
-constexpr uint32_t kPeelSolo = 32;  // ctr: kPeelStateWords words left by the solo CTA
+// ctr: kPeelStateWords words left by the solo CTA. Two slots taken in turn: a
+// stretch may follow another at once, and its state is written while the other
+// CTAs may still be reading that of the one before.
+constexpr uint32_t kPeelSolo = 32, kPeelSoloSlot = 16;
 constexpr uint32_t kPeelStateWords = 9;
 
 __global__ void k_peel_init(const uint32_t* __restrict__ rp, uint32_t n, int* deg) {
@@ -314,15 +322,16 @@ __device__ __forceinline__ uint32_t peel_scan(uint32_t v, uint32_t* wsum, uint32
   return incl - v + __shfl_sync(0xffffffffu, si - s, w);
 }
 
-// One CTA peels alone for as long as the next step is small (it takes at
-// least one step). Counters live in shared memory; lists in global memory.
+// One CTA peels alone for as long as the next step is small, kSoloSteps steps
+// at most (it takes at least one). Counters live in shared memory; lists in
+// global memory.
 __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
   __shared__ uint32_t pre[kSoloFront], beg[kSoloFront], wsum[kPeelThreads / 32];
   __shared__ uint2 sfront[kSoloFront];
   __shared__ uint32_t cn[2], cb, cmin;  // next front (pieces, vertices), bucket, smallest degree above the level (complemented)
   const uint32_t tid = threadIdx.x;
   bool in_shared = false;  // the front is in sfront
-  while (st.todo > 0 && solo_takes(st, a.n)) {
+  for (uint32_t steps = 0; steps < kSoloSteps && st.todo > 0 && solo_takes(st, a.n); ++steps) {
     uint32_t* bucket = (st.flips & 1u) ? a.bucket_b : a.bucket_a;
     uint32_t* bucket2 = (st.flips & 1u) ? a.bucket_a : a.bucket_b;
     uint2* front = (st.flips & 2u) ? a.front_b : a.front_a;
@@ -434,9 +443,16 @@ __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
 // CTA, 2.4k cycles), after which thread 0 of every CTA reads `words` words at
 // src for its CTA: with every warp of 148 CTAs reading the counters itself,
 // one L2 line served 40,000 requests, which took 15k cycles. The spin is
-// bounded: a CTA that waits for a minute records a timeout, and every CTA
-// leaves the kernel at its next barrier; the whole CTA returns false then.
+// bounded: a CTA whose polls (an L2 round trip each) run out records a timeout,
+// and every CTA leaves the kernel at its next barrier; the whole CTA returns
+// false then. The longest wait by design is one solo stretch or one grid step.
+// (The checked build gives up 256 times sooner, so that its tests see a wait
+// that grows with the graph.)
+#ifdef KC_CHECKED
+constexpr uint32_t kPeelSpins = 1u << 18;
+#else
 constexpr uint32_t kPeelSpins = 1u << 26;
+#endif
 
 __device__ __forceinline__ bool grid_barrier(const PeelArgs& a, uint32_t& target, const uint32_t* src, uint32_t words,
                                              uint32_t* got) {
@@ -449,8 +465,8 @@ __device__ __forceinline__ bool grid_barrier(const PeelArgs& a, uint32_t& target
       uint32_t seen = 0, spins = 0;
       do {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
-      } while (seen < target && ++spins < kPeelSpins);
-      ok = seen >= target;
+      } while ((int32_t)(seen - target) < 0 && ++spins < kPeelSpins);  // (the count may wrap)
+      ok = (int32_t)(seen - target) >= 0;
       if (!ok) set_error(a.out + 2, DEV_ERR_TIMEOUT);
     }
     __syncwarp();
@@ -469,20 +485,21 @@ __global__ void __launch_bounds__(kPeelThreads, 1) k_peel(PeelArgs a) {
   // Counters live in four phase slots; a phase zeroes the slot two phases
   // ahead, which every thread has finished reading by then.
   uint32_t phase = 0;
+  uint32_t stretch = 0;  // of the solo CTA
   auto slot = [&](uint32_t ph) { return a.ctr + (ph & 3u) * 4u; };
   while (st.todo > 0) {
     if (solo_takes(st, a.n)) {
+      uint32_t* o = a.ctr + kPeelSolo + (stretch++ & 1u) * kPeelSoloSlot;
       if (blockIdx.x == 0) {
         peel_solo(a, st);
         if (tid == 0) {
-          uint32_t* o = a.ctr + kPeelSolo;
           o[0] = st.todo; o[1] = st.L; o[2] = st.bucket_end; o[3] = st.bsize;
           o[4] = st.fsize; o[5] = st.pieces; o[6] = st.priority; o[7] = st.flips; o[8] = st.too_big;
         }
       }
-      if (!grid_barrier(a, bar, a.ctr + kPeelSolo, kPeelStateWords, got)) return;
+      if (!grid_barrier(a, bar, o, kPeelStateWords, got)) return;
       st = {got[0], got[1], got[2], got[3], got[4], got[5], got[6], got[7], got[8]};
-      continue;  // (the next step is a grid step, whose barrier comes before the state is written again)
+      continue;
     }
     uint32_t* bucket = (st.flips & 1u) ? a.bucket_b : a.bucket_a;
     uint32_t* bucket2 = (st.flips & 1u) ? a.bucket_a : a.bucket_b;
@@ -594,6 +611,7 @@ kc_status run_peel(kc_graph* g, uint32_t* prio, uint32_t* level) {
   KC_CUDA(t.alloc(&bb, sizeof(uint32_t) * n));
   KC_CUDA(t.alloc(&fa, sizeof(uint2) * front_cap));
   KC_CUDA(t.alloc(&fb, sizeof(uint2) * front_cap));
+  static_assert(kPeelSolo + 2 * kPeelSoloSlot <= 128 && kPeelStateWords <= kPeelSoloSlot, "state slots overlap");
   constexpr uint32_t kCtrWords = 128 + 1;  // the barrier's counter on a line of its own
   KC_CUDA(t.alloc(&ctr, sizeof(uint32_t) * kCtrWords));
   KC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * kCtrWords, s));

@@ -4,8 +4,9 @@ compute-sanitizer is closed on this pool, so the counting kernels carry their
 own checks in that build: every data-dependent scratch index (bitmap words,
 membership map, row table, candidate lists, lane stacks) is tested before the
 access, and a failure records DEV_ERR_BOUNDS, which the call returns as
-KC_ERR_INTERNAL. The parity and local-count suites run against that build in a
-child process (KC_LIBRARY selects it); they must pass unchanged.
+KC_ERR_INTERNAL. Its peel gives up waiting after a fraction of a second. The
+parity, local-count and peel suites run against that build in a child process
+(KC_LIBRARY selects it); they must pass unchanged.
 """
 import os
 import subprocess
@@ -27,6 +28,6 @@ def test_parity_suites_pass_on_the_checked_build():
                           cwd=ROOT, capture_output=True, text=True, check=True).stdout.strip()
     assert name.endswith("libkc_checked.so"), name
     r = subprocess.run([sys.executable, "-m", "pytest", "-m", "gpu", "-x", "-q", "-p", "no:cacheprovider",
-                        "tests/test_gpu_parity.py", "tests/test_gpu_local.py"],
+                        "tests/test_gpu_parity.py", "tests/test_gpu_local.py", "tests/test_gpu_peel.py"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=1800)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]

@@ -1,6 +1,8 @@
 """The degeneracy peel where its step sizes change: graphs peeled by one CTA
 alone, fronts and scans just past its limits, hubs whose rows are split over
-many warps, levels without vertices and windows of the bucket left empty."""
+many warps, levels without vertices, windows of the bucket left empty, and paths,
+whose sub-rounds of two vertices are one CTA's work for far longer than one
+stretch of it."""
 import numpy as np
 import pytest
 
@@ -20,6 +22,11 @@ def _complete(n: int):
     return s, d, n
 
 
+def _path(n: int):
+    a = np.arange(n - 1, dtype=np.uint32)
+    return a, a + 1, n
+
+
 CASES = {
     "one_cta": lambda: kc.gen_rmat(12, 8.0, seed=3).arrays(),
     "scan_limit": lambda: kc.gen_er(8193, 0.002, 5).arrays(),
@@ -28,6 +35,10 @@ CASES = {
     "star_hub_and_core": lambda: G.disjoint_union([_star(40_000), _complete(150), _star(1_023), _star(1_025)]),
     "empty_windows": lambda: G.disjoint_union([_complete(400), _complete(90), _complete(7), _star(9_000)]),
     "rmat15": lambda: kc.gen_rmat(15, 16.0, seed=9).arrays(),
+    "path_20k": lambda: _path(20_000),
+    "path_200k": lambda: _path(200_000),
+    "path_1m": lambda: _path(1_000_000),
+    "paths_and_core": lambda: G.disjoint_union([_path(30_001), _complete(90), _star(9_000), _path(17_000)]),
     "isolated": lambda: (np.array([1], np.uint32), np.array([20_000], np.uint32), 30_000),
 }
 

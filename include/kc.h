@@ -167,8 +167,9 @@ uint64_t kc_kernel_launches(void);
 /* Fault injection for tests, host side only (no counterpart in the reference,
  * whose allocation failures print and continue, include/utils.cuh:44-51).
  * kc_test_fail_alloc_after(n): the (n+1)-th device allocation the library makes
- * from now fails as out of memory (the call returns KC_ERR_OOM); one failure,
- * then the hook disarms; n < 0 disarms it. kc_test_live_allocations(): device
+ * from now fails as out of memory (the call returns KC_ERR_OOM, or its result
+ * where it has a way that takes less memory: batches built from bit rows are
+ * counted again without); one failure, then the hook disarms; n < 0 disarms it. kc_test_live_allocations(): device
  * allocations of the library not yet freed, to check that failing calls leak
  * nothing. Process-wide, not per context. */
 void kc_test_fail_alloc_after(int64_t n);

@@ -80,3 +80,37 @@ def test_endpoint_out_of_range(ctx):
     with pytest.raises(kc.KCError, match=f"graph {bad} "):
         kc.batch_count(ctx, s, d, off, nn, np.full(len(gs), 3, np.uint32))
     assert kc.batch_count(ctx, *_batch(gs)[:4], np.full(len(gs), 3, np.uint32)) is not None
+
+
+@pytest.mark.parametrize("orientation", ["degree", "degen"])
+def test_out_of_memory_takes_the_general_way(ctx, orientation):
+    """Every allocation of a batch built from bit rows fails in turn: the batch
+    is then counted without them, and nothing is left allocated. Staging
+    buffers of a pipeline, and batches that have no bit rows, still fail."""
+    L = kc.lib()
+    cases = [(_small() + [G.multipartite([520, 520, 520])], 0, True), (_small(), 2000, False),
+             (CASES["too_many_vertices"](), 0, False)]
+    for gs, chunk, always in cases:
+        s, d, off, nn = _batch(gs)
+        ks = np.full(len(gs), 3, np.uint32)
+        ctx.set_batch_chunk_edges(chunk)
+        try:
+            want = kc.batch_count(ctx, s, d, off, nn, ks, orientation=orientation)
+            L.kc_ctx_release_cached_memory(ctx.handle)
+            base = L.kc_test_live_allocations()
+            outcomes = []
+            for i in range(200):
+                L.kc_test_fail_alloc_after(i)
+                try:
+                    assert kc.batch_count(ctx, s, d, off, nn, ks, orientation=orientation) == want, i
+                    outcomes.append("right")
+                except kc.KCError as e:
+                    assert e.name == "KC_ERR_OOM" and not always, (i, str(e))
+                    outcomes.append("oom")
+                finally:
+                    L.kc_test_fail_alloc_after(-1)
+                L.kc_ctx_release_cached_memory(ctx.handle)
+                assert L.kc_test_live_allocations() == base, i
+            assert ("oom" in outcomes) == (not always) and outcomes[-1] == "right"
+        finally:
+            ctx.set_batch_chunk_edges(0)

@@ -424,10 +424,14 @@ __global__ void __launch_bounds__(128) k_seg_warp_wide(const uint32_t* __restric
 
 // CTA per row for rows above 1,024 entries with values below kBitmapUniverse:
 // every value sets its bit, and the bits in order are the sorted, distinct row.
-// Its cost is the row's plus universe / 32 words, where a bitonic sort of
-// 16,384 entries is 105 stages of barriers (0.3 ms on one CTA; R-MAT 18: the
-// long rows took 0.60 ms in two launches and a keyed radix sort of its largest
-// rows with a host synchronisation, 0.06 ms here).
+// Its cost is the row's plus two reads of universe / 32 words, where a bitonic
+// sort of 16,384 entries is 105 stages of barriers (0.3 ms on one CTA; R-MAT 18:
+// the long rows took 0.60 ms in two launches and a keyed radix sort of its
+// largest rows with a host synchronisation, 0.06 ms here). The shortest rows in
+// the largest universe are its worst case: builds with 25,000 rows of 1,100
+// entries and 2^20 vertices take 3.16 ms (sorted in shared memory 3.86 ms), with
+// 20,000 rows of 1,500 entries 3.05 ms (3.53 ms; 6.48 ms here when every lane
+// read a run of words of its own, 32 lanes in one bank).
 constexpr uint32_t kBitmapThreads = 1024;
 
 __global__ void __launch_bounds__(kBitmapThreads) k_seg_bitmap(const uint32_t* __restrict__ off, uint32_t* data,
@@ -437,35 +441,46 @@ __global__ void __launch_bounds__(kBitmapThreads) k_seg_bitmap(const uint32_t* _
   extern __shared__ __align__(16) uint32_t bits[];
   __shared__ uint32_t wsum[kBitmapThreads / 32];
   const uint32_t tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+  // a warp's words are consecutive and its lanes take them in turn: with a run
+  // of consecutive words per lane, up to 32 lanes met in one bank
   const uint32_t words = (universe + 31u) / 32u;
-  const uint32_t per = (words + kBitmapThreads - 1u) / kBitmapThreads;  // words per thread, consecutive
+  const uint32_t span = (words + kBitmapThreads - 1u) / kBitmapThreads * 32u;  // words of a warp
+  const uint32_t lo = min(words, w * span), hi = min(words, lo + span);
   const uint32_t c0 = min(counts[RC_B2K], n_rows), c1 = min(counts[RC_B16K], n_rows), c2 = min(counts[RC_B32K], n_rows),
                  c3 = min(counts[RC_HUGE], n_rows);
+  for (uint32_t i = tid; i < words; i += kBitmapThreads) bits[i] = 0u;
+  __syncthreads();
   for (uint32_t li = blockIdx.x; li < c0 + c1 + c2 + c3; li += gridDim.x) {
     const uint32_t r = li < c0             ? lists[(size_t)RC_B2K * n_rows + li]
                        : li < c0 + c1      ? lists[(size_t)RC_B16K * n_rows + (li - c0)]
                        : li < c0 + c1 + c2 ? lists[(size_t)RC_B32K * n_rows + (li - c0 - c1)]
                                            : lists[(size_t)RC_HUGE * n_rows + (li - c0 - c1 - c2)];
     const uint32_t b = off[r], len = off[r + 1] - b;
-    for (uint32_t i = tid; i < words; i += kBitmapThreads) bits[i] = 0u;
-    __syncthreads();
 #pragma unroll 4
     for (uint32_t i = tid; i < len; i += kBitmapThreads) {
       const uint32_t x = data[b + i];
       if (x < universe) atomicOr(&bits[x >> 5], 1u << (x & 31u));  // (always; never index past the bitmap)
     }
     __syncthreads();
-    const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
     uint32_t mine = 0;
-    for (uint32_t i = w0; i < w1; ++i) mine += __popc(bits[i]);
-    const uint32_t incl = warp_incl_scan(mine);
-    if (lane == 31) wsum[w] = incl;
+#pragma unroll 8
+    for (uint32_t i = lo + lane; i < hi; i += 32u) mine += __popc(bits[i]);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) wsum[w] = mine;
     __syncthreads();
     const uint32_t ws = warp_incl_scan(wsum[lane]);  // 32 warps
-    uint32_t pos = b + incl - mine + (w ? __shfl_sync(0xffffffffu, ws, w - 1) : 0u);
-    for (uint32_t i = w0; i < w1; ++i)
-      for (uint32_t x = bits[i]; x; x &= x - 1u) data[pos++] = i * 32u + (uint32_t)__ffs(x) - 1u;
-    if (tid == kBitmapThreads - 1u) ucnt[r] = pos - b;
+    uint32_t pos = b + __shfl_sync(0xffffffffu, ws, w) - mine;
+    for (uint32_t i0 = lo; i0 < hi; i0 += 32u) {
+      const uint32_t i = i0 + lane;
+      uint32_t x = i < hi ? bits[i] : 0u;
+      if (!__any_sync(0xffffffffu, x != 0u)) continue;
+      if (x) bits[i] = 0u;  // for the next row
+      const uint32_t c = __popc(x), incl = warp_incl_scan(c);
+      uint32_t at = pos + incl - c;
+      for (; x; x &= x - 1u) data[at++] = i * 32u + (uint32_t)__ffs(x) - 1u;
+      pos += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (tid == kBitmapThreads - 1u) ucnt[r] = ws;
     __syncthreads();
   }
 }

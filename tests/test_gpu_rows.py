@@ -37,6 +37,9 @@ CASES = {
     "longest_rows": lambda: _hubs([16_384, 16_385, 32_768, 32_769, 40_000], 60_000, 2, 60_000),
     "at_the_bitmap_limit": lambda: _hubs([1500, 3000, 33_000], 1 << 20, 3, 40_000),
     "past_the_bitmap_limit": lambda: _hubs([300, 1500, 3000, 17_000, 33_000], (1 << 20) + 1, 4, 40_000),
+    # more long rows than CTAs sort them
+    "many_long_rows": lambda: _hubs([1025 + 7 * (i % 147) for i in range(700)], 120_000, 5, 10_000),
+    "many_long_rows_wide": lambda: _hubs([1100] * 320, 1 << 20, 6, 10_000),
     # one scan tile and the one-CTA key sort end at 4,096 vertices
     "small_4095": lambda: kc.gen_er(4095, 0.004, 11).arrays(),
     "small_4096": lambda: kc.gen_er(4096, 0.004, 12).arrays(),

@@ -1,7 +1,8 @@
 """Row sorting, orientation and truss support at the edges of the row lengths
 their kernels are chosen by: 256/257, 512/513, 1024/1025 entries, rows past
 32,768, hubs whose rows one warp walks, a vertex range above and below the
-bitmaps' 2^20, and duplicate entries in every kind of row."""
+bitmaps' 2^20, duplicate entries in every kind of row, and the edge counts,
+degrees and vertex counts that the support kernels are chosen by."""
 import subprocess
 import sys
 from pathlib import Path
@@ -11,6 +12,7 @@ import pytest
 
 import kcgpu_b200 as kc
 from oracle.oracle import OracleGraph
+from tests import graphs as G
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +33,17 @@ def _hubs(degrees, n: int, seed: int, noise: int):
     return s[order], d[order], n
 
 
+def _star(leaves: int):
+    return np.zeros(leaves, np.uint32), np.arange(1, leaves + 1, dtype=np.uint32), leaves + 1
+
+
+def _matching_and_core(m: int):
+    """A complete graph of 300 vertices and single edges, m edges in all."""
+    s, d = G.complete(300)
+    k = m - s.size
+    return G.disjoint_union([(s, d, 300), (np.arange(k), np.arange(k, 2 * k), 2 * k)])
+
+
 CASES = {
     "edges_of_ranges": lambda: _hubs([1, 2, 31, 32, 33, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2047,
                                       2048, 2049], 6000, 1, 3000),
@@ -40,6 +53,14 @@ CASES = {
     # more long rows than CTAs sort them
     "many_long_rows": lambda: _hubs([1025 + 7 * (i % 147) for i in range(700)], 120_000, 5, 10_000),
     "many_long_rows_wide": lambda: _hubs([1100] * 320, 1 << 20, 6, 10_000),
+    # supports from bitmaps (49,152 edges and more): vertices around a warp's share
+    # with a small and with a wide bitmap, hubs cut into few and into many tasks,
+    # most of a bitmap set by one vertex
+    "support_shares": lambda: _hubs([31, 32, 33, 34, 127, 128, 129, 130, 255, 256, 257, 513], 30_000, 8, 80_000),
+    "support_shares_wide": lambda: _hubs([31, 32, 33, 34, 127, 128, 129, 130, 255, 256, 257, 1025] * 8, 400_000, 9, 80_000),
+    "support_stars": lambda: G.disjoint_union([_star(70_000), _star(17_000), G.multipartite([30, 40, 50])]),
+    "support_edges_below": lambda: _matching_and_core(49_151),
+    "support_edges_at": lambda: _matching_and_core(49_152),
     # one scan tile and the one-CTA key sort end at 4,096 vertices
     "small_4095": lambda: kc.gen_er(4095, 0.004, 11).arrays(),
     "small_4096": lambda: kc.gen_er(4096, 0.004, 12).arrays(),
@@ -77,7 +98,7 @@ AROUND_48K = (392_192, 392_193, 393_088, 393_089, 393_100, 393_200, 393_216, 393
 def check_around_48k():
     ctx = kc.Context(0)
     for n in AROUND_48K:
-        _check(ctx, *_hubs([1500, 3000], n, n, 2000))
+        _check(ctx, *_hubs([1500, 3000], n, n, 70_000))
     ctx.close()
 
 

@@ -34,6 +34,9 @@ CASES = {
     "star_past_edge_limit": lambda: _star(16_400),
     "star_hub_and_core": lambda: G.disjoint_union([_star(40_000), _complete(150), _star(1_023), _star(1_025)]),
     "empty_windows": lambda: G.disjoint_union([_complete(400), _complete(90), _complete(7), _star(9_000)]),
+    "one_cta_star": lambda: _star(4_095),
+    "several_ctas_star": lambda: _star(4_096),
+    "hubs_over_leaves": lambda: G.disjoint_union([_star(600)] * 27),
     "rmat15": lambda: kc.gen_rmat(15, 16.0, seed=9).arrays(),
     "path_20k": lambda: _path(20_000),
     "path_200k": lambda: _path(200_000),

@@ -63,7 +63,8 @@ typedef enum kc_orientation { KC_ORIENT_DEGREE = 0, KC_ORIENT_DEGEN = 1 } kc_ori
 /* KC_MODE_ORIENT and KC_MODE_PIVOT are the reference's two algorithms (-q o|p).
  * KC_MODE_AUTO (an engine extension) lists each small unit by orientation and
  * switches a unit to pivoting when its traversal outgrows a fixed budget, and
- * pivots every large unit; the count is the same in every mode. */
+ * pivots every large unit, and every unit for k > 19; the count is the same in
+ * every mode. */
 typedef enum kc_mode { KC_MODE_ORIENT = 0, KC_MODE_PIVOT = 1, KC_MODE_AUTO = 2 } kc_mode;
 typedef enum kc_unit { KC_UNIT_NODE = 0, KC_UNIT_EDGE = 1 } kc_unit;
 /* Sorted lists are the encoding of units above 1024 vertices; smaller units are

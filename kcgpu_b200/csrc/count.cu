@@ -402,12 +402,18 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
   }
   // Per-launch algorithm: orientation or pivot as requested; KC_MODE_AUTO
   // lists small units by orientation (cheap when their neighbourhood holds few
-  // cliques) and counts large units and over-budget units with the pivot.
+  // cliques) and counts large units and over-budget units with the pivot. Past
+  // the listing's lane stacks (k > 19) it pivots all units: listing there is a
+  // partition's work per subtree (R-MAT of 21k edges, k = 20: 3.66 ms, pivoting
+  // 0.30 ms; G(150, 0.7), k = 23: 5.0 and 3.8 ms; batch of 100 mixed graphs, k up to
+  // 23: 5.3 and 1.7 ms).
+  const uint32_t t_list = pl->edge ? (k_max >= 2 ? k_max - 2 : 0) : k_max - 1;
+  const bool auto_lists = t_list <= (uint32_t)kLaneStack + 2u;
   auto launch_mode = [&](bool warp_group, bool heavy_pass) -> uint32_t {
     if (req.mode != KC_MODE_AUTO) return req.mode;
     // orientation listing only where a budget can hand a clique-heavy unit
     // on to the pivot
-    return (warp_group && !heavy_pass) ? (uint32_t)KC_MODE_ORIENT : (uint32_t)KC_MODE_PIVOT;
+    return (warp_group && !heavy_pass && auto_lists) ? (uint32_t)KC_MODE_ORIENT : (uint32_t)KC_MODE_PIVOT;
   };
   bool any_budget = false;
   for (int c = 0; c <= kNumClasses; ++c) {
@@ -463,7 +469,6 @@ kc_status count_prepare(kc_graph* g, const CountRequest& req, unsigned long long
                                           : nullptr;
     p.time_limit_ns = ctx->time_limit_ns;
     p.t0 = reinterpret_cast<const unsigned long long*>(pl->scratch + kStartWord);
-    const uint32_t t_list = pl->edge ? (k_max >= 2 ? k_max - 2 : 0) : k_max - 1;
     if (warp_group && (lp.mode == KC_MODE_PIVOT || listing_bound(lp.dcap, t_list) > kUnitBudget)) {
       p.budget = lp.mode == KC_MODE_PIVOT ? kPivotUnitBudget : kUnitBudget;
       p.heavy = pl->heavy;

@@ -66,7 +66,6 @@ __device__ __forceinline__ uint32_t valid_mask(uint32_t d, uint32_t w) {  // bit
   return low_mask(d, w);
 }
 
-constexpr int kLaneStack = 16;  // lane-DFS levels: t - 2 <= 16, i.e. k <= 19 (node units)
 // Gather tables (shared memory, needed until the bitmap stands): the member
 // map of up to kSpanWords * 32 rank labels with its prefix, or, for a wider S,
 // a hash (hT keys, 16-bit local indices) behind a filter of one bit per hash

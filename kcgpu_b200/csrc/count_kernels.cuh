@@ -121,6 +121,7 @@ constexpr uint32_t kUnitBudget = KC_UNIT_BUDGET;  // traversal nodes before a wa
 // took 29.1 ms and k = 3..15 of a 55k-edge R-MAT 1.46 ms; 512: 25.1 and 1.50;
 // 256: 22.1 and 1.16. R-MAT 17 and Chung-Lu 1M did not move.
 constexpr uint32_t kPivotUnitBudget = KC_PIVOT_UNIT_BUDGET;
+constexpr int kLaneStack = 16;  // levels of the lane-per-subtree listing: t - 2 <= 16, i.e. k <= 19 (node units)
 constexpr uint32_t kHelpSetUp = 0xffffffffu;  // active-unit word of a CTA that is taking or setting up a unit
 constexpr uint32_t kHelpPolls = 4096;         // 0.5 us apart: the longest an idle CTA of the heavy pass looks on
 constexpr size_t kStaticSmemBytes = 64;

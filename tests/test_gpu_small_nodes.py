@@ -68,3 +68,27 @@ def test_several_k_complete_graph(ctx, n):
         g.orient("degree")
         for ks in (list(range(3, 17)), list(range(3, 34)), [15, 18]):
             assert g.count_multi(ks) == [math.comb(n, k) for k in ks], (n, ks)
+
+
+@pytest.mark.parametrize("n", [24, 33, 70, 140])
+def test_auto_past_the_listing_depth(ctx, n):
+    """k = 19 is the last k that the automatic mode lists; past it every unit is pivoted."""
+    s, d = np.triu_indices(n, 1)
+    s, d = s.astype(np.uint32), d.astype(np.uint32)
+    # the complete graph, padded with a sparse part so that units of every size occur
+    es, ed, en = kc.gen_er(3000, 0.004, n).arrays()
+    s, d = np.concatenate([s, es + n]), np.concatenate([d, ed + n])
+    with kc.Graph.from_edges(ctx, s, d, n + en) as g:
+        g.orient("degen")
+        for k in (18, 19, 20, 21, 30):
+            for unit in ("node", "edge"):
+                for encoding in ("bitmap", "list"):
+                    got = g.count(k, mode="auto", unit=unit, encoding=encoding, part=0)
+                    assert got == math.comb(n, k), (n, k, unit, encoding)
+            assert g.count_local(k, mode="auto")[:n] == [math.comb(n - 1, k - 1)] * n, (n, k)
+    # one pass of a batch whose largest k is past it
+    off = np.array([0, s.size, 2 * s.size], np.uint64)
+    for fixed in (None, dict(mode="auto", unit="node", part=0, encoding="bitmap")):
+        got = kc.batch_count(ctx, np.tile(s, 2), np.tile(d, 2), off, np.full(2, n + en, np.uint32), np.array([18, 21], np.uint32),
+                             autotune=fixed is None, fixed=fixed)
+        assert got == [math.comb(n, 18), math.comb(n, 21)], (n, fixed)

@@ -840,11 +840,12 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         __threadfence();
       }
       uint32_t tk = atomicAdd(p.ticket, 1u);
-      if (announce && !drained && tk >= ucnt) *(volatile uint32_t*)&p.help_active[blockIdx.x] = 0u;
       if (tk < ucnt && past_limit(p.time_limit_ns, p.t0)) {  // out of time: take no more units
         set_error(p.err, DEV_ERR_TIMEOUT);
         tk = 0xffffffffu;
       }
+      // (no unit: the announcement comes down, or the idle CTAs would look on for it)
+      if (announce && !drained && tk >= ucnt) *(volatile uint32_t*)&p.help_active[blockIdx.x] = 0u;
       hdr[0] = tk;
       hdr[1] = 0;  // subtree ticket of this unit
       hdr[4] = 0;  // nodes charged to this unit

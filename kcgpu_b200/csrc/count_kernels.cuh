@@ -123,9 +123,11 @@ constexpr uint32_t kUnitBudget = KC_UNIT_BUDGET;  // traversal nodes before a wa
 constexpr uint32_t kPivotUnitBudget = KC_PIVOT_UNIT_BUDGET;
 constexpr int kLaneStack = 16;  // levels of the lane-per-subtree listing: t - 2 <= 16, i.e. k <= 19 (node units)
 constexpr uint32_t kHelpSetUp = 0xffffffffu;  // active-unit word of a CTA that is taking or setting up a unit
-constexpr uint32_t kHelpPolls = 4096;         // 0.5 us apart: the longest an idle CTA of the heavy pass looks on
-constexpr size_t kStaticSmemBytes = 64;
-constexpr uint32_t kHelpMaxGrid = 2048;   // most CTAs of a launch that takes part in tail helping   // static shared memory of the bitmap kernel (phase clocks), kept off the plan
+// Looks of an idle CTA of the heavy pass, 0.5 us apart and up to 5 us each (it
+// reads a word of every CTA): 21 ms at most.
+constexpr uint32_t kHelpPolls = 4096;
+constexpr size_t kStaticSmemBytes = 64;   // static shared memory of the bitmap kernel (phase clocks), kept off the plan
+constexpr uint32_t kHelpMaxGrid = 2048;   // most CTAs of a launch that takes part in tail helping
 
 // Layout of a plan's scratch words (zeroed by every enqueue).
 constexpr uint32_t kScratchWords = 48;

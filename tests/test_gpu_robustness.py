@@ -11,6 +11,8 @@
   (kc_test_live_allocations), and the calls succeed again once the injection
   stops.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -49,6 +51,29 @@ def test_time_limit_stops_counting_and_context_recovers(ctx):
             assert g.count(5, mode="auto", unit="node", part=0) == want
         finally:
             ctx.set_time_limit(0)
+
+
+def test_time_limit_before_the_heavy_pass_ends_the_call(ctx):
+    """A limit that passes while the class launches run: the heavy pass finds it
+    passed, takes no unit, and its CTAs do not wait for each other's units."""
+    s, d, n = kc.gen_rmat(14, 12.0, seed=3).arrays()
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degen")
+        r = g.count(6, mode="pivot", part=0, stats=True)
+        assert r.stats["heavy_units"] > 0
+        ctx.set_time_limit(200_000)  # the class launches alone take four times that
+        try:
+            seconds = []
+            for _ in range(8):
+                t0 = time.perf_counter()
+                with pytest.raises(kc.KCError, match="KC_ERR_DEVICE_TIMEOUT"):
+                    g.count(6, mode="pivot", part=0)
+                seconds.append(time.perf_counter() - t0)
+        finally:
+            ctx.set_time_limit(0)
+        # the class launches end within their units (0.8 ms); looking on took 21 ms more
+        assert min(seconds) < 5e-3, seconds
+        assert g.count(6, mode="pivot", part=0) == r.count
 
 
 def _every_entry_point(ctx, s, d, n, bs, bd, off, nn, kk):

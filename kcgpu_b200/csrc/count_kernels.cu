@@ -118,7 +118,7 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t x, uint32_t r) {
 template <int NW>
 __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32_t* pre, uint32_t* hdr,
                          uint32_t budget, unsigned __int128& uacc, unsigned long long& st_nodes,
-                         unsigned long long& st_words) {
+                         unsigned long long& st_words KC_ERR_PARAM) {
   uint32_t stk[kLaneStack][NW];
   unsigned long long cnt = 0;
   uint32_t since = 0;
@@ -196,7 +196,7 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
       const uint32_t rem = t - (uint32_t)(lv + 2);
       if (rem == 1u) {
         cnt += n;
-      } else if (n >= rem && KC_IN_BOUNDS(lv, kLaneStack, nullptr)) {
+      } else if (n >= rem && KC_IN_BOUNDS(lv, kLaneStack, err)) {
 #pragma unroll
         for (int q = 0; q < NW; ++q) {
           stk[lv][q] = cur[q];
@@ -233,6 +233,11 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
 // way, a triangle count per vertex, took 42 ms where this had come to 30).
 // R-MAT of 21k edges, k = 8, built, oriented and counted: 3.5 ms before, 1.6 ms.
 
+// Words of the compact bitmap of up to `n` candidates.
+__host__ __device__ constexpr uint32_t compact_words(uint32_t n) {
+  return n <= 32u ? 36u : (n <= 64u ? 64u * 2u : 128u * 4u);
+}
+
 // The compact bitmap of the candidates cand[0, nc) (ascending): bit i of row j
 // is set when cand[i] and cand[j] are adjacent (UPPER: and i > j). The lanes
 // test a row's nc bits side by side, and a ballot makes 32 of them a word: the
@@ -240,7 +245,7 @@ __device__ bool lane_dfs(const uint32_t* B, uint32_t d, uint32_t t, const uint32
 // is no dependence between rows. Rows have ST words in out (ST = 1, 2 or 4).
 template <int NW, int ST, bool UPPER>
 __device__ __forceinline__ void compact_rows(const uint32_t* B, uint32_t Ws, const uint32_t* cand, uint32_t nc,
-                                             uint32_t* out) {
+                                             uint32_t* out KC_ERR_PARAM) {
   const uint32_t lane = lane_id();
   uint32_t cw[NW], cb[NW];
 #pragma unroll
@@ -265,7 +270,7 @@ __device__ __forceinline__ void compact_rows(const uint32_t* B, uint32_t Ws, con
           if (UPPER && t == jb) m[t] &= 0xfffffffeu << (j & 31u);
         }
       }
-      if (lane == 0) {
+      if (lane == 0 && KC_IN_BOUNDS(j * ST + ST - 1u, compact_words(32u * NW), err)) {
         if constexpr (ST == 4) *reinterpret_cast<uint4*>(out + j * 4u) = make_uint4(m[0], m[1], m[2], m[3]);
         else if constexpr (ST == 2) *reinterpret_cast<uint2*>(out + j * 2u) = make_uint2(m[0], m[1]);
         else out[j] = m[0];
@@ -357,11 +362,6 @@ __device__ __forceinline__ uint32_t count_triangles(const uint32_t* up, uint32_t
   return bc.total();
 }
 
-// Words of the compact bitmap of up to `n` candidates, and of the prefix table
-// of close_small.
-__host__ __device__ constexpr uint32_t compact_words(uint32_t n) {
-  return n <= 32u ? 36u : (n <= 64u ? 64u * 2u : 128u * 4u);
-}
 constexpr uint32_t kPairPrefix = 36;   // close_small: exclusive prefix of the row lengths
 constexpr uint32_t kWideMax = 128;     // most candidates of an r = 3 node closed whole
 constexpr uint32_t kSmallMax = 32;     // most candidates of any other node closed whole
@@ -376,10 +376,10 @@ constexpr uint32_t kHistWords = (kSmallMaxRMulti + 1u) * (kSmallMax + 1u);
 // returns its share.
 template <int NW, int ST>
 __device__ __forceinline__ unsigned long long close_wide(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
-                                                         uint32_t nc, uint32_t* up, uint32_t drop) {
+                                                         uint32_t nc, uint32_t* up, uint32_t drop KC_ERR_PARAM) {
   const uint32_t pad = (nc + 3u) & ~3u;
-  if (lane_id() < (pad - nc) * ST) up[nc * ST + lane_id()] = 0u;  // (nc is at most 32 NW, a multiple of four)
-  compact_rows<NW, ST, true>(B, Ws, cand, nc, up);
+  if (lane_id() < (pad - nc) * ST && KC_IN_BOUNDS(pad * ST - 1u, compact_words(32u * NW), err)) up[nc * ST + lane_id()] = 0u;  // (nc is at most 32 NW, a multiple of four)
+  compact_rows<NW, ST, true>(B, Ws, cand, nc, up KC_ERR_ARG(err));
   uint32_t edges = 0;
   const unsigned long long d1 = drop, d2 = drop >= 2u ? d1 * (d1 - 1ull) / 2ull : 0ull;
   unsigned long long t = count_triangles<NW, ST>(up, nc, edges);
@@ -421,13 +421,13 @@ __device__ __forceinline__ unsigned __int128 binom_at(const unsigned long long* 
 template <bool MK>
 __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, uint32_t* pre, uint32_t nc, uint32_t r,
                                                          uint32_t drop, const unsigned long long* binom, uint32_t cols,
-                                                         uint2* queue, uint32_t* hist) {
+                                                         uint2* queue, uint32_t* hist KC_ERR_PARAM) {
   const uint32_t lane = lane_id();
   const uint32_t mine = lane < nc ? adj[lane] : 0u;
   unsigned __int128 acc = 0;
   uint32_t it = 0, steps = 0;
   auto put = [&](uint32_t held, uint32_t dd, uint32_t times) {
-    if (times && KC_IN_BOUNDS(held * (kSmallMax + 1u) + (dd - drop), kHistWords, nullptr))
+    if (times && KC_IN_BOUNDS(held * (kSmallMax + 1u) + (dd - drop), kHistWords, err))
       atomicAdd(&hist[held * (kSmallMax + 1u) + (dd - drop)], times);
   };
   // a node (P, rr vertices to go, dd pivots) without candidates, or with rr <= 3
@@ -463,7 +463,7 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
     }
   };
   if (MK) {
-    for (uint32_t i = lane; i < (r + 1u) * (kSmallMax + 1u); i += 32u) hist[i] = 0u;
+    for (uint32_t i = lane; i < (r + 1u) * (kSmallMax + 1u) && KC_IN_BOUNDS(i, kHistWords, err); i += 32u) hist[i] = 0u;
     __syncwarp();
   }
   if (r <= 4u) {
@@ -494,6 +494,7 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
         if (pre[i + s] <= t) i += s;
       const uint32_t ui = adj[i] & (0xfffffffeu << i);
       const uint32_t j = select_bit(ui, t - pre[i]);
+      if (!KC_IN_BOUNDS(j, nc, err)) break;
       listed(ui & adj[j] & (0xfffffffeu << j), r - 2u, drop);
     }
     steps = __reduce_max_sync(0xffffffffu, it);
@@ -570,7 +571,7 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
             kids = (uint32_t)__popc(R) + 1u;
             break;
           }
-          if (open && KC_IN_BOUNDS(lv, kSmallStack, nullptr)) {
+          if (open && KC_IN_BOUNDS(lv, kSmallStack, err)) {
             sP[lv] = P;
             sR[lv] = R;
             sX[lv] = (rr << 24) | (piv << 16) | dd;
@@ -609,7 +610,7 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
           if (lane >= o) incl += y;
         }
         const bool fits = top + incl <= kQueueCap;
-        if (kids && fits) {
+        if (kids && fits && KC_IN_BOUNDS(top + incl - 1u, kQueueCap, err)) {
           uint2* q = queue + top + (incl - kids);
           *q++ = make_uint2(P & ~R & adj[piv], (rr << 16) | (dd + 1u));
           for (uint32_t x = R; x; x &= x - 1u) {
@@ -641,23 +642,23 @@ __device__ __forceinline__ unsigned __int128 close_small(const uint32_t* adj, ui
 // the node's cost, in tree nodes of the work budget.
 __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t Ws, const uint32_t* cand, uint32_t nc,
                                                      uint32_t* cmp, uint32_t r, uint32_t drop,
-                                                     const unsigned long long* binom, uint32_t cols) {
+                                                     const unsigned long long* binom, uint32_t cols KC_ERR_PARAM) {
   unsigned __int128 t;
   uint32_t cost = 1u + (nc >> 5);
   if (r > 3u && nc <= kSmallMax) {
-    if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
+    if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp KC_ERR_ARG(err));
     t = close_small<false>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols,
-                           reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), nullptr);
+                           reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), nullptr KC_ERR_ARG(err));
     __syncwarp();
     cost = 1u + (cmp[kPairPrefix + 32u] >> 4);
   } else if (nc <= 32u) {
-    t = close_wide<1, 1>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<1, 1>(B, Ws, cand, nc, cmp, drop KC_ERR_ARG(err));
   } else if (nc <= 64u) {
-    t = close_wide<2, 2>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<2, 2>(B, Ws, cand, nc, cmp, drop KC_ERR_ARG(err));
   } else if (nc <= 96u) {
-    t = close_wide<3, 4>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<3, 4>(B, Ws, cand, nc, cmp, drop KC_ERR_ARG(err));
   } else {
-    t = close_wide<4, 4>(B, Ws, cand, nc, cmp, drop);
+    t = close_wide<4, 4>(B, Ws, cand, nc, cmp, drop KC_ERR_ARG(err));
   }
   __syncwarp();
   if (lane_id() == 0) cmp[0] = cost;
@@ -671,12 +672,12 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
 __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
                                                            uint32_t nc, uint32_t* cmp, uint32_t r, uint32_t drop,
                                                            const unsigned long long* binom, uint32_t cols,
-                                                           uint32_t kr, bool open) {
+                                                           uint32_t kr, bool open KC_ERR_PARAM) {
   const uint32_t lane = lane_id();
   uint32_t* hist = cmp + 2u * kPairPrefix + 2u * kQueueCap;
-  if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp);
+  if (cand) compact_rows<1, 1, false>(B, Ws, cand, nc, cmp KC_ERR_ARG(err));
   close_small<true>(cand ? cmp : B, cmp + kPairPrefix, nc, r, drop, binom, cols,
-                    reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), hist);
+                    reinterpret_cast<uint2*>(cmp + 2u * kPairPrefix), hist KC_ERR_ARG(err));
   __syncwarp();
   unsigned __int128 t = 0;
   const uint32_t words = (r + 1u) * (kSmallMax + 1u);
@@ -1314,9 +1315,9 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         __syncwarp();
         pre = hkey;
       }
-      if (W == 1u) lane_dfs<1>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words);
-      else if (W == 2u) lane_dfs<2>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words);
-      else lane_dfs<4>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words);
+      if (W == 1u) lane_dfs<1>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words KC_ERR_ARG(p.err));
+      else if (W == 2u) lane_dfs<2>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words KC_ERR_ARG(p.err));
+      else lane_dfs<4>(B, d, t, pre, hdr, bud, uacc, st_nodes, st_words KC_ERR_ARG(p.err));
     } else if (MODE == 0) {
       // ---- orientation traversal
       const uint32_t t = p.edge_units ? k - 2u : k - 1u;
@@ -1428,9 +1429,11 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         for (uint32_t i = pt.plane; i < d; i += 32u) cand[i] = i;
         __syncwarp();
         if constexpr (MK)  // the k with k - hold0 <= 2 are closed already
-          uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r), kon && kl + r >= k + 3u);
+          uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r),
+                                   kon && kl + r >= k + 3u KC_ERR_ARG(p.err));
         else
-          uacc += close_node(B, Ws, r > 3u && d <= kSmallMax ? nullptr : cand, d, cmp, r, 0u, p.binom, p.binom_cols);
+          uacc += close_node(B, Ws, r > 3u && d <= kSmallMax ? nullptr : cand, d, cmp, r, 0u, p.binom,
+                             p.binom_cols KC_ERR_ARG(p.err));
         st_words += 32u * cmp[0];
       }
     } else {
@@ -1601,9 +1604,10 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         nw = narrow ? (uint32_t)__popc(nzm) : W;
         if (whole) {
           if constexpr (MK)
-            uacc += close_node_multi(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols, kl - hold, kopen);
+            uacc += close_node_multi(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols, kl - hold,
+                                     kopen KC_ERR_ARG(p.err));
           else
-            uacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols);
+            uacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols KC_ERR_ARG(p.err));
           const uint32_t cost = cmp[0];
           since_charge += cost;
           st_words += 32u * cost;

@@ -24,11 +24,21 @@ __device__ __forceinline__ void set_error(uint32_t* err, uint32_t code) {
 // KC_IN_BOUNDS(i, n, err): in a KC_CHECKED build, true when i < n and
 // otherwise records DEV_ERR_BOUNDS and returns false, so the caller skips the
 // access; in a normal build, true (no code). The checked library
-// (libkc_checked.so) stands in for the closed compute-sanitizer.
+// (libkc_checked.so) needs no compute-sanitizer.
 #ifdef KC_CHECKED
 #define KC_IN_BOUNDS(i, n, err) ((uint64_t)(i) < (uint64_t)(n) ? true : (::kc::set_error((err), ::kc::DEV_ERR_BOUNDS), false))
 #else
 #define KC_IN_BOUNDS(i, n, err) true
+#endif
+
+// The error word as a last parameter of a device function whose indices are
+// checked, in a KC_CHECKED build only.
+#ifdef KC_CHECKED
+#define KC_ERR_PARAM , uint32_t* err
+#define KC_ERR_ARG(e) , (e)
+#else
+#define KC_ERR_PARAM
+#define KC_ERR_ARG(e)
 #endif
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }

@@ -1,12 +1,13 @@
 """The bounds-checked engine build (libkc_checked.so, compiled with -DKC_CHECKED).
 
-compute-sanitizer is closed on this pool, so the counting kernels carry their
-own checks in that build: every data-dependent scratch index (bitmap words,
-membership map, row table, candidate lists, lane stacks) is tested before the
-access, and a failure records DEV_ERR_BOUNDS, which the call returns as
-KC_ERR_INTERNAL. Its peel gives up waiting after a fraction of a second. The
-parity, local-count and peel suites run against that build in a child process
-(KC_LIBRARY selects it); they must pass unchanged.
+The counting kernels carry checks of their own in that build, which need no
+compute-sanitizer: the data-dependent scratch indices of the bitmap
+kernels (bitmap words, membership map, candidate lists, lane stacks, and the
+compact rows, shared stack and histogram of the nodes counted whole) are tested
+before the access, and a failure records DEV_ERR_BOUNDS, which the call returns
+as KC_ERR_INTERNAL. Its peel gives up waiting after a fraction of a second. The
+suites that reach these run against that build in a child process (KC_LIBRARY
+selects it); they must pass unchanged.
 """
 import os
 import subprocess
@@ -28,6 +29,7 @@ def test_parity_suites_pass_on_the_checked_build():
                           cwd=ROOT, capture_output=True, text=True, check=True).stdout.strip()
     assert name.endswith("libkc_checked.so"), name
     r = subprocess.run([sys.executable, "-m", "pytest", "-m", "gpu", "-x", "-q", "-p", "no:cacheprovider",
-                        "tests/test_gpu_parity.py", "tests/test_gpu_local.py", "tests/test_gpu_peel.py"],
+                        "tests/test_gpu_parity.py", "tests/test_gpu_local.py", "tests/test_gpu_peel.py",
+                        "tests/test_gpu_small_nodes.py", "tests/test_gpu_batch_bits.py", "tests/test_gpu_queue.py"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=1800)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]

@@ -588,7 +588,7 @@ kc_status count_readback(const CountPlan& pl, cudaStream_t s, PassResult* r, uns
 }
 
 uint32_t count_kernels(const CountPlan& pl) {
-  uint32_t k = pl.n_units <= kSmallQueue ? 1u : 7u;  // the queue (its scan is three)
+  uint32_t k = pl.n_units <= kSmallQueue ? 1u : 4u + prim::scan_launches((size_t)kNumClasses * pl.n_chunks);  // the queue
   for (int c = 0; c <= kNumClasses; ++c) k += pl.active[c] ? 1u : 0u;
   return k;
 }

@@ -614,6 +614,8 @@ int num_sms() {
   return g_sms;
 }
 
+uint32_t scan_launches(size_t n) { return n <= (size_t)TILE ? 1u : 3u; }
+
 cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s) {
   return scan_impl<uint32_t>(in, out, n, s);
 }

@@ -12,11 +12,13 @@ namespace prim {
 
 // out[i] = sum(in[0..i)), out[n] = total (out has n+1 entries). in may alias out.
 cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s);
+// Kernels either scan launches for n values.
+uint32_t scan_launches(size_t n);
 // 64-bit offsets variant (out has n+1 entries).
 cudaError_t scan_exclusive_u32_to_u64(const uint32_t* in, unsigned long long* out, size_t n,
                                       cudaStream_t s);
 
-// Sorts keys[0,n) ascending on bits [0, bits). tmp must hold n keys.
+// Sorts keys[0,n) ascending; bits [bits, 64) of every key are zero. tmp must hold n keys.
 // The result ends in keys (the passes ping-pong through tmp).
 cudaError_t radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, size_t n, int bits,
                            cudaStream_t s);

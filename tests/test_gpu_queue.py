@@ -48,3 +48,17 @@ def test_all_classes(ctx, isolated):
                 for unit, enc in (("node", "bitmap"), ("edge", "bitmap"), ("node", "list")):
                     r = g.count(k, mode=mode, unit=unit, encoding=enc, stats=True)
                     assert r.count == want and r.stats["units"] > 0, (k, mode, unit, enc)
+
+
+@pytest.mark.parametrize("n", [500, 16_384, 16_385, 2_097_152, 2_097_153])
+def test_launches_are_counted(ctx, n):
+    """stats["kernels"] is what the call launched: the queue is one kernel for up
+    to 16,384 units, five up to 2,097,152, then seven."""
+    s, d = G.complete(60)
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degree")
+        g.count(5, mode="pivot", stats=True)
+        before = kc.lib().kc_kernel_launches()
+        r = g.count(5, mode="pivot", stats=True)
+        assert r.count == G.comb(60, 5)
+        assert r.stats["kernels"] == kc.lib().kc_kernel_launches() - before

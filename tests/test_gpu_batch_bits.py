@@ -114,3 +114,20 @@ def test_out_of_memory_takes_the_general_way(ctx, orientation):
             assert ("oom" in outcomes) == (not always) and outcomes[-1] == "right"
         finally:
             ctx.set_batch_chunk_edges(0)
+
+
+@pytest.mark.parametrize("device", [True, False])
+def test_phases_hold_their_own_time(ctx, device):
+    import torch
+
+    gs = [kc.gen_er(1200, 0.2, i).arrays() for i in range(40)]
+    s, d, off, nn = _batch(gs)
+    dev = tuple(torch.from_numpy(x.view(np.int32)).cuda() for x in (s, d))
+    torch.cuda.synchronize()
+    ptrs = tuple(t.data_ptr() for t in dev) if device else None
+    ks = np.full(len(gs), 3, np.uint32)
+    kc.batch_count(ctx, s, d, off, nn, ks, device_ptrs=ptrs)
+    _, st = kc.batch_count(ctx, s, d, off, nn, ks, device_ptrs=ptrs, return_stats=True)
+    host = st["host_ms"]
+    assert all(x >= 0 for x in host) and abs(sum(host) - st["ms_total"]) < 0.1 + 0.01 * st["ms_total"]
+    assert host[0] >= 0.9 * st["ms_h2d"] and host[1] >= 0.9 * st["ms_build"], (host, st["ms_h2d"], st["ms_build"])

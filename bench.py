@@ -664,11 +664,14 @@ def main():
                                                 "traverse": cycles[2] / tot_cy},
                           "tree_nodes_per_step": trav["tree_nodes"] / steps,
                           "heavy_units_per_step": trav["heavy_units"] / steps}
-        # CSR build + orientation: algorithmic bytes = read the input pairs
-        # (8 E), write the symmetric CSR (8 m + 4 (n + 1)), read it again for the
-        # orientation (8 m + 4 (n + 1)) and write the DAG (4 m + 4 (n + 1)).
-        nv, mm = sizes.get("vertices", 0), sizes.get("edges_dedup", 0)
-        build_bytes = 8 * E + 20 * mm + 12 * (nv + 1)
+        # Bit-row build + orientation: algorithmic bytes = read the input pairs
+        # (8 E), write the rows by vertex id once, read them for the degrees and
+        # again for the orientation, write the rows by rank from the diagonal on
+        # (half of them), and write the five vertex arrays (row pointers, ranks,
+        # their inverse, out-degrees, DAG row pointers: 4 (n + 1) each).
+        nv = sizes.get("vertices", 0)
+        row_bytes = int((nn.astype(np.int64) * ((nn.astype(np.int64) + 127) // 128 * 16)).sum())
+        build_bytes = 8 * E + 3 * row_bytes + row_bytes // 2 + 20 * (nv + 1)
         roofline_build = {"bound": "hbm", "kernel": "bit-row build + degree orientation (bits.cu, prims.cu, orient.cu)",
                           "achieved": build_bytes / (ms_build / 1e3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                           "frac": build_bytes / (ms_build / 1e3) / 1e9 / hbm_peak, "peak_source": peak_src,

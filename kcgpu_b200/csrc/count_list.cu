@@ -16,13 +16,13 @@
 //
 // Unlike the reference's list kernels (|S| <= 512 or 1024 through fixed shared
 // arrays, kclique.cuh:505-516, kckernels_orientation.cuh:72-79) the lists live in
-// per-group global scratch sized from the launch's largest unit.
+// per-CTA global scratch sized from the launch's largest unit.
 //
 // The pivot traversal shares the bitmap kernel's structure: nodes with
 // r = k - held <= 2 are closed (1, |C| + drop, edges(G[C]) + drop |C| +
 // C(drop, 2)), the pivot's own branch is taken last in its parent's frame
 // (stack depth bounded by k), and a unit's tree is cut at depth 1-3 with the
-// nodes at the cut handed to the group's partitions by ticket.
+// nodes at the cut handed to the CTA's partitions by ticket.
 #include <algorithm>
 
 #include "count_kernels.cuh"
@@ -66,7 +66,7 @@ __device__ __forceinline__ uint32_t part_filter(const uint32_t* a, uint32_t na, 
   return cnt;
 }
 
-// Layout of one group's global scratch (words).
+// Layout of one CTA's global scratch (words).
 struct ListLayout {
   size_t S, off, cnt, col, fr, total;
 };
@@ -85,11 +85,8 @@ __host__ __device__ inline ListLayout list_layout(uint32_t dcap, size_t cap_edge
 
 template <int MODE>
 __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_edges) {
-  __shared__ uint32_t shdr[8][16];  // per group header (up to 8 groups per block)
-  const uint32_t G = p.G;
-  const uint32_t gpb = blockDim.x / G;
-  const uint32_t gib = threadIdx.x / G;
-  const uint32_t gt = threadIdx.x - gib * G;
+  __shared__ uint32_t hdr[16];
+  const uint32_t G = blockDim.x, gt = threadIdx.x;  // a CTA per unit
   const uint32_t lane = lane_id();
   const uint32_t wig = gt >> 5, nwg = G >> 5;
   LPart pt;
@@ -100,8 +97,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
   const uint32_t part = gt / p.P;
   const uint32_t nparts = G / p.P;
   const ListLayout LY = list_layout(p.dcap, cap_edges, nparts, p.depth, p.fw);
-  uint32_t* gb = p.gbuf + (size_t)(blockIdx.x * gpb + gib) * p.gbuf_words;
-  uint32_t* hdr = shdr[gib];
+  uint32_t* gb = p.gbuf + (size_t)blockIdx.x * p.gbuf_words;
   uint32_t* S = gb + LY.S;
   uint32_t* Loff = gb + LY.off;
   uint32_t* Lcnt = gb + LY.cnt;
@@ -115,9 +111,6 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
   unsigned __int128 acc = 0;
   uint32_t acc_graph = 0xffffffffu;
   unsigned long long st_nodes = 0, st_words = 0, st_bytes = 0;
-  auto gsync = [&]() {
-    if (G == 32) __syncwarp(); else __syncthreads();
-  };
   auto flush = [&]() {
     if (pt.plane == 0 && acc != 0 && acc_graph != 0xffffffffu) atomic_add_u128(p.out + 2ull * acc_graph, acc);
     acc = 0;
@@ -133,7 +126,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
       hdr[0] = tk;
       hdr[1] = 0;
     }
-    gsync();
+    __syncthreads();
     const uint32_t ui = hdr[0];
     if (ui >= ucnt) break;
     const uint32_t unit = p.queue[ubeg + (size_t)ui * p.qstride];
@@ -165,38 +158,38 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
         }
         if (lane == 0) hdr[2] = cnt;
       }
-      gsync();
+      __syncthreads();
       d = hdr[2];
     }
     const uint32_t gph = p.vgraph ? p.vgraph[src] : 0u;
     const uint32_t k = p.gk ? p.gk[gph] : p.k0;
     __threadfence_block();
-    gsync();
+    __syncthreads();
     if (gph != acc_graph) { flush(); acc_graph = gph; }
     if (d > D) {
       if (gt == 0) set_error(p.err, DEV_ERR_CAPACITY);
-      gsync();
+      __syncthreads();
       continue;
     }
     if (MODE == 0) {
       const uint32_t t = p.edge_units ? k - 2u : k - 1u;
       if (t <= 1u || d < t) {
         if (part == 0 && d >= t) acc += (t == 0u) ? 1u : d;
-        gsync();
+        __syncthreads();
         continue;
       }
     } else {
       const uint32_t hold0 = p.edge_units ? 2u : 1u;
       if (d == 0u || hold0 + d < k) {
         if (part == 0 && d == 0u && k == hold0) acc += 1u;
-        gsync();
+        __syncthreads();
         continue;
       }
     }
 
     // ---- local CSR of G[S] ---------------------------------------------------
     for (uint32_t j = gt; j < d; j += G) Lcnt[j] = 0;
-    gsync();
+    __syncthreads();
     const uint32_t last = S[d - 1];
     // pass 1: forward counts (and in-counts for the symmetric rows)
     for (uint32_t j = wig; j < d; j += nwg) {
@@ -221,7 +214,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
       st_bytes += 4ull * (min(i0 + 32u, e) - b);
       if (lane == 0) atomicAdd(&Lcnt[j], c);
     }
-    gsync();
+    __syncthreads();
     // offsets (one warp scans), and the forward counts again for pass 2
     if (wig == 0) {
       uint32_t run = 0;
@@ -239,15 +232,15 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
       }
       if (lane == 0) Loff[d] = run;
     }
-    gsync();
+    __syncthreads();
     const uint32_t E_S = Loff[d];
     if (E_S > cap_edges) {
       if (gt == 0) set_error(p.err, DEV_ERR_CAPACITY);
-      gsync();
+      __syncthreads();
       continue;
     }
     for (uint32_t j = gt; j < d; j += G) Lcnt[j] = 0;  // becomes the in-neighbour cursor
-    gsync();
+    __syncthreads();
     if (MODE == 1) {
       // in-neighbours first (smaller indices), taken in row order by one warp
       // so each row's prefix stays sorted; it needs the forward rows, which
@@ -269,7 +262,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
           __syncwarp();
         }
       }
-      gsync();
+      __syncthreads();
     }
     // forward entries (larger indices) after the in-neighbours
     for (uint32_t j = wig; j < d; j += nwg) {
@@ -293,7 +286,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
       }
     }
     __threadfence_block();
-    gsync();
+    __syncthreads();
 
     auto row = [&](uint32_t v) { return Lcol + Loff[v]; };
     auto rowlen = [&](uint32_t v) { return Loff[v + 1] - Loff[v]; };
@@ -354,13 +347,13 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
       for (uint32_t v = gt; v < d; v += G) key = max(key, (rowlen(v) << 16) | (0xffffu - v));
       key = __reduce_max_sync(0xffffffffu, key);
       if (lane == 0) hdr[8 + wig] = key;
-      gsync();
+      __syncthreads();
       if (gt == 0) {
         uint32_t m = 0;
         for (uint32_t q = 0; q < nwg; ++q) m = max(m, hdr[8 + q]);
         hdr[3] = 0xffffu - (m & 0xffffu);
       }
-      gsync();
+      __syncthreads();
       const uint32_t p0 = hdr[3];
       const uint32_t* Lp0 = row(p0);
       const uint32_t lp0 = rowlen(p0);
@@ -504,7 +497,7 @@ __global__ void __launch_bounds__(256) k_count_list(CountParams p, size_t cap_ed
         }
       }
     }
-    gsync();
+    __syncthreads();
   }
   flush();
   if (p.stats && pt.plane == 0) {
@@ -523,7 +516,7 @@ kc_status prepare_launch_list(kc_ctx* ctx, const LaunchPlan& lp, const CountPara
   if (P == 0 || P > 32 || (P & (P - 1)) != 0)
     return fail(KC_ERR_INVALID_ARG, "partition size %u is not one of 1,2,4,8,16,32", P);
   const uint32_t G = lp.G, block = lp.block;
-  if (block / G > 8) return fail(KC_ERR_INTERNAL, "list kernel supports at most 8 groups per block");
+  if (G != block || block > 256) return fail(KC_ERR_INTERNAL, "the list kernel takes a unit per CTA of at most 256 threads");
   const uint32_t D = std::max<uint32_t>(1, lp.dcap);
   const uint32_t nparts = G / P;
   uint32_t depth, fw;
@@ -547,13 +540,12 @@ kc_status prepare_launch_list(kc_ctx* ctx, const LaunchPlan& lp, const CountPara
   p.depth = depth;
   p.fw = fw;
   p.gbuf_words = LY.total;
-  const uint32_t gpb = block / G;
   auto kern = lp.mode == KC_MODE_ORIENT ? k_count_list<0> : k_count_list<1>;
   int per_sm = 0;
   KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0));
   per_sm = std::max(1, per_sm);
-  uint64_t grid = std::min<uint64_t>((uint64_t)ctx->sms * per_sm, ((uint64_t)p.n_units_max + gpb - 1) / gpb);
-  const uint64_t per_block = (uint64_t)gpb * LY.total * 4;
+  uint64_t grid = std::min<uint64_t>((uint64_t)ctx->sms * per_sm, (uint64_t)p.n_units_max);
+  const uint64_t per_block = (uint64_t)LY.total * 4;
   grid = std::max<uint64_t>(1, std::min<uint64_t>(grid, std::max<uint64_t>(1, (16ull << 30) / per_block)));
   KC_CUDA(dmalloc(&out->gbuf, grid * per_block, s));
   p.gbuf = out->gbuf;

@@ -38,6 +38,10 @@ CASES = {
     "small": _small,
     "deep_out_degrees": lambda: _small() + [G.multipartite([520, 520, 520])],
     "sparse": lambda: [kc.gen_er(6000, 0.001, 3).arrays(), kc.gen_rmat(12, 8.0, seed=4).arrays()],
+    # rows of 157 words (160 held), of 256 and one vertex past the most
+    "wide_rows": lambda: [kc.gen_er(5000, 0.02, 6).arrays(), kc.gen_er(8192, 0.01, 7).arrays(),
+                          kc.gen_er(8161, 0.012, 8).plant_cliques(3, 12, 20, 5).arrays()] + _small(),
+    "past_wide_rows": lambda: [kc.gen_er(5000, 0.02, 6).arrays(), kc.gen_er(8193, 0.01, 7).arrays()] + _small(),
     "too_many_vertices": lambda: _small() + [kc.gen_er(16_385, 0.0002, 5).arrays()],
 }
 

@@ -656,11 +656,12 @@ kc_status kc_truss_support(kc_graph* g, uint32_t* support) {
 uint64_t kc_footprint_bytes(uint32_t n, uint64_t E, uint32_t max_out) {
   // Resident graph: symmetric CSR (4(n+1) + 8m), rank maps (8n), DAG
   // (4(n+1) + 4m), edge rows (4m), peel arrays (8n); build temporaries peak
-  // at about 16E + 16n; counting adds the unit queue (8 max(n, m)) and the
-  // per-group scratch of the largest class (bounded by 24 GiB).
+  // at about 16E + 16n; the peel's are degrees, two buckets and two fronts of
+  // 8 bytes a row piece (28n + m/4); counting adds the unit queue (8 max(n, m))
+  // and the per-group scratch of the largest class (bounded by 24 GiB).
   const uint64_t m = E;
   uint64_t resident = 4ull * (n + 1) + 8ull * m + 8ull * n + 4ull * (n + 1) + 4ull * m + 4ull * m + 8ull * n;
-  uint64_t build = 16ull * E + 16ull * n;
+  uint64_t build = std::max(16ull * E + 16ull * n, 28ull * n + E / 4);
   const uint64_t W = (max_out + 31) / 32;
   uint64_t scratch = max_out > 1024 ? std::min<uint64_t>(24ull << 30, 148ull * 4 * max_out * W) : 64ull << 20;
   uint64_t queue = 8ull * std::max<uint64_t>(n, m);

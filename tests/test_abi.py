@@ -99,3 +99,10 @@ def test_footprint_model_monotone():
     c = kc.footprint_bytes(100_000, 100_000, 50)
     assert 0 < a < b < c
     assert kc.footprint_bytes(4_000_000, 40_000_000, 2000) < 180e9
+
+
+def test_footprint_covers_the_peel_of_a_sparse_graph():
+    """Resident arrays of 24 bytes a vertex, and while the peel runs its degrees,
+    two buckets and two fronts: 28 bytes more."""
+    n = 4_000_000
+    assert kc.footprint_bytes(n, 1000, 0) >= (24 + 28) * n

@@ -695,8 +695,11 @@ __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, ui
   return t;
 }
 
-// Register budgets: orientation fits 56 registers without spills (four
-// 256-thread CTAs per SM); pivoting needs 80 (three), spilling below that.
+// Register budgets: orientation fits 64 registers without spills (four
+// 256-thread CTAs per SM). Pivoting is held to 80 (three): local counts fit them,
+// the walk for one k spills (384 bytes stored, 640 loaded), the walk for several
+// a little (52 and 92). Two CTAs without spills: a batch 29.0 to 31.1 ms, Chung-Lu
+// 1M no faster.
 // MK: several k in one walk (pivoting, one graph).
 template <int MODE, bool LOCAL, bool MK>
 __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountParams p) {

@@ -119,7 +119,10 @@ constexpr uint32_t kUnitBudget = KC_UNIT_BUDGET;  // traversal nodes before a wa
 // the same for a warp unit walked by pivoting, in tree nodes (a node counted
 // whole is charged for its work): with 2048 a burst of 256 server requests
 // took 29.1 ms and k = 3..15 of a 55k-edge R-MAT 1.46 ms; 512: 25.1 and 1.50;
-// 256: 22.1 and 1.16. R-MAT 17 and Chung-Lu 1M did not move.
+// 256: 22.1 and 1.16. R-MAT 17 and Chung-Lu 1M did not move. Walks that count no
+// node whole gain by it too (R-MAT of 21k edges, 256 and 2048: local counts k = 8
+// 1.8 and 5.3 ms, k = 3..33 in one walk 1.9 and 3.9; the exception that was
+// measured: local counts k = 5, 1.38 and 0.93).
 constexpr uint32_t kPivotUnitBudget = KC_PIVOT_UNIT_BUDGET;
 constexpr int kLaneStack = 16;  // levels of the lane-per-subtree listing: t - 2 <= 16, i.e. k <= 19 (node units)
 constexpr uint32_t kHelpSetUp = 0xffffffffu;  // active-unit word of a CTA that is taking or setting up a unit

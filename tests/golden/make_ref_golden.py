@@ -9,7 +9,7 @@ k. The count of a run is the last "Counter = N" line it prints
 (kclique/kclique.cuh:1671-1672); a run that prints none had no unit with
 enough out-degree and counted 0. Needs a GPU; run once, on a B200:
 
-    python tests/golden/make_ref_golden.py --out gpurun_out/ref_counts.json
+    python tests/golden/make_ref_golden.py --out ref_counts.json
 
 The graphs, the exact binomial table the pivot methods read (written in the
 reference's format, 1001 x 401 comma-separated values, C(r, c) and 0 for

@@ -1,7 +1,8 @@
 """Clique-tree nodes that the pivoting kernel counts whole: r = k - held = 3
 with up to 128 candidates and any r with up to 32, at the edges of the word
 and size ranges, with pivots already dropped (dense graphs), universal
-vertices (planted cliques), the largest r (20) and one beyond it."""
+vertices (planted cliques), the largest r (19: k = 20 by node units) and ones
+beyond it."""
 import math
 
 import numpy as np

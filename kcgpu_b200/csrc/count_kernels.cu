@@ -368,8 +368,12 @@ constexpr uint32_t kSmallMax = 32;     // most candidates of any other node clos
 constexpr int kSmallStack = 16;        // close_small: a lane's own frames (r - 3 at most)
 constexpr uint32_t kSmallMaxR = 19;
 constexpr uint32_t kQueueCap = 236;    // close_small: nodes on its shared stack
-// several k: the largest r closed whole, and the words of its histogram
+// several k: the largest r closed whole, and the words of its histogram. No more
+// vertices than the node has can be held, so a node of nc candidates is closed
+// as one of r = nc where r is larger (multi_r): k = 3..33 over blocks of 100
+// vertices (p = 0.4) took 1.62 ms with r alone deciding, 0.40 ms so.
 constexpr uint32_t kSmallMaxRMulti = 15;
+__device__ __forceinline__ uint32_t multi_r(uint32_t r, uint32_t nc) { return min(r, max(nc, 3u)); }
 constexpr uint32_t kHistWords = (kSmallMaxRMulti + 1u) * (kSmallMax + 1u);
 
 // r = 3: triangles + drop edges + C(drop, 2) vertices + C(drop, 3). Every lane
@@ -666,8 +670,8 @@ __device__ __noinline__ unsigned __int128 close_node(const uint32_t* B, uint32_t
   return t;
 }
 
-// close_node for several k at once (nc <= 32, r <= kSmallMaxRMulti for the
-// largest k): the lane's own k has kr = k - held vertices to go (`open`: it is
+// close_node for several k at once (nc <= 32; r of the largest k, or multi_r of
+// it, at most kSmallMaxRMulti): the lane's own k has kr = k - held vertices to go (`open`: it is
 // still to be counted), and its whole count below the node is returned.
 __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, uint32_t Ws, const uint32_t* cand,
                                                            uint32_t nc, uint32_t* cmp, uint32_t r, uint32_t drop,
@@ -1424,7 +1428,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         }
       }
     } else if (MODE == 1 && compact && (d <= kSmallMax || (!mk && d <= kWideMax && k == (p.edge_units ? 5u : 4u))) &&
-               k <= (mk ? kSmallMaxRMulti : kSmallMaxR)) {
+               (mk ? multi_r(k - (p.edge_units ? 2u : 1u), d) <= kSmallMaxRMulti : k <= kSmallMaxR)) {
       // ---- a unit counted whole (edge roots: their sum is the unit's count)
       const uint32_t r = k - (p.edge_units ? 2u : 1u);  // >= 3 here
       if (part == 0 && !helper) {
@@ -1432,7 +1436,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         for (uint32_t i = pt.plane; i < d; i += 32u) cand[i] = i;
         __syncwarp();
         if constexpr (MK)  // the k with k - hold0 <= 2 are closed already
-          uacc += close_node_multi(B, Ws, nullptr, d, cmp, r, 0u, p.binom, p.binom_cols, kl - (k - r),
+          uacc += close_node_multi(B, Ws, nullptr, d, cmp, multi_r(r, d), 0u, p.binom, p.binom_cols, kl - (k - r),
                                    kon && kl + r >= k + 3u KC_ERR_ARG(p.err));
         else
           uacc += close_node(B, Ws, r > 3u && d <= kSmallMax ? nullptr : cand, d, cmp, r, 0u, p.binom,
@@ -1574,7 +1578,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         // and counts it (see close_node)
         auto small = [&](uint32_t n) {
           return compact && r >= 3u && n <= (!mk && r == 3u ? kWideMax : kSmallMax) &&
-                 r <= (mk ? kSmallMaxRMulti : kSmallMaxR);
+                 (mk ? multi_r(r, n) <= kSmallMaxRMulti : r <= kSmallMaxR);
         };
         bool whole = small(nc);
         if (whole && !(above ? claim() : own)) return false;
@@ -1607,7 +1611,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
         nw = narrow ? (uint32_t)__popc(nzm) : W;
         if (whole) {
           if constexpr (MK)
-            uacc += close_node_multi(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols, kl - hold,
+            uacc += close_node_multi(B, Ws, cand, nc, cmp, multi_r(r, nc), drop, p.binom, p.binom_cols, kl - hold,
                                      kopen KC_ERR_ARG(p.err));
           else
             uacc += close_node(B, Ws, cand, nc, cmp, r, drop, p.binom, p.binom_cols KC_ERR_ARG(p.err));

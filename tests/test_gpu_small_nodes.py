@@ -93,3 +93,27 @@ def test_auto_past_the_listing_depth(ctx, n):
         got = kc.batch_count(ctx, np.tile(s, 2), np.tile(d, 2), off, np.full(2, n + en, np.uint32), np.array([18, 21], np.uint32),
                              autotune=fixed is None, fixed=fixed)
         assert got == [math.comb(n, 18), math.comb(n, 21)], (n, fixed)
+
+
+@pytest.mark.parametrize("n", [15, 16, 17, 18, 33, 34, 48, 70])
+@pytest.mark.parametrize("p", [0.4, 0.9])
+def test_several_k_past_the_histogram(ctx, n, p):
+    """Largest k above 16: nodes of up to 15 candidates are counted whole all the same."""
+    s, d, n = _dense(n, p, n + 2)
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degen")
+        single = {k: g.count(k, mode="pivot") for k in range(3, 34)}
+        for ks in (list(range(3, 34)), [5, 24], [17, 20, 31], [3, 16, 17], [33]):
+            for unit in ("node", "edge"):
+                assert g.count_multi(ks, unit=unit) == [single[k] for k in ks], (n, p, ks, unit)
+
+
+def test_several_k_past_the_histogram_on_blocks(ctx):
+    s, d, n = kc.gen_sbm(2000, 20, 0.4, 0.002, 3).plant_cliques(3, 18, 30, 7).arrays()
+    with kc.Graph.from_edges(ctx, s, d, n) as g:
+        g.orient("degen")
+        ks = list(range(3, 31))
+        want = [g.count(k, mode="pivot") for k in ks]
+        for unit in ("node", "edge"):
+            assert g.count_multi(ks, unit=unit) == want
+            assert g.count_multi([4, 25], unit=unit) == [want[1], want[22]]

@@ -249,9 +249,9 @@ __device__ __forceinline__ void warp_append(bool pred, uint32_t x, uint32_t* lis
 // The lanes with pred put their vertex v into the front that sub-round
 // `priority` of level L will peel: level and priority are written now, the
 // row's pieces appended to `front` (the first kSoloFront of them to `sfront`
-// too, where there is one). cnt[0] counts pieces, cnt[1] vertices, in one atomic:
-// what the warps of a large scan wait for is the counter (G(4M, 32M edges): 11.4 ms
-// with an atomic each, 8.1 ms so).
+// too, where there is one: in the solo CTA). cnt[0] counts pieces, cnt[1]
+// vertices; in global memory with one atomic, since what the warps of a large scan
+// wait for is the counter (G(4M, 32M edges): 11.4 ms with an atomic each, 8.1 ms so).
 __device__ __forceinline__ void front_append(const PeelArgs& a, bool pred, uint32_t v, uint32_t L, uint32_t priority,
                                              uint2* front, uint2* sfront, uint32_t* cnt) {
   const uint32_t m = __ballot_sync(0xffffffffu, pred);
@@ -271,9 +271,15 @@ __device__ __forceinline__ void front_append(const PeelArgs& a, bool pred, uint3
     if (lane_id() >= (uint32_t)o) incl += y;
   }
   uint32_t base = 0;
-  if (lane_id() == 31u)
-    base = (uint32_t)atomicAdd(reinterpret_cast<unsigned long long*>(cnt),
-                               (unsigned long long)__popc(m) << 32 | incl);
+  if (lane_id() == 31u) {
+    if (sfront != nullptr) {  // (counters in shared memory: a 64-bit add there is a loop of exchanges)
+      base = atomicAdd(&cnt[0], incl);
+      atomicAdd(&cnt[1], (uint32_t)__popc(m));
+    } else {
+      base = (uint32_t)atomicAdd(reinterpret_cast<unsigned long long*>(cnt),
+                                 (unsigned long long)__popc(m) << 32 | incl);
+    }
+  }
   base = __shfl_sync(0xffffffffu, base, 31) + incl - pieces;
   for (uint32_t i = 0; i < pieces; ++i) {
     const uint2 pc = make_uint2(b + i * kPiece, min(e, b + (i + 1u) * kPiece));
@@ -329,8 +335,7 @@ __device__ __forceinline__ uint32_t peel_scan(uint32_t v, uint32_t* wsum, uint32
 __device__ void peel_solo(const PeelArgs& a, PeelState& st) {
   __shared__ uint32_t pre[kSoloFront], beg[kSoloFront], wsum[kPeelThreads / 32];
   __shared__ uint2 sfront[kSoloFront];
-  __shared__ __align__(8) uint32_t cn[2];
-  __shared__ uint32_t cb, cmin;  // cn: next front (pieces, vertices), bucket, smallest degree above the level (complemented)
+  __shared__ uint32_t cn[2], cb, cmin;  // next front (pieces, vertices), bucket, smallest degree above the level (complemented)
   const uint32_t tid = threadIdx.x;
   bool in_shared = false;  // the front is in sfront
   for (uint32_t steps = 0; steps < kSoloSteps && st.todo > 0 && solo_takes(st, a.n); ++steps) {

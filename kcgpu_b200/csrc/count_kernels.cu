@@ -702,10 +702,17 @@ __device__ __noinline__ unsigned __int128 close_node_multi(const uint32_t* B, ui
 // Register budgets: orientation fits 64 registers without spills (four
 // 256-thread CTAs per SM). Pivoting is held to 80 (three): local counts fit them,
 // the walk for one k spills (384 bytes stored, 640 loaded), the walk for several
-// a little (52 and 92). Two CTAs without spills: a batch 29.0 to 31.1 ms, Chung-Lu
+// a little (52 and 88). Two CTAs without spills: a batch 29.0 to 31.1 ms, Chung-Lu
 // 1M no faster.
-// MK: several k in one walk (pivoting, one graph).
-template <int MODE, bool LOCAL, bool MK>
+// MK: several k in one walk (pivoting, one graph). GATHER: out-lists, a batch's
+// bit rows, or either. Listing has a kernel for each: with the code of both in
+// one, its traversal was slower (k = 5, partition 32: Chung-Lu 1M 217 ms, 192 ms
+// so; R-MAT 16 73 and 68). The walk for one k has one kernel for both, which
+// compiles to the faster walk (R-MAT 17, k = 5, node units: 10.0 ms, 10.9 ms
+// with a kernel for each; the batch 13.0 ms either way).
+enum Gather { kLists, kBitRows, kEither };
+
+template <int MODE, bool LOCAL, bool MK, Gather GATHER>
 __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountParams p) {
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t G = p.G;
@@ -840,7 +847,7 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) k_count_bitmap(CountPa
   // looks again (kHelpPolls times at most, then it leaves).
   const bool announce = help && p.class_exit == nullptr;
   bool drained = false;
-  const bool pairs = p.bits.words != nullptr;  // out-lists are bit rows
+  const bool pairs = GATHER == kEither ? p.bits.words != nullptr : GATHER == kBitRows;  // out-lists are bit rows
   for (;;) {
     if (gt == 0) {
       if (announce && !drained) {
@@ -2092,9 +2099,14 @@ kc_status prepare_launch(kc_ctx* ctx, const LaunchPlan& lp, const CountParams& p
   p.gbuf = nullptr;
 
   const size_t smem_bytes = (size_t)gpb * p.group_words * 4;
-  auto kern = !pivot ? (lp.local ? k_count_bitmap<0, true, false> : k_count_bitmap<0, false, false>)
-              : lp.local ? k_count_bitmap<1, true, false>
-              : mk ? k_count_bitmap<1, false, true> : k_count_bitmap<1, false, false>;
+  const bool bits = p.bits.words != nullptr;
+  if (bits && (lp.local || mk)) return fail(KC_ERR_INTERNAL, "bit rows are a batch's");
+  auto kern = !pivot ? (lp.local ? k_count_bitmap<0, true, false, kLists>
+                        : bits   ? k_count_bitmap<0, false, false, kBitRows>
+                                 : k_count_bitmap<0, false, false, kLists>)
+              : lp.local ? k_count_bitmap<1, true, false, kLists>
+              : mk       ? k_count_bitmap<1, false, true, kLists>
+                         : k_count_bitmap<1, false, false, kEither>;
   // Several classes launch the same kernel with different shared-memory sizes;
   // the attribute is per function, so it is set to the device maximum, once per
   // context (and the occupancy is looked up once per launch shape).
